@@ -141,8 +141,10 @@ def _planes3d(g, n_a, n_b, t):
     normal; B such points turned by one degree about z, 0.1 % of them replaced
     by points of the whole cube."""
     c = 100 * torch.rand(500, 3, generator=g, device="cuda", dtype=t)
-    u, v, w = torch.linalg.qr(torch.randn(500, 3, 3, generator=g, device="cuda",
-                                          dtype=t))[0].unbind(2)
+    w, u = torch.nn.functional.normalize(
+        torch.randn(2, 500, 3, generator=g, device="cuda", dtype=t), dim=2)
+    u = torch.nn.functional.normalize(torch.linalg.cross(w, u))  # in the plane
+    v = torch.linalg.cross(w, u)
 
     def some(n):
         p = torch.empty(n, 3, device="cuda", dtype=t)
