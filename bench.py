@@ -483,10 +483,11 @@ def bench_single(eng, name, n, steps, warmup, args, ctx):
                 "issue_active_ncu": profile_figures("eb_main").get("issue_active"),
                 "peak_source": "SMs x 128 FP32 lanes x sampled SM clock (non-fused ops)"}
     elif res.variant_used == hd._lib.VARIANT_BF16:
-        # Split-BF16 contraction: 3 products x 2 K FLOP per pair and direction.
+        # Split-BF16 contraction: 3 products x 2 K FLOP per pair that met a tile
+        # (rows drop out between runs of tiles; the instrumented solve counts).
         K = ((dims + 15) // 16) * 16
         dirs = 2 if undirected else 1
-        flops = dirs * 3.0 * 2.0 * K * float(n) * float(n)
+        flops = 3.0 * 2.0 * K * float(rc.visited_pairs)
         t_ms = phase[3]
         ach = flops / (t_ms / 1e3) / 1e12
         fig = profile_figures("bf16_rowmin")
@@ -494,7 +495,8 @@ def bench_single(eng, name, n, steps, warmup, args, ctx):
                 "peak": peaks["bf16_tflops"], "unit": "TFLOP/s",
                 "frac": ach / peaks["bf16_tflops"],
                 "frac_of_sustained": ach / peaks["bf16_tflops_sustained"],
-                "traffic": traffic_from_profiles("bf16_rowmin", float(n) * float(n)),
+                "traffic": traffic_from_profiles("bf16_rowmin", rc.visited_pairs / dirs),
+                "visited_pairs": int(rc.visited_pairs),
                 "algorithmic_flops_per_launch": flops / dirs, "ms": t_ms,
                 "tensor_pipe_active_ncu": fig.get("tensor_pipe_active"),
                 "peak_source": pkind + " bf16_tflops (burst); frac_of_sustained against "

@@ -15,6 +15,15 @@
 // Hausdorff distance — bit-identical to the FP32 scans.  The certifying
 // pair's distance is then recomputed in FP64 (certify()).
 //
+// Early break at the grain of tensor tiles (run_bf16_k, bf16_rounds): the work
+// is bound by the tensor pipe, and meeting every (row, tile) pair is what costs.
+// B's tiles are taken in runs; a row whose m + E over the tiles seen so far is
+// below the lower bound L of some completed row cannot be the maximum and is
+// dropped, and the remaining rows are packed together before the next run.
+// Undirected, one GB300, every pair before, runs now: 64-D unit rows 1M x 1M
+// 422 -> 85 ms, 250k x 250k 28.1 -> 7.4 ms, 64k x 64k 2.19 -> 1.60 ms; 16-D
+// 500k x 300k directed 21.7 -> 3.9 ms.
+//
 // Kernel shape (one CTA per 256 A rows = two 128-row regions, 6 warps, 1 CTA
 // per SM):
 //   warp 0      producer: TMA bulk copies (cp.async.bulk) of the A block once
@@ -65,10 +74,10 @@ __host__ __device__ __forceinline__ uint32_t pack_off(uint32_t row, uint32_t k, 
 
 // One thread per (row, 8-element chunk): splits, writes hi and lo chunks.
 // Tile t of rows [t*R, t*R+R) occupies 2 * R * Kp * 2 bytes: hi then lo.
+// Packed row j is row perm(j) of X.
 __global__ void k_bf16_pack(const float* __restrict__ X, uint64_t n, int D, int Kp, int R,
-                            uint64_t nPad, unsigned char* __restrict__ out,
-                            float* __restrict__ norms, uint32_t* __restrict__ maxnorm_ord,
-                            int pad_norm_inf) {
+                            uint64_t nPad, Perm perm, unsigned char* __restrict__ out,
+                            float* __restrict__ norms) {
   const uint64_t chunks = (uint64_t) Kp / 8;
   const uint64_t total = nPad * chunks;
   for (uint64_t t = blockIdx.x * (uint64_t) blockDim.x + threadIdx.x; t < total;
@@ -77,9 +86,10 @@ __global__ void k_bf16_pack(const float* __restrict__ X, uint64_t n, int D, int 
     const uint32_t c = (uint32_t) (t % chunks);
     __align__(16) __nv_bfloat16 hi[8], lo[8];
     float part = 0.0f;
+    const uint64_t src = row < n ? (perm.mul == 1 ? row : perm(row)) : 0;
     for (int e = 0; e < 8; ++e) {
       const int k = (int) c * 8 + e;
-      const float v = (row < n && k < D) ? X[row * D + k] : 0.0f;
+      const float v = (row < n && k < D) ? X[src * D + k] : 0.0f;
       const __nv_bfloat16 h = __float2bfloat16_rn(v);
       const float r = v - __bfloat162float(h);
       hi[e] = h;
@@ -97,20 +107,27 @@ __global__ void k_bf16_pack(const float* __restrict__ X, uint64_t n, int D, int 
     // consecutive threads).
     atomicAdd(&norms[row], part);
   }
-  (void) maxnorm_ord;
-  (void) pad_norm_inf;
 }
 
+// B's norms: their maximum, and +inf for the padded rows, which then never win
+// a minimum.  The same launch starts A's row minima and candidate minima at
+// their largest.
 __global__ void k_bf16_norm_finish(float* __restrict__ norms, uint64_t n, uint64_t nPad,
-                                   uint32_t* __restrict__ maxnorm_ord, int pad_inf) {
+                                   uint32_t* __restrict__ maxnorm_ord,
+                                   uint32_t* __restrict__ rowmin, uint32_t* __restrict__ cand_min,
+                                   uint64_t nA) {
   uint32_t local = 0;
-  for (uint64_t i = blockIdx.x * (uint64_t) blockDim.x + threadIdx.x; i < nPad;
-       i += (uint64_t) gridDim.x * blockDim.x) {
-    if (i < n) {
+  const uint64_t t = blockIdx.x * (uint64_t) blockDim.x + threadIdx.x;
+  const uint64_t stride = (uint64_t) gridDim.x * blockDim.x;
+  for (uint64_t i = t; i < nPad; i += stride) {
+    if (i < n)
       local = max(local, f2ord(sqrtf(norms[i])));
-    } else if (pad_inf) {
-      norms[i] = INFINITY;  // padded B rows never win a minimum
-    }
+    else
+      norms[i] = INFINITY;
+  }
+  for (uint64_t i = t; i < nA; i += stride) {
+    rowmin[i] = 0xFFFFFFFFu;
+    cand_min[i] = 0xFFFFFFFFu;
   }
 #pragma unroll
   for (int o = 16; o; o >>= 1) local = max(local, __shfl_xor_sync(0xFFFFFFFFu, local, o));
@@ -224,18 +241,47 @@ __device__ __forceinline__ double row_bound(double a, double b, int K) {
   return 2.0 * e + 1e-30;
 }
 
+constexpr int kMaxRounds = 12;
+
 struct Bf16Scalars {
   uint32_t bmax_ord;   // max ||b|| (order-preserving bits)
-  uint32_t lo_ord;     // max_i (m_i - E_i) (order-preserving bits)
+  uint32_t lo_ord;     // L: max over completed rows of (m_i - E_i) (order-preserving bits)
   uint32_t cand;       // candidate count
   uint32_t status;
+  uint32_t live[kMaxRounds];   // rows still open after each round
+  uint32_t seeds[kMaxRounds];  // rows completed ahead of their turn after each round
+  float seed_level;            // rows with a partial minimum above it are taken as seeds
 };
+
+// Work of one rowmin launch: cnt rows in blocks of kAM against the tiles
+// [tile0, tile1) of B.  The launch is cut into items of (row block, part of
+// the tiles); one CTA runs on an SM at a time, so S parts take
+// ceil(blocks * S / SMs) turns of tiles / S tiles plus an item's fixed cost
+// (its 64 KB A block, barriers and TMEM: about kItemTiles tiles).  S is the
+// cheapest of 1 .. kMaxParts; blocks * S stays below kMaxTurns * SMs + blocks.
+constexpr uint32_t kItemTiles = 6;
+constexpr uint32_t kMaxParts = 32;
+constexpr uint32_t kMaxTurns = 4;
+__device__ __forceinline__ uint32_t tile_parts(uint32_t blocks, uint32_t tiles, uint32_t sms) {
+  uint32_t best = 1, cost = 0xFFFFFFFFu;
+  for (uint32_t p = 1; p <= min(kMaxParts, tiles); ++p) {
+    if ((uint64_t) (p - 1) * blocks >= kMaxTurns * sms) break;
+    const uint32_t turns = (blocks * p + sms - 1) / sms;
+    const uint32_t c = turns * ((tiles + p - 1) / p + kItemTiles);
+    if (c < cost) {
+      cost = c;
+      best = p;
+    }
+  }
+  return best;
+}
 
 template <int Kp>
 __global__ void __launch_bounds__(kThreads, 1)
     k_bf16_rowmin(const unsigned char* __restrict__ Apack, const unsigned char* __restrict__ Bpack,
-                  const float* __restrict__ anorm, const float* __restrict__ bnorm, uint64_t nA,
-                  uint32_t nTilesB, float* __restrict__ rowmin, Bf16Scalars* bs) {
+                  const float* __restrict__ bnorm, const uint32_t* __restrict__ list,
+                  const uint32_t* cnt_dev, uint32_t cnt_host, uint32_t tile0, uint32_t tile1,
+                  uint32_t sms, uint32_t* __restrict__ rowmin, Bf16Scalars* bs) {
   constexpr uint32_t kAReg = kBM * Kp * 2;   // bytes of one A region's hi (or lo) operand
   constexpr uint32_t kBReg = kBN * Kp * 2;   // bytes of one B tile's hi (or lo) operand
   constexpr uint32_t kABlock = 4 * kAReg;    // A block: (hi, lo) of region 0, then of region 1
@@ -251,6 +297,19 @@ __global__ void __launch_bounds__(kThreads, 1)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   unsigned char* sA = smem;
   unsigned char* sB = smem + kABlock;
+
+  // This CTA's item: all row blocks of one part of the tiles, then of the
+  // next, so that CTAs running together stream the same B tiles through L2.
+  const uint32_t cnt = cnt_dev ? *cnt_dev : cnt_host;
+  const uint32_t blocks = (cnt + kAM - 1) / kAM;
+  const uint32_t parts = tile_parts(blocks, tile1 - tile0, sms);
+  if (blocks == 0 || blockIdx.x >= (uint64_t) blocks * parts) return;
+  const uint32_t part = blockIdx.x / blocks, block = blockIdx.x - part * blocks;
+  const uint32_t len = tile1 - tile0;
+  const uint32_t first_tile = tile0 + (uint32_t) ((uint64_t) part * len / parts);
+  const uint32_t nTilesB = tile0 + (uint32_t) ((uint64_t) (part + 1) * len / parts) - first_tile;
+  Bpack += (uint64_t) first_tile * kBTile;
+  bnorm += (uint64_t) first_tile * kBN;
 
   if (threadIdx.x == 0) {
     mbar_init(&a_full, 1);
@@ -281,7 +340,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   if (warp == 0) {
     if (lane == 0) {
       mbar_expect_tx(&a_full, kABlock);
-      tma_load_1d(sA, Apack + (uint64_t) blockIdx.x * kABlock, kABlock, &a_full);
+      tma_load_1d(sA, Apack + (uint64_t) block * kABlock, kABlock, &a_full);
       for (uint32_t t = 0; t < nTilesB && ok; ++t) {
         const uint32_t st = t % kStages;
         if (t >= kStages) ok = mbar_wait(&b_empty[st], ((t / kStages) - 1) & 1, status, kWaitLimit);
@@ -390,20 +449,13 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
     }
     if (ok) {
-      const double bmax = (double) ord2f(bs->bmax_ord);
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
         float m = m8[r][0];
 #pragma unroll
         for (int q = 1; q < 8; ++q) m = fminf(m, m8[r][q]);
-        const uint64_t row = (uint64_t) blockIdx.x * kAM + (uint64_t) r * kBM + lrow;
-        if (row < nA) {
-          const float an = anorm[row];
-          const float mi = an + m;
-          rowmin[row] = mi;
-          const double E = row_bound(sqrt((double) an), bmax, Kp);
-          atomicMax(&bs->lo_ord, f2ord((float) ((double) mi - E)));
-        }
+        const uint32_t slot = block * kAM + (uint32_t) r * kBM + lrow;
+        if (slot < cnt) atomicMin(&rowmin[list ? list[slot] : slot], f2ord(m));
       }
     }
   }
@@ -419,18 +471,133 @@ __global__ void __launch_bounds__(kThreads, 1)
   }
 }
 
-__global__ void k_bf16_candidates(const float* __restrict__ rowmin, const float* __restrict__ anorm,
-                                  uint64_t nA, int Kp, Bf16Scalars* bs, uint32_t* __restrict__ list) {
+// A row's approximate nearest squared distance so far.
+__device__ __forceinline__ float row_value(uint32_t rowmin_ord, float anorm) {
+  return anorm + ord2f(rowmin_ord);
+}
+
+// L from the listed rows (list null: rows [0, cnt)), whose minima cover all
+// of B: every one of them bounds the result from below by m - E.
+__global__ void k_bf16_raise(const uint32_t* __restrict__ list, const uint32_t* cnt_dev,
+                             uint32_t cnt_host, const uint32_t* __restrict__ rowmin,
+                             const float* __restrict__ anorm, int Kp, Bf16Scalars* bs) {
+  const uint32_t cnt = cnt_dev ? *cnt_dev : cnt_host;
+  const double bmax = (double) ord2f(bs->bmax_ord);
+  uint32_t best = 0;
+  for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < cnt; e += gridDim.x * blockDim.x) {
+    const uint32_t row = list ? list[e] : e;
+    const float an = anorm[row];
+    const double E = row_bound(sqrt((double) an), bmax, Kp);
+    best = max(best, f2ord((float) ((double) row_value(rowmin[row], an) - E)));
+  }
+#pragma unroll
+  for (int o = 16; o; o >>= 1) best = max(best, __shfl_xor_sync(0xFFFFFFFFu, best, o));
+  if ((threadIdx.x & 31) == 0 && best) atomicMax(&bs->lo_ord, best);
+}
+
+// Rows of a list that can still reach L: m + E >= L, m over the tiles seen so
+// far.  A dropped row's FP32 distance is below that of a completed row, so it
+// cannot be the maximum.  A comparison with a NaN keeps the row.
+// final: all of B has been seen; the kept rows are the candidates of the
+// exact re-scan, and there the comparison has to hold.
+__global__ void k_bf16_keep(const uint32_t* __restrict__ list, const uint32_t* cnt_dev,
+                            uint32_t cnt_host, const uint32_t* __restrict__ rowmin,
+                            const float* __restrict__ anorm, int Kp, const Bf16Scalars* bs,
+                            bool final, uint32_t* __restrict__ out, uint32_t* out_cnt) {
+  const uint32_t cnt = cnt_dev ? *cnt_dev : cnt_host;
   const double L = (double) ord2f(bs->lo_ord);
   const double bmax = (double) ord2f(bs->bmax_ord);
-  for (uint64_t i = blockIdx.x * (uint64_t) blockDim.x + threadIdx.x; i < nA;
-       i += (uint64_t) gridDim.x * blockDim.x) {
-    const double E = row_bound(sqrt((double) anorm[i]), bmax, Kp);
-    if ((double) rowmin[i] + E >= L) {
-      const uint32_t s = atomicAdd(&bs->cand, 1u);
-      list[s] = (uint32_t) i;
+  const int lane = threadIdx.x & 31;
+  const uint32_t stride = gridDim.x * blockDim.x;
+  for (uint64_t e0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); e0 < cnt; e0 += stride) {
+    const uint64_t e = e0 + lane;
+    bool keep = false;
+    uint32_t row = 0;
+    if (e < cnt) {
+      row = list ? list[e] : (uint32_t) e;
+      const float an = anorm[row];
+      const double hi = (double) row_value(rowmin[row], an) + row_bound(sqrt((double) an), bmax, Kp);
+      keep = final ? hi >= L : !(hi < L);
+    }
+    const unsigned ballot = __ballot_sync(0xFFFFFFFFu, keep);
+    uint32_t base = 0;
+    if (lane == 0 && ballot) base = atomicAdd(out_cnt, (uint32_t) __popc(ballot));
+    base = __shfl_sync(0xFFFFFFFFu, base, 0);
+    if (keep) out[base + __popc(ballot & ((1u << lane) - 1u))] = row;
+  }
+}
+
+// The level that about `want` of the listed rows' partial minima exceed: the
+// (want / cnt)-quantile of 1,024 of them, spread over the list.
+__global__ void __launch_bounds__(1024)
+    k_bf16_seed_level(const uint32_t* __restrict__ list, const uint32_t* cnt_dev,
+                      uint32_t cnt_host, const uint32_t* __restrict__ rowmin,
+                      const float* __restrict__ anorm, uint32_t want, Bf16Scalars* bs) {
+  __shared__ float v[1024];
+  const uint32_t cnt = cnt_dev ? *cnt_dev : cnt_host;
+  const uint32_t n = min(cnt, 1024u), t = threadIdx.x;
+  float x = -INFINITY;
+  if (t < n) {
+    const uint32_t e = (uint32_t) ((uint64_t) t * cnt / n);
+    const uint32_t row = list ? list[e] : e;
+    x = row_value(rowmin[row], anorm[row]);
+  }
+  v[t] = x;
+  __syncthreads();
+  if (cnt <= want) {
+    if (t == 0) bs->seed_level = -INFINITY;
+    return;
+  }
+  const uint32_t rank = (uint32_t) ((uint64_t) want * n / cnt);  // < n
+  uint32_t above = 0;
+  for (uint32_t k = 0; k < n; ++k) above += v[k] > x || (v[k] == x && k < t);
+  if (t < n && above == rank) bs->seed_level = x;
+}
+
+// The rows above the level, at most cap of them.
+__global__ void k_bf16_seed_pick(const uint32_t* __restrict__ list, const uint32_t* cnt_dev,
+                                 uint32_t cnt_host, const uint32_t* __restrict__ rowmin,
+                                 const float* __restrict__ anorm, const Bf16Scalars* bs,
+                                 uint32_t cap, uint32_t* __restrict__ out, uint32_t* out_cnt) {
+  const uint32_t cnt = cnt_dev ? *cnt_dev : cnt_host;
+  const float level = bs->seed_level;
+  for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < cnt; e += gridDim.x * blockDim.x) {
+    const uint32_t row = list ? list[e] : e;
+    if (row_value(rowmin[row], anorm[row]) >= level && *(volatile uint32_t*) out_cnt < cap) {
+      const uint32_t s = atomicAdd(out_cnt, 1u);
+      if (s < cap) out[s] = row;
     }
   }
+}
+
+// A seed count may have run past the cap.
+__global__ void k_bf16_seed_clamp(uint32_t* cnt, uint32_t cap) { *cnt = min(*cnt, cap); }
+
+// The listed rows' packed operands, copied together in 16-byte pieces into
+// row blocks of the same layout.  Slots of the last block past the count keep
+// whatever they held: their accumulators are never read.
+__global__ void k_bf16_gather(const uint32_t* __restrict__ list, const uint32_t* cnt_dev, int Kp,
+                              const unsigned char* __restrict__ src,
+                              unsigned char* __restrict__ dst) {
+  const uint32_t per = (uint32_t) Kp / 4;  // pieces per row: Kp / 8 chunks, hi and lo
+  const uint64_t total = (uint64_t) *cnt_dev * per;
+  const uint64_t reg = (uint64_t) 2 * kBM * Kp * 2;
+  for (uint64_t t = blockIdx.x * (uint64_t) blockDim.x + threadIdx.x; t < total;
+       t += (uint64_t) gridDim.x * blockDim.x) {
+    const uint32_t slot = (uint32_t) (t / per), q = (uint32_t) (t % per);
+    const uint32_t half = q & 1, c = q >> 1, row = list[slot];
+    const uint64_t in = row / kBM * reg + (uint64_t) half * kBM * Kp * 2 + pack_off(row % kBM, c * 8, kBM);
+    const uint64_t out = slot / kBM * reg + (uint64_t) half * kBM * Kp * 2 + pack_off(slot % kBM, c * 8, kBM);
+    *reinterpret_cast<uint4*>(dst + out) = *reinterpret_cast<const uint4*>(src + in);
+  }
+}
+
+// Row minima as floats (the test hook's output).
+__global__ void k_bf16_values(uint32_t* __restrict__ rowmin, const float* __restrict__ anorm,
+                              uint64_t n) {
+  for (uint64_t i = blockIdx.x * (uint64_t) blockDim.x + threadIdx.x; i < n;
+       i += (uint64_t) gridDim.x * blockDim.x)
+    rowmin[i] = __float_as_uint(row_value(rowmin[i], anorm[i]));
 }
 
 // Exact FP32 re-scan of the candidate rows with the reference formula: every
@@ -491,47 +658,149 @@ __global__ void k_bf16_recheck_final(const uint32_t* __restrict__ list, const Bf
     atomicMax(&sc->max_key, pack_max(__uint_as_float(cand_min[e]), list[e]));
 }
 
+// Rounds over B.  With one round every row meets every tile.  With several,
+// B is packed in a pseudo-random order and cut into runs of tiles that grow
+// by kGrowth; after each run the rows that can no longer reach L are dropped
+// and the rest are packed together for the next run, and the rows with the
+// largest partial minima are completed at once to raise L (early break, as
+// the reference's scan has it, at the grain of tensor tiles).
+// Measured, 64-D unit rows, undirected (1M x 1M; 250k x 250k), before the
+// first run's floor of 48 tiles: growth 1.6 and 1/128 seeds 87 and 7.9 ms; 1/64
+// seeds 101 and 8.9; 1/256 83 and 8.4; growth 2.0 with 1/256 95 and 9.1; 1.4
+// with 1/64 108 and 10.0.  A round costs about ten launches and an uneven last
+// turn of items: 32,000 x 32,000 took 0.72 ms with rounds and 0.70 without,
+// 50,000 x 50,000 1.25 and 1.31 ms, so rounds start between the two.
+constexpr double kGrowth = 1.6;
+constexpr uint32_t kFirstDiv = 32;       // the first run is 1/32 of the tiles
+constexpr uint32_t kFirstTiles = 48;     // but at least this many
+constexpr double kRoundPairs = 2e9;      // several rounds from this |A| * |B| up
+constexpr uint32_t kSeedDiv = 128;       // seeds after a round: 1/128 of A's rows at most
+
+int bf16_rounds(uint64_t nA, uint64_t nB, uint32_t tiles, uint32_t* ends) {
+  int r = 0;
+  if ((double) nA * (double) nB >= kRoundPairs) {
+    double step = std::max(kFirstTiles, tiles / kFirstDiv);
+    for (double end = step; r < kMaxRounds - 1 && end * kGrowth < tiles; ++r) {
+      ends[r] = (uint32_t) end;
+      end = std::floor(end * kGrowth);
+    }
+  }
+  ends[r++] = tiles;
+  return r;
+}
+
 template <int Kp>
 hd_status run_bf16_k(Ctx& c, const DirInput& in, DirResult* extra, float* rowmin_host) {
   hd_status s;
   const uint64_t nCta = (in.nA + kAM - 1) / kAM, nTB = (in.nB + kBN - 1) / kBN;
   if (nCta >= (1u << 31) || nTB >= 0xFFFFFFFFull) return fail(c, HD_ERR_INVALID_ARG, "too large");
   const uint64_t padA = nCta * kAM, padB = nTB * kBN;
-  void *pa, *pb, *na, *nb, *rm, *cand, *bsv;
+  void *pa, *pb, *zeroed, *rm, *cand;
   if ((s = ensure(c, kBufBf16A, padA * Kp * 4, &pa)) != HD_OK) return s;
   if ((s = ensure(c, kBufBf16B, padB * Kp * 4, &pb)) != HD_OK) return s;
-  if ((s = ensure(c, kBufNormsA, padA * 4, &na)) != HD_OK) return s;
-  if ((s = ensure(c, kBufNormsB, padB * 4, &nb)) != HD_OK) return s;
-  if ((s = ensure(c, kBufRowMin, padA * 4, &rm)) != HD_OK) return s;
+  // What has to start at zero lies together: the scalars and both norms.
+  const size_t zero_bytes = 256 + (padA + padB) * 4;
+  static_assert(sizeof(Bf16Scalars) <= 256, "scalars");
+  if ((s = ensure(c, kBufNorms, zero_bytes, &zeroed)) != HD_OK) return s;
+  Bf16Scalars* bs = (Bf16Scalars*) zeroed;
+  float* na = (float*) ((char*) zeroed + 256);
+  float* nb = na + padA;
+  if ((s = ensure(c, kBufRowMin, in.nA * 4, &rm)) != HD_OK) return s;
   if ((s = ensure(c, kBufCand, in.nA * 8 + 128, &cand)) != HD_OK) return s;
-  if ((s = ensure(c, kBufAux2, sizeof(Bf16Scalars), &bsv)) != HD_OK) return s;
-  Bf16Scalars* bs = (Bf16Scalars*) bsv;
+  // Candidate minima live after the candidate list (one uint per row of A).
+  uint32_t* cand_min = (uint32_t*) cand + in.nA + 16;
+  uint32_t ends[kMaxRounds];
+  int rounds = rowmin_host ? 1 : bf16_rounds(in.nA, in.nB, (uint32_t) nTB, ends);
+  // Several rounds keep the open rows packed together (as many as A has, less
+  // those dropped after the first run), the seeds, and their lists; where the
+  // device has no room for that, one round does the work.
+  const uint32_t seed_cap = (uint32_t) std::max<uint64_t>(kAM, in.nA / kSeedDiv / kAM * kAM);
+  void *open_pack = nullptr, *open_list = nullptr;
+  if (rounds > 1) {
+    const std::string before = c.last_error;
+    if (ensure(c, kBufBf16Open, (padA + seed_cap) * Kp * 4, &open_pack) != HD_OK ||
+        ensure(c, kBufKeys, (2 * in.nA + seed_cap) * 4, &open_list) != HD_OK) {
+      c.last_error = before;
+      rounds = 1;
+    }
+  }
+  if (rounds == 1) ends[0] = (uint32_t) nTB;
   cudaError_t e;
-  if ((e = cudaMemsetAsync(na, 0, padA * 4, c.stream)) != cudaSuccess) return cuda_fail(c, e, "memset");
-  if ((e = cudaMemsetAsync(nb, 0, padB * 4, c.stream)) != cudaSuccess) return cuda_fail(c, e, "memset");
-  if ((e = cudaMemsetAsync(bs, 0, sizeof(Bf16Scalars), c.stream)) != cudaSuccess)
+  if ((e = cudaMemsetAsync(zeroed, 0, zero_bytes, c.stream)) != cudaSuccess)
     return cuda_fail(c, e, "memset");
   const int g = c.num_sms * 16;
-  k_bf16_pack<<<g, 256, 0, c.stream>>>(in.A, in.nA, in.dims, Kp, kBM, padA, (unsigned char*) pa,
-                                       (float*) na, nullptr, 0);
+  const Perm same_a{in.nA, 1, 0};
+  const Perm order_b{in.nB, rounds > 1 ? pick_multiplier(in.nB, c.opt.seed + 1) : 1, 0};
+  k_bf16_pack<<<g, 256, 0, c.stream>>>(in.A, in.nA, in.dims, Kp, kBM, padA, same_a,
+                                       (unsigned char*) pa, na);
   if ((s = after_launch(c, "bf16_pack_a")) != HD_OK) return s;
-  k_bf16_pack<<<g, 256, 0, c.stream>>>(in.B, in.nB, in.dims, Kp, kBN, padB, (unsigned char*) pb,
-                                       (float*) nb, nullptr, 0);
+  k_bf16_pack<<<g, 256, 0, c.stream>>>(in.B, in.nB, in.dims, Kp, kBN, padB, order_b,
+                                       (unsigned char*) pb, nb);
   if ((s = after_launch(c, "bf16_pack_b")) != HD_OK) return s;
   // A's norm maximum is not needed; B's gives the bound.
-  k_bf16_norm_finish<<<c.num_sms * 4, 256, 0, c.stream>>>((float*) nb, in.nB, padB, &bs->bmax_ord, 1);
+  k_bf16_norm_finish<<<c.num_sms * 4, 256, 0, c.stream>>>(nb, in.nB, padB, &bs->bmax_ord,
+                                                          (uint32_t*) rm, cand_min, in.nA);
   if ((s = after_launch(c, "bf16_norms")) != HD_OK) return s;
   mark(c, 1);
   mark(c, 2);
   mark(c, 3);
   auto kern = k_bf16_rowmin<Kp>;
   cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) kSmemBytes);
-  kern<<<(unsigned) nCta, kThreads, kSmemBytes, c.stream>>>(
-      (const unsigned char*) pa, (const unsigned char*) pb, (const float*) na, (const float*) nb,
-      in.nA, (uint32_t) nTB, (float*) rm, bs);
-  if ((s = after_launch(c, "bf16_rowmin")) != HD_OK) return s;
+  uint32_t* rowmin = (uint32_t*) rm;
+  const float* an = na;
+  const uint32_t nA32 = (uint32_t) in.nA;
+  const uint32_t sms = (uint32_t) c.num_sms;
+  // A launch over at most `most` rows: as many CTAs as the device may find
+  // items; those without one return at once.
+  auto scan = [&](const void* pack, const uint32_t* list, const uint32_t* cnt, uint64_t most,
+                  uint32_t t0, uint32_t t1) -> hd_status {
+    const uint64_t blocks = (most + kAM - 1) / kAM;
+    const unsigned grid = (unsigned) std::min<uint64_t>(blocks * std::min(kMaxParts, t1 - t0),
+                                                        blocks + (uint64_t) kMaxTurns * sms);
+    kern<<<grid, kThreads, kSmemBytes, c.stream>>>((const unsigned char*) pack,
+                                                   (const unsigned char*) pb, nb,
+                                                   list, cnt, (uint32_t) most, t0, t1, sms,
+                                                   rowmin, bs);
+    return after_launch(c, "bf16_rowmin");
+  };
+  unsigned char* seed_pack = (unsigned char*) open_pack + (rounds > 1 ? padA * Kp * 4 : 0);
+  uint32_t* lists[2] = {(uint32_t*) open_list, (uint32_t*) open_list + (rounds > 1 ? in.nA : 0)};
+  uint32_t* seed_list = (uint32_t*) open_list + (rounds > 1 ? 2 * in.nA : 0);
+  const void* pack = pa;            // the open rows' operands,
+  const uint32_t* list = nullptr;   // their row numbers (null: all rows in order)
+  const uint32_t* cnt = nullptr;    // and their count
+  uint32_t t0 = 0;
+  for (int r = 0; r < rounds; ++r) {
+    if ((s = scan(pack, list, cnt, in.nA, t0, ends[r])) != HD_OK) return s;
+    t0 = ends[r];
+    if (r == rounds - 1) break;
+    uint32_t* seeds = &bs->seeds[r];
+    k_bf16_seed_level<<<1, 1024, 0, c.stream>>>(list, cnt, nA32, rowmin, an, seed_cap, bs);
+    k_bf16_seed_pick<<<c.num_sms * 4, 256, 0, c.stream>>>(list, cnt, nA32, rowmin, an, bs, seed_cap,
+                                                          seed_list, seeds);
+    k_bf16_seed_clamp<<<1, 1, 0, c.stream>>>(seeds, seed_cap);
+    k_bf16_gather<<<c.num_sms * 4, 256, 0, c.stream>>>(seed_list, seeds, Kp,
+                                                       (const unsigned char*) pa, seed_pack);
+    c.launches += 3;
+    if ((s = after_launch(c, "bf16_seeds")) != HD_OK) return s;
+    if ((s = scan(seed_pack, seed_list, seeds, seed_cap, t0, (uint32_t) nTB)) != HD_OK) return s;
+    k_bf16_raise<<<c.num_sms, 256, 0, c.stream>>>(seed_list, seeds, 0, rowmin, an, Kp, bs);
+    if ((s = after_launch(c, "bf16_raise")) != HD_OK) return s;
+    uint32_t* kept = lists[r & 1];
+    k_bf16_keep<<<c.num_sms * 4, 256, 0, c.stream>>>(list, cnt, nA32, rowmin, an, Kp, bs, false,
+                                                     kept, &bs->live[r]);
+    if ((s = after_launch(c, "bf16_keep")) != HD_OK) return s;
+    list = kept;
+    cnt = &bs->live[r];
+    k_bf16_gather<<<c.num_sms * 8, 256, 0, c.stream>>>(list, cnt, Kp, (const unsigned char*) pa,
+                                                       (unsigned char*) open_pack);
+    if ((s = after_launch(c, "bf16_gather")) != HD_OK) return s;
+    pack = open_pack;
+  }
   mark(c, 4);
   if (rowmin_host) {
+    k_bf16_values<<<c.num_sms * 4, 256, 0, c.stream>>>(rowmin, an, in.nA);
+    if ((s = after_launch(c, "bf16_values")) != HD_OK) return s;
     e = cudaMemcpyAsync(rowmin_host, rm, in.nA * 4, cudaMemcpyDeviceToHost, c.stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c.stream);
     if (e != cudaSuccess) return cuda_fail(c, e, "rowmin copy");
@@ -541,14 +810,12 @@ hd_status run_bf16_k(Ctx& c, const DirInput& in, DirResult* extra, float* rowmin
     if (h.status) return fail(c, HD_ERR_DEVICE_TIMEOUT, "a bounded device wait ran out");
     return HD_OK;
   }
-  k_bf16_candidates<<<c.num_sms * 4, 256, 0, c.stream>>>((const float*) rm, (const float*) na, in.nA,
-                                                         Kp, bs, (uint32_t*) cand);
+  k_bf16_raise<<<c.num_sms * 2, 256, 0, c.stream>>>(list, cnt, nA32, rowmin, an, Kp, bs);
+  if ((s = after_launch(c, "bf16_raise")) != HD_OK) return s;
+  k_bf16_keep<<<c.num_sms * 4, 256, 0, c.stream>>>(list, cnt, nA32, rowmin, an, Kp, bs, true,
+                                                   (uint32_t*) cand, &bs->cand);
   if ((s = after_launch(c, "bf16_candidates")) != HD_OK) return s;
   DevScalars* sc = scalars(c, in.dir);
-  // Candidate minima live after the candidate list (one uint per row of A).
-  uint32_t* cand_min = (uint32_t*) cand + in.nA + 16;
-  if ((e = cudaMemsetAsync(cand_min, 0xFF, in.nA * 4, c.stream)) != cudaSuccess)
-    return cuda_fail(c, e, "memset");
   k_bf16_recheck<<<dim3(c.num_sms * 2, 16), 256, 0, c.stream>>>(in.A, in.B, in.nB, in.dims,
                                                                (const uint32_t*) cand, bs, cand_min);
   if ((s = after_launch(c, "bf16_recheck")) != HD_OK) return s;
@@ -567,6 +834,16 @@ hd_status run_bf16_k(Ctx& c, const DirInput& in, DirResult* extra, float* rowmin
   }
   if (extra) {
     extra->rechecked = h.cand;
+    if (in.count) {
+      uint64_t open = in.nA;
+      for (int r = 0; r < rounds; ++r) {
+        const uint32_t begin = r ? ends[r - 1] : 0;
+        extra->pairs += open * (uint64_t) (ends[r] - begin) * kBN;
+        if (r == rounds - 1) break;
+        extra->pairs += (uint64_t) h.seeds[r] * (nTB - ends[r]) * kBN;
+        open = h.live[r];
+      }
+    }
     // Report the bound of the largest-norm pair (||a|| ~ ||b|| ~ max ||b||).
     const double b = (double) ord2f(h.bmax_ord);
     const double cK = 4.0 * std::ldexp(1.0, -18) + (3.0 * Kp + 16.0) * std::ldexp(1.0, -23);

@@ -610,7 +610,7 @@ hd_status hd_solve(hd_ctx* c, const float* A, uint64_t n_a, const float* B,
   out->direction = win;
   out->ia = w.ia;
   out->ib = w.ib;
-  out->visited_pairs = r0.pairs + (undirected ? h->s[1].pairs : 0);
+  out->visited_pairs = r0.pairs + (undirected ? h->s[1].pairs : 0) + ex[0].pairs + ex[1].pairs;
   out->visited_nodes = r0.nodes + (undirected ? h->s[1].nodes : 0);
   out->visited_leaves = r0.leaves + (undirected ? h->s[1].leaves : 0);
   out->variant_used = used[0];

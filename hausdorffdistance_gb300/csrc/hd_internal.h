@@ -80,8 +80,8 @@ enum BufSlot {
   kBufSample,
   kBufBf16A,      // split-BF16 operands
   kBufBf16B,
-  kBufNormsA,
-  kBufNormsB,
+  kBufBf16Open,   // the rows still open after a round, packed together, and the seeds
+  kBufNorms,      // BF16 scalars and the squared norms of both sets
   kBufRowMin,
   kBufCand,
   kBufBatch,

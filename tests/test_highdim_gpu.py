@@ -85,3 +85,32 @@ def test_bf16_rejects_unsupported_dims(engine):
     with pytest.raises(hd.HDError) as ei:
         engine.solve(a, a, variant="bf16")
     assert ei.value.status == 5
+
+
+# Runs of tiles with rows dropped between them (|A| * |B| >= 2e9): fewer rows
+# than one seed block, a ragged last row block and tile, B far from A (no row
+# drops out early), exact copies (every early seed may be one), one repeated
+# point (every row ties, none can be dropped).
+@pytest.mark.parametrize("na,nb,dims,kind", [
+    (200, 10_000_019, 16, "gauss"), (45_000, 44_501, 64, "copies"), (50_001, 40_003, 48, "far"),
+    (70_000, 30_000, 32, "repeated"), (2_000_003, 1025, 16, "gauss")])
+def test_bf16_runs_of_tiles(engine, na, nb, dims, kind):
+    rng = np.random.default_rng(na + dims)
+    a = rng.standard_normal((na, dims), dtype=np.float32)
+    if kind == "copies":
+        b = a[rng.permutation(na)[:nb]].copy()
+        b[::100] = rng.standard_normal(b[::100].shape, dtype=np.float32)
+    elif kind == "repeated":
+        a[:] = a[0]
+        b = np.repeat(a[:1] + np.float32(0.5), nb, axis=0)
+    else:
+        b = rng.standard_normal((nb, dims), dtype=np.float32)
+        if kind == "far":
+            b += np.float32(10.0)
+    r = engine.solve(a, b, variant="bf16")
+    if kind == "repeated":
+        d2 = hd_oracle.dist2_f32(a[0], b[0])
+    else:
+        d2 = hd_oracle.exact(a, b, 32)[0]
+    assert np.float32(r.hd_f32) == np.sqrt(np.float32(d2))
+    assert hd_oracle.dist2_f32(a[r.ia], b[r.ib]) == np.float32(d2)
