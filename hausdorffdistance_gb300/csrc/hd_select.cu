@@ -9,7 +9,7 @@
 //   1. Eight points of A get their exact nearest-neighbour distance (one
 //      grid-wide scan of B) and seed the running maximum.  Then k further
 //      points of A (k = sample_rate * |A|, clamped to [64, 256]) run the
-//      early-break scan against B, one warp each, B visited in a
+//      early-break scan against B, one CTA each, B visited in a
 //      pseudo-random order, counting the B points each visited before it
 //      stopped (in rounds of 64, capped at 16,384).  Seeds and completed samples also seed the running maximum
 //      that the chosen variant starts from.
@@ -66,52 +66,69 @@ namespace {
 
 constexpr uint32_t kSampleCap = 16384;
 
-// Sampled early-break scans: one warp per sampled point of A, B visited in
-// a pseudo-random order, 64 B points per round (two per lane), a warp vote
-// after every round; the count of B points visited before the point stopped
-// (or the cap) is its statistic.
+// Sampled early-break scans: one CTA per sampled point of A, B visited in a
+// pseudo-random order in rounds of 64 points; the statistic is the count of B
+// points visited when a round first brings the point's minimum to or below the
+// running maximum (or the cap).  A step takes 32 rounds at once, 8 points per
+// thread with their loads in flight together, and finds the first such round
+// among them: a round is a chain of two memory latencies, and taking them one
+// by one cost 300 us per direction for samples that reach the cap of 256
+// rounds (now 24 us).
+constexpr int kSampleStep = 2048;
+
 __global__ void __launch_bounds__(256)
     k_sample_eb(const float* __restrict__ A, Perm pA, uint32_t k, const float* __restrict__ B,
                 Perm pB, uint64_t nB, int dims, uint32_t cap, DevScalars* sc,
                 uint32_t* __restrict__ iters) {
-  const uint32_t e = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (e >= k) return;
+  __shared__ uint32_t s_round;  // first round of the step with a point within the maximum
+  __shared__ float s_thr;
+  __shared__ uint32_t s_min;    // float bits of the smallest distance so far
+  const uint32_t e = blockIdx.x;
   const uint32_t ia = (uint32_t) pA(e);
   const float a0 = A[(uint64_t) ia * dims], a1 = A[(uint64_t) ia * dims + 1];
   const float a2 = dims == 3 ? A[(uint64_t) ia * dims + 2] : 0.0f;
-  float cmin = INFINITY;
   const uint64_t limit = min((uint64_t) cap, nB);
+  if (threadIdx.x == 0) s_min = 0x7F800000u;
   uint64_t done = 0;
   bool broke = false;
-  unsigned long long key = 0;
-  while (done < limit) {
-    const uint64_t end = min(limit, done + 64);
+  while (done < limit && !broke) {
+    if (threadIdx.x == 0) {
+      s_round = 0xFFFFFFFFu;
+      s_thr = threshold_of(ld_relaxed_u64(&sc->max_key));
+    }
+    __syncthreads();
+    float d[8];
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      const uint64_t j = done + lane + 32 * u;
-      if (j < end) {
+    for (int u = 0; u < 8; ++u) {
+      const uint64_t j = done + u * 256 + threadIdx.x;
+      d[u] = INFINITY;
+      if (j < limit) {
         const uint64_t b = pB(j);
-        const float d = dims == 2 ? d2_2(a0, a1, B[2 * b], B[2 * b + 1])
-                                  : d2_3(a0, a1, a2, B[3 * b], B[3 * b + 1], B[3 * b + 2]);
-        cmin = fminf(cmin, d);
+        d[u] = dims == 2 ? d2_2(a0, a1, B[2 * b], B[2 * b + 1])
+                         : d2_3(a0, a1, a2, B[3 * b], B[3 * b + 1], B[3 * b + 2]);
       }
     }
-    done = end;
-    float m = cmin;
+    float m = INFINITY;
+    uint32_t first = 0xFFFFFFFFu;
 #pragma unroll
-    for (int o = 16; o; o >>= 1) m = fminf(m, __shfl_xor_sync(0xFFFFFFFFu, m, o));
-    cmin = m;
-    if (lane == 0) key = ld_relaxed_u64(&sc->max_key);
-    if (cmin <= threshold_of(__shfl_sync(0xFFFFFFFFu, key, 0))) {
-      broke = true;
-      break;
+    for (int u = 7; u >= 0; --u) {
+      m = fminf(m, d[u]);
+      if (d[u] <= s_thr) first = (u * 256 + threadIdx.x) / 64;
     }
+    if (first != 0xFFFFFFFFu) atomicMin(&s_round, first);
+    // A minimum kept from the steps before may be within a maximum that rose.
+    if (threadIdx.x == 0 && __uint_as_float(s_min) <= s_thr) atomicMin(&s_round, 0u);
+    __syncthreads();
+    atomicMin(&s_min, __float_as_uint(m));
+    broke = s_round != 0xFFFFFFFFu;
+    done = broke ? min(limit, done + (uint64_t) (s_round + 1) * 64)
+                 : min(limit, done + (uint64_t) kSampleStep);
+    __syncthreads();
   }
-  if (lane == 0) {
+  if (threadIdx.x == 0) {
     iters[e] = (uint32_t) done;
     // A sample that scanned all of B without stopping has its exact minimum.
-    if (!broke && done == nB) atomicMax(&sc->max_key, pack_max(cmin, ia));
+    if (!broke && done == nB) atomicMax(&sc->max_key, pack_max(__uint_as_float(s_min), ia));
   }
 }
 
@@ -308,7 +325,7 @@ hd_status select_variants(Ctx& c, const DirInput* ins, int ndir, int* v) {
       k_seed_finish<<<1, 32, 0, c.stream>>>(pA, k[d], seed_min, sc);
       if ((s = after_launch(c, "seed_finish")) != HD_OK) return s;
     }
-    k_sample_eb<<<(k[d] * 32 + 255) / 256, 256, 0, c.stream>>>(
+    k_sample_eb<<<k[d], 256, 0, c.stream>>>(
         in.A, pA, k[d], in.B, pB, in.nB, in.dims, kSampleCap, sc, w + o_it[d]);
     if ((s = after_launch(c, "sample_eb")) != HD_OK) return s;
     c.seeded[in.dir] = in.nA > k[d];
