@@ -130,6 +130,22 @@ struct Perm {
   }
 };
 
+// The FP64 input path's listing pass stops a row only below soft_stop(thr):
+// a lower bound, from the running maximum thr alone, of the threshold under
+// which an FP32 distance proves an FP64 distance below the final answer's
+// seed (the bound is derived in hd_f64.cu; every step here rounds toward
+// zero, r = how far a cut pair's distance can move).  -1: no row stops.
+__device__ __forceinline__ float soft_stop(float thr, float r) {
+  if (!(thr >= 0.0f)) return -1.0f;
+  const float abs32 = 5.0f * 0x1p-126f;  // (n_dims + 2) 2^-126, n_dims <= 3
+  const float base = __fsub_rd(thr, abs32);
+  if (!(base > 0.0f)) return -1.0f;
+  const float sg = __fsub_rd(__fmul_rd(__fsqrt_rd(base), 0.99999f), __fmul_ru(2.01f, r));
+  if (!(sg > 0.0f)) return -1.0f;
+  const float g = __fsub_rd(__fmul_rd(__fmul_rd(sg, sg), 0.999999f), abs32);
+  return g > 0.0f ? g : -1.0f;
+}
+
 // Error bits written to the context's device status word.
 enum : uint32_t {
   kErrWaitTimeout = 1u,   // an mbarrier / flag wait hit its iteration cap

@@ -57,6 +57,17 @@ hd_status ensure(Ctx& c, BufSlot slot, size_t bytes, void** out) {
     if (e != cudaSuccess) {
       (void) cudaGetLastError();
       e = cudaMalloc(&b.p, bytes);
+      DevBuf& filter = c.bufs[kBufCells];
+      if (e != cudaSuccess && slot != kBufCells && !c.cells_live && filter.p) {
+        // The cell filter's bitmaps and lists are not needed any more: their
+        // room goes to the index.
+        (void) cudaGetLastError();
+        if ((e = cudaStreamSynchronize(c.stream)) != cudaSuccess)
+          return cuda_fail(c, e, "sync before realloc");
+        cudaFree(filter.p);
+        filter = DevBuf{};
+        e = cudaMalloc(&b.p, bytes);
+      }
       if (e != cudaSuccess) {
         (void) cudaGetLastError();
         b.p = nullptr;
@@ -135,8 +146,8 @@ __global__ void k_init_scalars(DevScalars* sc, int n) {
 __global__ void k_argmin(const float* __restrict__ A, const float* __restrict__ B,
                          uint64_t nB, int D, DevScalars* sc) {
   const unsigned long long key = sc->max_key;
-  if (key == 0) return;
   const uint32_t ia = unpack_max_index(key);
+  if (key == 0 || ia == kInvalid) return;  // no row has completed
   float a[4] = {0, 0, 0, 0};
   const bool small = D <= 4;
   const bool vec = D > 4 && (D % 4) == 0 && ((reinterpret_cast<uintptr_t>(A) & 15) == 0) &&
@@ -216,27 +227,7 @@ __global__ void k_argmin(const float* __restrict__ A, const float* __restrict__ 
 
 __global__ void k_finalize(const float* __restrict__ A, const float* __restrict__ B,
                            int D, DevScalars* sc) {
-  const unsigned long long key = sc->max_key;
-  if (key == 0) {
-    sc->status |= kErrInternal;
-    return;
-  }
-  const uint32_t ia = unpack_max_index(key);
-  const uint32_t d2bits = (uint32_t) (key >> 32);
-  const unsigned long long mk = sc->min_key;
-  const uint32_t ib = (uint32_t) (mk & 0xFFFFFFFFull);
-  // The argmin over B of A[ia] must reproduce the maximum exactly: it is the
-  // same FP32 formula over the same coordinates.
-  if ((uint32_t) (mk >> 32) != d2bits) sc->status |= kErrInternal;
-  double s = 0.0;
-  for (int k = 0; k < D; ++k) {
-    double t = (double) A[(uint64_t) ia * D + k] - (double) B[(uint64_t) ib * D + k];
-    s += t * t;
-  }
-  sc->d2_64 = s;
-  sc->d2 = __uint_as_float(d2bits);
-  sc->ia = ia;
-  sc->ib = ib;
+  finalize_scalars(A, B, D, sc);
 }
 
 }  // namespace
@@ -247,6 +238,47 @@ hd_status certify(Ctx& c, const DirInput& in) {
   int grid = (int) std::min<uint64_t>((in.nB + 255) / 256, (uint64_t) c.num_sms * 4);
   grid = std::max(grid, 1);
   k_argmin<<<grid, 256, 0, c.stream>>>(in.A, in.B, in.nB, in.dims, sc);
+  hd_status s = after_launch(c, "argmin");
+  if (s != HD_OK) return s;
+  k_finalize<<<1, 1, 0, c.stream>>>(in.A, in.B, in.dims, sc);
+  return after_launch(c, "finalize");
+}
+
+namespace {
+
+// The same argmin over the cell filter's targets (x, y, z, row).
+template <int D>
+__global__ void k_argmin_left(const float* __restrict__ A, const float4* __restrict__ T, uint32_t n,
+                              DevScalars* sc) {
+  const unsigned long long key = sc->max_key;
+  if (key == 0 || unpack_max_index(key) == kInvalid) return;  // no row has completed
+  const float* q = A + (uint64_t) unpack_max_index(key) * D;
+  const float4 a = make_float4(q[0], q[1], D == 3 ? q[2] : 0.0f, 0.0f);
+  unsigned long long best = ~0ull;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const float4 t = T[i];
+    const unsigned long long k = pack_min(d2_pt<D>(a, t), __float_as_uint(t.w));
+    best = k < best ? k : best;
+  }
+#pragma unroll
+  for (int o = 16; o; o >>= 1) {
+    unsigned long long v = __shfl_xor_sync(0xFFFFFFFFu, best, o);
+    best = v < best ? v : best;
+  }
+  if ((threadIdx.x & 31) == 0 && best != ~0ull) atomicMin(&sc->min_key, best);
+}
+
+}  // namespace
+
+hd_status certify_left(Ctx& c, const DirInput& in, const CellsLeft& left) {
+  mark(c, 5);
+  DevScalars* sc = scalars(c, in.dir);
+  const int grid = (int) std::max<uint64_t>(
+      1, std::min<uint64_t>((left.nt + 255) / 256, (uint64_t) c.num_sms * 4));
+  if (in.dims == 2)
+    k_argmin_left<2><<<grid, 256, 0, c.stream>>>(in.A, left.t, (uint32_t) left.nt, sc);
+  else
+    k_argmin_left<3><<<grid, 256, 0, c.stream>>>(in.A, left.t, (uint32_t) left.nt, sc);
   hd_status s = after_launch(c, "argmin");
   if (s != HD_OK) return s;
   k_finalize<<<1, 1, 0, c.stream>>>(in.A, in.B, in.dims, sc);
@@ -422,6 +454,8 @@ hd_status hd_destroy(hd_ctx* c) {
   if (c->batch_side) cudaStreamDestroy(c->batch_side);
   if (c->host_pinned) cudaFreeHost(c->host_pinned);
   if (c->sel_pinned) cudaFreeHost(c->sel_pinned);
+  if (c->sel_event) cudaEventDestroy(c->sel_event);
+  if (c->cells_event) cudaEventDestroy(c->cells_event);
   if (c->batch_pinned) cudaFreeHost(c->batch_pinned);
   if (c->own_stream) cudaStreamDestroy(c->own_stream);
   delete c;
@@ -460,6 +494,8 @@ hd_status hd_solve(hd_ctx* c, const float* A, uint64_t n_a, const float* B,
   out->hd_ba = -1.0;
   c->timing = (flags & HD_TIMING) != 0;
   c->sorted_valid = false;
+  c->boxes_known = false;
+  c->cells_live = false;
   c->ev_base = 0;
   c->last_p80[0] = c->last_p80[1] = 0.0;
   c->last_mean[0] = c->last_mean[1] = 0.0;
@@ -482,7 +518,7 @@ hd_status hd_solve(hd_ctx* c, const float* A, uint64_t n_a, const float* B,
       known = select_variant_by_size(*c, n_a, n_b, n_dims, &v0) &&
               select_variant_by_size(*c, n_b, n_a, n_dims, &v1);
     if (undirected && known && v0 == HD_VARIANT_LBVH && v1 == HD_VARIANT_LBVH &&
-        n_a + n_b >= kSplitMinPoints) {
+        n_a + n_b >= kSplitMinPoints && !cells_apply(*c, n_a, n_b, n_dims)) {
       if ((s = spatial_upload_sort(*c, A, n_a, B, n_b, n_dims, &dA, &dB)) != HD_OK) return s;
     } else {
       if ((s = copy_in(*c, A, n_a, n_dims, kBufA, &dA)) != HD_OK) return s;
@@ -499,21 +535,107 @@ hd_status hd_solve(hd_ctx* c, const float* A, uint64_t n_a, const float* B,
                       d == 0 ? n_b : n_a, n_dims, d, count};
     used[d] = variant;
   }
+  // The cell filter runs before the indexes (not before an early-break scan,
+  // which eb_only_threshold may ask for).  It does not wait for the selector:
+  // its kernels follow the sample's, and the host evaluates the sample while
+  // they run.
+  bool cells = cells_apply(*c, n_a, n_b, n_dims) &&
+               (variant == HD_VARIANT_LBVH ||
+                (variant == HD_VARIANT_AUTO && c->opt.eb_only_threshold == 0));
+  bool have_result = false;  // the scalars are already in the pinned staging
+  CellsRun cells_state;
+  const int level = cells_level(n_a + n_b, n_dims);
+  auto filter = [&]() -> hd_status {
+    mark(*c, 0);
+    const hd_status r = cells_begin(*c, ins, ndir, level, nullptr, false, &cells_state);
+    c->boxes_known = cells_state.ran;
+    return r;
+  };
   if (variant == HD_VARIANT_AUTO) {
+    Selection sel;
     c->ev_base = 0;
-    if ((s = select_variants(*c, ins, ndir, used)) != HD_OK) return s;
-  }
-  if (variant == HD_VARIANT_AUTO && undirected) {
-    // The grid only when both directions qualify; otherwise both directions
-    // share the fused LBVH launches.
-    auto index = [](int v) { return v == HD_VARIANT_GRID || v == HD_VARIANT_LBVH; };
-    if (index(used[0]) && index(used[1]) && used[0] != used[1])
-      used[0] = used[1] = HD_VARIANT_LBVH;
+    if ((s = select_begin(*c, ins, ndir, used, &sel)) != HD_OK) return s;
+    for (int d = 0; d < ndir; ++d)
+      if (sel.decided[d] && used[d] != HD_VARIANT_LBVH) cells = false;
+    if (cells && (s = filter()) != HD_OK) return s;
+    if ((s = select_finish(*c, ins, ndir, used, sel)) != HD_OK) {
+      cudaStreamSynchronize(c->stream);  // the filter still reads the caller's sets
+      return s;
+    }
+    if (undirected) {
+      // The grid only when both directions qualify; otherwise both directions
+      // share the fused LBVH launches.
+      auto index = [](int v) { return v == HD_VARIANT_GRID || v == HD_VARIANT_LBVH; };
+      if (index(used[0]) && index(used[1]) && used[0] != used[1])
+        used[0] = used[1] = HD_VARIANT_LBVH;
+    }
+  } else if (cells && (s = filter()) != HD_OK) {
+    return s;
   }
   const bool fused = undirected && used[0] == HD_VARIANT_LBVH && used[1] == HD_VARIANT_LBVH;
   auto run_all = [&]() -> hd_status {
     hd_status r;
-    if (fused) {
+    if (cells) {
+      // What the cell filter left: lists go to the LBVH; a direction whose
+      // answer is too few cells is filtered on a finer grid; sets that it
+      // still leaves whole go to the chosen index.  (Lists are used before the
+      // next filter run reuses their buffer.)
+      CellsLeft left[2];
+      DirInput rest[2];
+      CellsLeft rest_left[2];
+      int n = 0;
+      // A direction that the filter's seeds already rule out (and that no finer
+      // grid takes) starts on its index behind the filter's other kernels.
+      bool off[2], indexed[2] = {false, false};
+      float reach[2];
+      if ((r = cells_hopeless(*c, ndir, n_dims, cells_state, off, reach)) != HD_OK) return r;
+      for (int d = 0; d < ndir; ++d)
+        indexed[d] = off[d] && cells_finer(n_a + n_b, n_dims, level, reach[d]) < 0;
+      if (indexed[0] && indexed[1] && fused) {
+        if ((r = run_lbvh_pair(*c, ins[0], ins[1])) != HD_OK) return r;
+      } else {
+        for (int d = 0; d < ndir; ++d)
+          if (indexed[d] && (r = run_direction(*c, ins[d], used[d], &used[d], &ex[d])) != HD_OK)
+            return r;
+      }
+      if ((r = cells_finish(*c, ndir, true, cells_state, left)) != HD_OK) return r;
+      have_result = cells_state.ran;
+      for (int d = 0; d < ndir; ++d) left[d].done |= indexed[d];
+      for (int d = 0; d < ndir; ++d)
+        if (!left[d].done && left[d].narrowed) {
+          rest[n] = ins[d];
+          rest_left[n++] = left[d];
+        }
+      if (n && (r = run_lbvh_left(*c, rest, n, nullptr, rest_left)) != HD_OK) return r;
+      bool lists = n > 0;
+      n = 0;
+      for (int d = 0; d < ndir; ++d) {
+        if (left[d].done || left[d].narrowed) continue;
+        const int finer = cells_finer(n_a + n_b, n_dims, level, left[d].reach);
+        CellsLeft fine;
+        if (finer >= 0) {
+          CellsRun again;
+          if ((r = cells_begin(*c, &ins[d], 1, finer, nullptr, true, &again)) != HD_OK) return r;
+          if ((r = cells_finish(*c, 1, true, again, &fine)) != HD_OK) return r;
+        }
+        if (!fine.done && fine.narrowed) {
+          if ((r = run_lbvh_left(*c, &ins[d], 1, nullptr, &fine)) != HD_OK) return r;
+          lists = true;
+        } else if (!fine.done) {
+          rest[n++] = ins[d];
+        }
+      }
+      if (lists || n) have_result = false;
+      if (n == 2 && fused) {
+        if ((r = run_lbvh_pair(*c, rest[0], rest[1])) != HD_OK) return r;
+      } else {
+        for (int i = 0; i < n; ++i) {
+          const int d = rest[i].dir;
+          if ((r = run_direction(*c, rest[i], used[d], &used[d], &ex[d])) != HD_OK) return r;
+        }
+      }
+      mark(*c, 6);
+    } else if (fused) {
       // Fused undirected pass: one sort of both sets, both trees and both
       // directions' queries in shared launches.
       c->ev_base = 0;
@@ -535,7 +657,7 @@ hd_status hd_solve(hd_ctx* c, const float* A, uint64_t n_a, const float* B,
   // a CUDA graph and later ones replay it (no per-kernel launch cost).
   // Timed solves (HD_TIMING) always launch directly.
   auto graphable = [&](int v) { return v == HD_VARIANT_LBVH || v == HD_VARIANT_EB; };
-  const bool eligible = !c->timing && graphable(used[0]) && (!undirected || graphable(used[1]));
+  const bool eligible = !c->timing && !cells && graphable(used[0]) && (!undirected || graphable(used[1]));
   const uint64_t key[11] = {(uint64_t) dA, (uint64_t) dB, n_a, n_b, (uint64_t) n_dims, flags,
                             (uint64_t) (int64_t) used[0], (uint64_t) (int64_t) used[1],
                             (uint64_t) c->stream, c->buf_gen, 1};
@@ -587,11 +709,13 @@ hd_status hd_solve(hd_ctx* c, const float* A, uint64_t n_a, const float* B,
     }
   }
   HostScalars* h = reinterpret_cast<HostScalars*>(c->host_pinned);
-  cudaError_t e = cudaMemcpyAsync(h, c->bufs[kBufScalars].p, sizeof(HostScalars),
-                                  cudaMemcpyDeviceToHost, c->stream);
+  cudaError_t e = cudaSuccess;
+  if (!have_result)
+    e = cudaMemcpyAsync(h, c->bufs[kBufScalars].p, sizeof(HostScalars), cudaMemcpyDeviceToHost,
+                        c->stream);
   if (e != cudaSuccess) return cuda_fail(*c, e, "copy result");
   mark_abs(*c, 25);
-  e = cudaStreamSynchronize(c->stream);
+  if (!have_result || c->timing) e = cudaStreamSynchronize(c->stream);
   if (e != cudaSuccess) return cuda_fail(*c, e, "solve");
   if ((s = check_status(*c, *h, ndir)) != HD_OK) return s;
 

@@ -182,33 +182,80 @@ __device__ __forceinline__ float prune32(double best, double rxy) {
 
 // Cuts a set to float (Xf may be null: check only); records the largest
 // exponent, non-finite and out-of-range values, and tiny magnitudes.
-// Integer operations only.
+// Integer operations only, but for D = 2 or 3: there the box of the cut
+// points goes to ord as well (order-preserving bits, as k_mbr2 leaves it),
+// which saves the cell filter a pass over them.  D = 0: any n_dims.
+template <int D>
 __global__ void k_f64_round(const double* __restrict__ X, uint64_t total, float* __restrict__ Xf,
-                            RoundStats* st) {
+                            RoundStats* st, uint32_t* __restrict__ ord) {
   uint32_t emax = 0, fl = 0;
-  for (uint64_t t = blockIdx.x * (uint64_t) blockDim.x + threadIdx.x; t < total;
-       t += (uint64_t) gridDim.x * blockDim.x) {
-    const double x = X[t];
-    const unsigned long long a = dbits(x) & 0x7FFFFFFFFFFFFFFFull;
-    const uint32_t ex = (uint32_t) (a >> 52);
-    if (ex == 0x7FFu)
-      fl |= kF64NonFinite;
-    else if (a > kRangeBits)
-      fl |= kF64Range;
-    if (ex >= 1023u - 126u)
-      emax = max(emax, ex);
-    else if (a != 0ull)
-      fl |= kF64Tiny;
-    if (Xf) Xf[t] = cut_to_float(x);
+  constexpr int kStep = D ? D : 1;
+  float lo[kStep], hi[kStep];
+#pragma unroll
+  for (int k = 0; k < kStep; ++k) {
+    lo[k] = FLT_MAX;
+    hi[k] = -FLT_MAX;
+  }
+  const uint64_t stride = (uint64_t) gridDim.x * blockDim.x;
+  for (uint64_t t = blockIdx.x * (uint64_t) blockDim.x + threadIdx.x; t < total / kStep; t += stride) {
+    double x[kStep];
+#pragma unroll
+    for (int k = 0; k < kStep; ++k) x[k] = X[t * kStep + k];
+#pragma unroll
+    for (int k = 0; k < kStep; ++k) {
+      const unsigned long long a = dbits(x[k]) & 0x7FFFFFFFFFFFFFFFull;
+      const uint32_t ex = (uint32_t) (a >> 52);
+      if (ex == 0x7FFu)
+        fl |= kF64NonFinite;
+      else if (a > kRangeBits)
+        fl |= kF64Range;
+      if (ex >= 1023u - 126u)
+        emax = max(emax, ex);
+      else if (a != 0ull)
+        fl |= kF64Tiny;
+      const float f = cut_to_float(x[k]);
+      if (Xf) Xf[t * kStep + k] = f;
+      if (D) {
+        lo[k] = fminf(lo[k], f);
+        hi[k] = fmaxf(hi[k], f);
+      }
+    }
   }
 #pragma unroll
   for (int o = 16; o; o >>= 1) {
     emax = max(emax, __shfl_xor_sync(0xFFFFFFFFu, emax, o));
     fl |= __shfl_xor_sync(0xFFFFFFFFu, fl, o);
+    if (D) {
+#pragma unroll
+      for (int k = 0; k < kStep; ++k) {
+        lo[k] = fminf(lo[k], __shfl_xor_sync(0xFFFFFFFFu, lo[k], o));
+        hi[k] = fmaxf(hi[k], __shfl_xor_sync(0xFFFFFFFFu, hi[k], o));
+      }
+    }
   }
   if ((threadIdx.x & 31) == 0) {
     if (emax) atomicMax(&st->emax, emax);
     if (fl) atomicOr(&st->flags, fl);
+  }
+  if constexpr (D > 0) {
+    __shared__ uint32_t s_lo[D], s_hi[D];
+    if (threadIdx.x < D) {
+      s_lo[threadIdx.x] = 0xFFFFFFFFu;
+      s_hi[threadIdx.x] = 0u;
+    }
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) {
+#pragma unroll
+      for (int k = 0; k < D; ++k) {
+        atomicMin(&s_lo[k], f2ord(lo[k]));
+        atomicMax(&s_hi[k], f2ord(hi[k]));
+      }
+    }
+    __syncthreads();
+    if (threadIdx.x < D) {
+      atomicMin(&ord[threadIdx.x], s_lo[threadIdx.x]);
+      atomicMax(&ord[4 + threadIdx.x], s_hi[threadIdx.x]);
+    }
   }
 }
 
@@ -669,6 +716,7 @@ hd_status hd_solve_f64(hd_ctx* c, const double* A, uint64_t n_a, const double* B
   out->hd_ba = -1.0;
   c->timing = (flags & HD_TIMING) != 0;
   c->sorted_valid = false;
+  c->cells_live = false;
   c->ev_base = 0;
   if (c->timing) cudaEventRecord(c->ev[24], c->stream);
   const bool undirected = (flags & HD_UNDIRECTED) != 0;
@@ -709,9 +757,12 @@ hd_status hd_solve_f64(hd_ctx* c, const double* A, uint64_t n_a, const double* B
     const uint64_t total = nn[k] * (uint64_t) n_dims;
     const int grid =
         (int) std::max<uint64_t>(1, std::min<uint64_t>((total + 255) / 256, (uint64_t) c->num_sms * 8));
-    k_f64_round<<<grid, 256, 0, c->stream>>>(d64[k], total, (float*) p, &aux->round[k]);
+    uint32_t* ord = &scalars(*c, 0)->mbr_ord[k][0][0];
+    auto kern = n_dims == 2 ? k_f64_round<2> : n_dims == 3 ? k_f64_round<3> : k_f64_round<0>;
+    kern<<<grid, 256, 0, c->stream>>>(d64[k], total, (float*) p, &aux->round[k], ord);
     if ((s = after_launch(*c, "f64_round")) != HD_OK) return s;
   }
+  c->boxes_known = spatial_dims;
   static_assert(sizeof(F64Aux) + 1024 <= 4096, "pinned staging");
   F64Aux* h = reinterpret_cast<F64Aux*>((char*) c->host_pinned + 1024);
   auto read_aux = [&]() -> hd_status {
@@ -766,7 +817,21 @@ hd_status hd_solve_f64(hd_ctx* c, const double* A, uint64_t n_a, const double* B
       if ((double) rf < call.rxy[k]) rf = std::nextafter(rf, INFINITY);
       plan.soft_r[k] = rf;
     }
-    if ((s = run_lbvh_f64(*c, ins, ndir, &plan)) != HD_OK) return s;
+    // The cell filter first, by the listing pass's level; the lists it leaves
+    // are searched in place of the sets when it narrowed every direction and no
+    // list of rows can overflow (then every row of the set would be walked).
+    CellsLeft left[2];
+    bool narrowed = false;
+    if (cells_apply(*c, n_a, n_b, n_dims)) {
+      CellsRun run;
+      if ((s = cells_begin(*c, ins, ndir, cells_level(n_a + n_b, n_dims), &plan, true, &run)) != HD_OK) return s;
+      if ((s = cells_finish(*c, ndir, false, run, left)) != HD_OK) return s;
+      narrowed = true;
+      for (int k = 0; k < ndir; ++k) narrowed &= left[k].narrowed && left[k].nq <= kListCap;
+    }
+    if (!narrowed) c->cells_live = false;
+    s = narrowed ? run_lbvh_left(*c, ins, ndir, &plan, left) : run_lbvh_f64(*c, ins, ndir, &plan);
+    if (s != HD_OK) return s;
     if ((s = read_aux()) != HD_OK) return s;
     DevScalars hs[2];
     cudaError_t e = cudaMemcpy(hs, scalars(*c, 0), sizeof(hs), cudaMemcpyDeviceToHost);

@@ -7,6 +7,9 @@
 #include <vector>
 
 #include "../../include/hd_gpu.h"
+#ifdef __CUDACC__
+#include "hd_common.cuh"
+#endif
 
 namespace hdg {
 
@@ -50,6 +53,35 @@ struct DevScalars {
   uint32_t mbr_ord[2][2][4];      // [set][lo/hi][dim], order-preserving uints
 };
 
+#ifdef __CUDACC__
+// The result words of a direction from its running maximum and argmin.
+__device__ __forceinline__ void finalize_scalars(const float* __restrict__ A,
+                                                 const float* __restrict__ B, int D,
+                                                 DevScalars* sc) {
+  const unsigned long long key = sc->max_key;
+  const uint32_t ia = unpack_max_index(key);
+  if (key == 0 || ia == kInvalid) {  // no row has completed
+    sc->status |= kErrInternal;
+    return;
+  }
+  const uint32_t d2bits = (uint32_t) (key >> 32);
+  const unsigned long long mk = sc->min_key;
+  const uint32_t ib = (uint32_t) (mk & 0xFFFFFFFFull);
+  // The argmin over B of A[ia] must reproduce the maximum exactly: it is the
+  // same FP32 formula over the same coordinates.
+  if ((uint32_t) (mk >> 32) != d2bits) sc->status |= kErrInternal;
+  double s = 0.0;
+  for (int k = 0; k < D; ++k) {
+    double t = (double) A[(uint64_t) ia * D + k] - (double) B[(uint64_t) ib * D + k];
+    s += t * t;
+  }
+  sc->d2_64 = s;
+  sc->d2 = __uint_as_float(d2bits);
+  sc->ia = ia;
+  sc->ib = ib;
+}
+#endif
+
 // A growable device buffer cached in the context across solves.
 struct DevBuf {
   void* p = nullptr;
@@ -90,6 +122,8 @@ enum BufSlot {
   kBufF64A,       // FP64 input path: caller's double A / B on the device
   kBufF64B,
   kBufF64Aux,     // FP64 scalars and candidate lists
+  kBufCells,      // cell filter: bitmaps and lists
+  kBufLeft,       // sorted points that the cell filter left open
   kBufF64Rows,    // FP64 nearest distance and column of every walked row
   kNumBufs
 };
@@ -174,6 +208,9 @@ struct Ctx {
   size_t host_pinned_bytes = 0;
   void* sel_pinned = nullptr;    // pinned staging of the selector's samples
   size_t sel_pinned_bytes = 0;
+  cudaEvent_t sel_event = nullptr;  // after the samples' copy
+  bool cells_live = false;  // kernels yet to be enqueued read kBufCells
+  cudaEvent_t cells_event = nullptr;  // after the copy of the filter's seeds
   void* batch_pinned = nullptr;  // pinned staging of grouped batch results
   size_t batch_pinned_bytes = 0;
   std::string last_error;
@@ -213,6 +250,7 @@ struct Ctx {
   // are shared by both directions of an undirected solve.
   SortedSet sorted[2];
   bool sorted_valid = false;
+  bool boxes_known = false;  // DevScalars[0].mbr_ord holds the call's boxes
   // Sampler statistic of the last AUTO decision per direction (p80 of the
   // sampled early-break iteration counts; 0 when no sample was drawn).
   double last_p80[2] = {0.0, 0.0};
@@ -278,6 +316,16 @@ hd_status select_variant(Ctx& c, const DirInput& in, int* variant);
 // directions query and target the same two sets): one sample of each set, one
 // read-back.  v[d] receives each direction's variant.
 hd_status select_variants(Ctx& c, const DirInput* ins, int ndir, int* v);
+// The same in two steps: begin enqueues the samples and their copy (pending:
+// some direction needs them), finish waits for that copy alone and decides, so
+// that kernels enqueued in between run while the host works it out.
+struct Selection {
+  bool pending = false, decided[2] = {false, false};
+  uint32_t k[2], m[2];
+  size_t o_it[2], o_smp[2];
+};
+hd_status select_begin(Ctx& c, const DirInput* ins, int ndir, int* v, Selection* sel);
+hd_status select_finish(Ctx& c, const DirInput* ins, int ndir, int* v, const Selection& sel);
 // The selector's choice when the sizes alone decide it (no sampling of the
 // data); false when it needs the sample pass.
 bool select_variant_by_size(const Ctx& c, uint64_t nA, uint64_t nB, int dims, int* variant);
@@ -315,9 +363,53 @@ struct F64Plan {
 hd_status run_lbvh_f64(Ctx& c, const DirInput* ins, int count, F64Plan* plan);
 hd_status f64_seed(Ctx& c, F64Plan& plan, int count);
 
+// Cell filter (hd_cells.cu).  What it left of one direction: done (its result
+// is in DevScalars), or narrowed to the listed queries and targets (float4 x,
+// y, z, row), or neither (the whole sets have to be searched).
+struct CellsLeft {
+  bool done = false, narrowed = false;
+  float reach = 0.0f;  // L in cells, 0 if unknown
+  const float4* q = nullptr;
+  const float4* t = nullptr;
+  uint64_t nq = 0, nt = 0;
+};
+constexpr uint64_t kCellsMinPoints = 40000;
+bool cells_apply(const Ctx& c, uint64_t nA, uint64_t nB, int dims);
+// The grid (level) to start on, and the one to try again on when the filter
+// neither finished nor narrowed a direction (its L: `reach` cells); -1: none.
+int cells_level(uint64_t points, int dims);
+int cells_finer(uint64_t points, int dims, int level, float reach);
+// Filters `count` directions: the call's (ins[k].dir == k), or one of them.  With a plan, queries are
+// settled by the FP64 listing pass's level, and no direction is finished here.
+// scalars_too: also copies both DevScalars to the pinned staging.  boxes_known:
+// DevScalars[0].mbr_ord already holds the sets' boxes.
+//   cells_begin enqueues the filter, cells_finish waits for the stream and
+//   reads what it left (begin's `ran` false: there was no room for its lists).
+struct CellsRun {
+  bool ran = false;
+  const void* state = nullptr;  // device words to read back
+  const float4* q[2];
+  const float4* t[2];
+  uint32_t cap_q[2], cap_t[2];
+};
+hd_status cells_begin(Ctx& c, const DirInput* ins, int count, int level, const F64Plan* plan,
+                      bool boxes_known, CellsRun* run);
+// Waits for the filter's seeds alone: off[k] where it will give direction k up
+// (reach[k]: its L in cells), so that the index can be enqueued behind it.
+hd_status cells_hopeless(Ctx& c, int count, int dims, const CellsRun& run, bool* off,
+                         float* reach);
+hd_status cells_finish(Ctx& c, int count, bool scalars_too, const CellsRun& run, CellsLeft* left);
+// LBVH over what the filter left of `count` directions.
+hd_status run_lbvh_left(Ctx& c, const DirInput* ins, int count, F64Plan* plan,
+                        const CellsLeft* left);
+
 // Common tail: exact argmin of A[ia] over B, FP64 recomputation, written to
 // DevScalars[dir].  Used by every variant.
 hd_status certify(Ctx& c, const DirInput& in);
+
+// The same with the argmin over the targets the cell filter collected: every
+// target at the certifying row's distance is among them.
+hd_status certify_left(Ctx& c, const DirInput& in, const CellsLeft& left);
 
 // Resets both directions' DevScalars (allocating the scalars buffer).
 hd_status init_scalars(Ctx& c);
@@ -343,6 +435,11 @@ hd_status spatial_prepare(Ctx& c, const DirInput& in, const SortedSet** q,
 // then sorts B (sets c.sorted, c.sorted_valid); *dA, *dB = device copies.
 hd_status spatial_upload_sort(Ctx& c, const float* hA, uint64_t nA, const float* hB, uint64_t nB,
                               int dims, const float** dA, const float** dB);
+// Boxes of the call's two sets, into DevScalars[0].mbr_ord.
+hd_status spatial_boxes(Ctx& c, const DirInput& in);
+// Morton-sorts listed points in the common frame of the call's boxes: out[2k]
+// = queries, out[2k + 1] = targets (with leaf boxes) of direction k.
+hd_status spatial_sort_left(Ctx& c, const CellsLeft* left, int count, int dims, SortedSet* out);
 // k random positions in [0, n) (with replacement), k from opt.sample_rate.
 hd_status make_sample(Ctx& c, uint64_t n, uint64_t seed, uint32_t* k, uint32_t** list);
 

@@ -183,22 +183,6 @@ __device__ __forceinline__ float box_max_d2(const float4& q, const float4& xy, f
 // box bound and the FP32 pair formula each carry a few ulps of rounding.
 constexpr float kMaxDistMargin = 1.0f + 1.0f / 65536.0f;
 
-// The FP64 input path's listing pass stops a row only below soft_stop(thr):
-// a lower bound, from the running maximum thr alone, of the threshold under
-// which an FP32 distance proves an FP64 distance below the final answer's
-// seed (the bound is derived in hd_f64.cu; every step here rounds toward
-// zero, r = how far a cut pair's distance can move).  -1: no row stops.
-__device__ __forceinline__ float soft_stop(float thr, float r) {
-  if (!(thr >= 0.0f)) return -1.0f;
-  const float abs32 = 5.0f * 0x1p-126f;  // (n_dims + 2) 2^-126, n_dims <= 3
-  const float base = __fsub_rd(thr, abs32);
-  if (!(base > 0.0f)) return -1.0f;
-  const float sg = __fsub_rd(__fmul_rd(__fsqrt_rd(base), 0.99999f), __fmul_ru(2.01f, r));
-  if (!(sg > 0.0f)) return -1.0f;
-  const float g = __fsub_rd(__fmul_rd(__fmul_rd(sg, sg), 0.999999f), abs32);
-  return g > 0.0f ? g : -1.0f;
-}
-
 // Division of a 32-bit value by a run-time constant d, with the multiplier
 // m and shifts s1, s2 prepared on the host (Granlund and Montgomery,
 // "Division by Invariant Integers using Multiplication", PLDI 1994):
@@ -790,13 +774,25 @@ static hd_status build_lbvhs(Ctx& c, const SortedSet* const* sets, int count, Bu
 // with shared launches.  With a plan (the FP64 input path), the query pass
 // is the listing pass (rows stop only below the soft bound and the open ones
 // are listed), and the certified FP32 solve is followed by f64_seed.
-static hd_status run_lbvh_dirs(Ctx& c, const DirInput* ins, int count, F64Plan* plan) {
+// left: the queries and targets the cell filter left open (else null: the
+// whole sets).
+static hd_status run_lbvh_dirs(Ctx& c, const DirInput* ins, int count, F64Plan* plan,
+                               const CellsLeft* left) {
   const int dims = ins[0].dims;
   if (dims != 2 && dims != 3) return fail(c, HD_ERR_UNSUPPORTED, "LBVH needs n_dims 2 or 3");
   hd_status s;
   const SortedSet *q[2], *t[2];
-  for (int k = 0; k < count; ++k)
-    if ((s = spatial_prepare(c, ins[k], &q[k], &t[k])) != HD_OK) return s;
+  SortedSet open[4];
+  if (left) {
+    if ((s = spatial_sort_left(c, left, count, dims, open)) != HD_OK) return s;
+    for (int k = 0; k < count; ++k) {
+      q[k] = &open[2 * k];
+      t[k] = &open[2 * k + 1];
+    }
+  } else {
+    for (int k = 0; k < count; ++k)
+      if ((s = spatial_prepare(c, ins[k], &q[k], &t[k])) != HD_OK) return s;
+  }
   mark(c, 1);
   QuerySets qs;
   // Two queries per lane when the launch answers at least
@@ -907,24 +903,30 @@ static hd_status run_lbvh_dirs(Ctx& c, const DirInput* ins, int count, F64Plan* 
   if ((s = launch_queries(ins[0].count)) != HD_OK) return s;
   mark(c, 4);
   for (int k = 0; k < count; ++k)
-    if ((s = certify(c, ins[k])) != HD_OK) return s;
+    if ((s = left ? certify_left(c, ins[k], left[k]) : certify(c, ins[k])) != HD_OK) return s;
   if (plan) {
     for (int k = 0; k < count; ++k)
       plan->tree[k] = LbvhTree{bs.s[k].nodes, bs.s[k].root, t[k]->pts, t[k]->n, bs.s[k].L};
     if ((s = f64_seed(c, *plan, count)) != HD_OK) return s;
   }
+  if (left) c.cells_live = false;  // the lists are used up
   return HD_OK;
 }
 
-hd_status run_lbvh(Ctx& c, const DirInput& in) { return run_lbvh_dirs(c, &in, 1, nullptr); }
+hd_status run_lbvh(Ctx& c, const DirInput& in) { return run_lbvh_dirs(c, &in, 1, nullptr, nullptr); }
 
 hd_status run_lbvh_pair(Ctx& c, const DirInput& ab, const DirInput& ba) {
   const DirInput ins[2] = {ab, ba};
-  return run_lbvh_dirs(c, ins, 2, nullptr);
+  return run_lbvh_dirs(c, ins, 2, nullptr, nullptr);
 }
 
 hd_status run_lbvh_f64(Ctx& c, const DirInput* ins, int count, F64Plan* plan) {
-  return run_lbvh_dirs(c, ins, count, plan);
+  return run_lbvh_dirs(c, ins, count, plan, nullptr);
+}
+
+hd_status run_lbvh_left(Ctx& c, const DirInput* ins, int count, F64Plan* plan,
+                        const CellsLeft* left) {
+  return run_lbvh_dirs(c, ins, count, plan, left);
 }
 
 }  // namespace hdg

@@ -170,10 +170,16 @@ __global__ void k_seed_finish(Perm pA, uint32_t offset, const uint32_t* __restri
     atomicMax(&sc->max_key, pack_max(__uint_as_float(seed_min[e]), (uint32_t) pA(offset + e)));
 }
 
-// Strided sample of m points of P (point i*n/m), rows of dims floats.
-__global__ void k_gather_sample(const float* __restrict__ P, uint64_t n, int dims, uint32_t m,
-                                float* __restrict__ out) {
+// Strided samples of both sets (blockIdx.y = set): m of its n points (point
+// i*n/m), rows of dims floats.
+__global__ void k_gather_sample(const float* __restrict__ P0, uint64_t n0, uint32_t m0,
+                                float* __restrict__ out0, const float* __restrict__ P1, uint64_t n1,
+                                uint32_t m1, float* __restrict__ out1, int dims) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  const float* P = blockIdx.y ? P1 : P0;
+  const uint64_t n = blockIdx.y ? n1 : n0;
+  const uint32_t m = blockIdx.y ? m1 : m0;
+  float* out = blockIdx.y ? out1 : out0;
   if (i >= m) return;
   const uint64_t src = (uint64_t) i * n / m;
   for (int d = 0; d < dims; ++d) out[(uint64_t) i * dims + d] = P[src * dims + d];
@@ -255,23 +261,25 @@ bool select_variant_by_size(const Ctx& c, uint64_t nA, uint64_t nB, int dims, in
   return false;
 }
 
-hd_status select_variants(Ctx& c, const DirInput* ins, int ndir, int* v) {
+hd_status select_begin(Ctx& c, const DirInput* ins, int ndir, int* v, Selection* sel) {
   const Tuning& tu = tuning();
-  bool need = false, decided[2] = {false, false};
+  sel->pending = false;
+  bool* decided = sel->decided;
   for (int d = 0; d < ndir; ++d) {
     decided[d] = select_variant_by_size(c, ins[d].nA, ins[d].nB, ins[d].dims, &v[d]);
-    need |= !decided[d];
+    sel->pending |= !decided[d];
   }
-  if (!need) return HD_OK;
+  if (!sel->pending) return HD_OK;
   // One sample of each set serves both directions (query in one, target in
   // the other); the early-break samples run per direction.  Everything comes
-  // back in one copy, with one synchronisation.
+  // back in one copy.
   const int dims = ins[0].dims;
   const float* P[2] = {ins[0].A, ins[0].B};
   const uint64_t nP[2] = {ins[0].nA, ins[0].nB};
   const uint32_t m[2] = {(uint32_t) std::min<uint64_t>(nP[0], kStatSamples),
                          (uint32_t) std::min<uint64_t>(nP[1], kStatSamples)};
-  uint32_t k[2] = {0, 0};
+  uint32_t* k = sel->k;
+  k[0] = k[1] = 0;
   const double rate = c.opt.sample_rate > 0 ? c.opt.sample_rate : 0.01;
   for (int d = 0; d < ndir; ++d) {
     if (decided[d]) continue;
@@ -300,12 +308,14 @@ hd_status select_variants(Ctx& c, const DirInput* ins, int ndir, int* v) {
     }
     c.sel_pinned_bytes = words * 4;
   }
-  uint32_t* w = (uint32_t*) buf;
-  for (int t = 0; t < 2; ++t) {
-    k_gather_sample<<<(m[t] + 255) / 256, 256, 0, c.stream>>>(P[t], nP[t], dims, m[t],
-                                                              (float*) (w + o_smp[t]));
-    if ((s = after_launch(c, "gather_sample")) != HD_OK) return s;
+  if (!c.sel_event) {
+    cudaError_t e = cudaEventCreateWithFlags(&c.sel_event, cudaEventDisableTiming);
+    if (e != cudaSuccess) return cuda_fail(c, e, "selector event");
   }
+  uint32_t* w = (uint32_t*) buf;
+  k_gather_sample<<<dim3((std::max(m[0], m[1]) + 255) / 256, 2), 256, 0, c.stream>>>(
+      P[0], nP[0], m[0], (float*) (w + o_smp[0]), P[1], nP[1], m[1], (float*) (w + o_smp[1]), dims);
+  if ((s = after_launch(c, "gather_sample")) != HD_OK) return s;
   const uint64_t seed = c.opt.seed;
   for (int d = 0; d < ndir; ++d) {
     if (k[d] == 0) continue;
@@ -330,12 +340,32 @@ hd_status select_variants(Ctx& c, const DirInput* ins, int ndir, int* v) {
     if ((s = after_launch(c, "sample_eb")) != HD_OK) return s;
     c.seeded[in.dir] = in.nA > k[d];
   }
-  uint32_t* h = (uint32_t*) c.sel_pinned;
-  cudaError_t e = cudaMemcpyAsync(h, buf, words * 4, cudaMemcpyDeviceToHost, c.stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(c.stream);
+  cudaError_t e = cudaMemcpyAsync(c.sel_pinned, buf, words * 4, cudaMemcpyDeviceToHost, c.stream);
+  if (e == cudaSuccess) e = cudaEventRecord(c.sel_event, c.stream);
   if (e != cudaSuccess) return cuda_fail(c, e, "sample statistics");
+  for (int t = 0; t < 2; ++t) {
+    sel->m[t] = m[t];
+    sel->o_it[t] = o_it[t];
+    sel->o_smp[t] = o_smp[t];
+  }
+  return HD_OK;
+}
+
+hd_status select_finish(Ctx& c, const DirInput* ins, int ndir, int* v, const Selection& sel) {
+  if (!sel.pending) return HD_OK;
+  const Tuning& tu = tuning();
+  cudaError_t e = cudaEventSynchronize(c.sel_event);
+  if (e != cudaSuccess) return cuda_fail(c, e, "sample statistics");
+  const uint32_t* h = (const uint32_t*) c.sel_pinned;
+  const int dims = ins[0].dims;
+  const float* P[2] = {ins[0].A, ins[0].B};
+  const uint64_t nP[2] = {ins[0].nA, ins[0].nB};
+  const uint32_t* m = sel.m;
+  const uint32_t* k = sel.k;
+  const size_t* o_it = sel.o_it;
+  const size_t* o_smp = sel.o_smp;
   for (int d = 0; d < ndir; ++d) {
-    if (decided[d]) continue;
+    if (sel.decided[d]) continue;
     const DirInput& in = ins[d];
     // Direction d queries set q against set t (set 0 is the call's A).
     const int q = in.A == P[0] && in.nA == nP[0] ? 0 : 1, t = 1 - q;
@@ -365,6 +395,12 @@ hd_status select_variants(Ctx& c, const DirInput* ins, int ndir, int* v) {
       v[d] = HD_VARIANT_LBVH;
   }
   return HD_OK;
+}
+
+hd_status select_variants(Ctx& c, const DirInput* ins, int ndir, int* v) {
+  Selection sel;
+  hd_status s = select_begin(c, ins, ndir, v, &sel);
+  return s != HD_OK ? s : select_finish(c, ins, ndir, v, sel);
 }
 
 hd_status select_variant(Ctx& c, const DirInput& in, int* v) {

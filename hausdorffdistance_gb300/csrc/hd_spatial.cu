@@ -332,7 +332,7 @@ hd_status sort_set(Ctx& c, int k, const float* P, uint64_t n, int dims, const So
   const uint64_t base = k ? x.nA : 0;
   uint32_t* ord = &scalars(c, 0)->mbr_ord[k][0][0];
   Frame* fr = frame(c, k);
-  {
+  if (!c.boxes_known) {
     const int gx = grid_for(c, (n + 3) / 4, 256);
     k_mbr2<<<dim3(gx, 1), 256, 0, st>>>(P, n, P, n, dims, ord, ord);
     if ((s = after_launch(c, "mbr")) != HD_OK) return s;
@@ -377,7 +377,7 @@ static hd_status spatial_sort_fused(Ctx& c, const float* A, uint64_t nA, const f
   SortScratch x;
   if ((s = sort_scratch(c, nA, nB, true, &x)) != HD_OK) return s;
   DevScalars* sc = scalars(c, 0);
-  {
+  if (!c.boxes_known) {
     const int gx = grid_for(c, (std::max(nA, nB) + 3) / 4, 256);
     k_mbr2<<<dim3(gx, 2), 256, 0, c.stream>>>(A, nA, B, nB, dims, &sc->mbr_ord[0][0][0],
                                               &sc->mbr_ord[1][0][0]);
@@ -462,13 +462,135 @@ hd_status spatial_upload_sort(Ctx& c, const float* hA, uint64_t nA, const float*
   return HD_OK;
 }
 
+hd_status spatial_boxes(Ctx& c, const DirInput& in) {
+  DevScalars* sc = scalars(c, 0);
+  const int gx = grid_for(c, (std::max(in.nA, in.nB) + 3) / 4, 256);
+  k_mbr2<<<dim3(gx, 2), 256, 0, c.stream>>>(in.A, in.nA, in.B, in.nB, in.dims,
+                                            &sc->mbr_ord[0][0][0], &sc->mbr_ord[1][0][0]);
+  return after_launch(c, "mbr");
+}
+
+namespace {
+
+// Up to four lists of (x, y, z, row) points.
+struct LeftLists {
+  const float4* p[4];
+  uint32_t begin[5];  // positions of the lists in the sorted order
+  uint32_t leaf0[5];  // and of their leaves
+};
+
+// Codes of the listed points in the common frame (blockIdx.y = list); the list
+// is bits 30 and 31 of the key, so one sort orders them all.
+template <int D>
+__global__ void k_morton_left(LeftLists l, const Frame* __restrict__ fr, uint32_t* __restrict__ keys,
+                              uint32_t* __restrict__ vals) {
+  const int k = blockIdx.y;
+  const Frame f = *fr;
+  const uint32_t n = l.begin[k + 1] - l.begin[k];
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const float4 p = l.p[k][i];
+    keys[l.begin[k] + i] = frame_code<D>(f, p.x, p.y, p.z) | ((uint32_t) k << 30);
+    vals[l.begin[k] + i] = i;
+  }
+}
+
+__global__ void k_gather_left(LeftLists l, const uint32_t* __restrict__ order,
+                              float4* __restrict__ out, uint32_t L, float4* __restrict__ lb) {
+  const int k = blockIdx.y;
+  const uint32_t n = l.begin[k + 1] - l.begin[k], stride = gridDim.x * blockDim.x;
+  for (uint64_t j0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); j0 < n; j0 += stride) {
+    const uint32_t j = (uint32_t) j0 + (threadIdx.x & 31u);
+    const bool valid = j < n;
+    float lx = FLT_MAX, ly = FLT_MAX, lz = FLT_MAX, hx = -FLT_MAX, hy = -FLT_MAX, hz = -FLT_MAX;
+    if (valid) {
+      const float4 p = l.p[k][order[l.begin[k] + j]];
+      out[l.begin[k] + j] = p;
+      lx = hx = p.x;
+      ly = hy = p.y;
+      lz = hz = p.z;
+    }
+    if (!(k & 1)) continue;  // queries have no leaves
+    for (uint32_t o = 1; o < L; o <<= 1) {
+      lx = fminf(lx, __shfl_xor_sync(0xFFFFFFFFu, lx, o));
+      ly = fminf(ly, __shfl_xor_sync(0xFFFFFFFFu, ly, o));
+      lz = fminf(lz, __shfl_xor_sync(0xFFFFFFFFu, lz, o));
+      hx = fmaxf(hx, __shfl_xor_sync(0xFFFFFFFFu, hx, o));
+      hy = fmaxf(hy, __shfl_xor_sync(0xFFFFFFFFu, hy, o));
+      hz = fmaxf(hz, __shfl_xor_sync(0xFFFFFFFFu, hz, o));
+    }
+    if (valid && (j & (L - 1)) == 0) {
+      const uint64_t leaf = l.leaf0[k] + j / L;
+      lb[2 * leaf] = make_float4(lx, ly, lz, 0.f);
+      lb[2 * leaf + 1] = make_float4(hx, hy, hz, 0.f);
+    }
+  }
+}
+
+}  // namespace
+
+hd_status spatial_sort_left(Ctx& c, const CellsLeft* left, int count, int dims, SortedSet* out) {
+  hd_status s;
+  uint32_t L = c.opt.leaf_size ? std::min<uint32_t>(c.opt.leaf_size, 32) : 16;
+  while (L & (L - 1)) L &= L - 1;
+  LeftLists l{};
+  uint64_t n = 0, leaves = 0, most = 0;
+  for (int k = 0; k < 2 * count; ++k) {
+    const uint64_t m = (k & 1) ? left[k / 2].nt : left[k / 2].nq;
+    l.p[k] = (k & 1) ? left[k / 2].t : left[k / 2].q;
+    l.begin[k] = (uint32_t) n;
+    l.leaf0[k] = (uint32_t) leaves;
+    n += m;
+    if (k & 1) leaves += (m + L - 1) / L;
+    most = std::max(most, m);
+    l.begin[k + 1] = (uint32_t) n;
+    l.leaf0[k + 1] = (uint32_t) leaves;
+  }
+  if (n >= 0xFFFFFFFFull) return fail(c, HD_ERR_INVALID_ARG, "too many points");
+  void *keys, *keys2, *vals, *vals2, *tmp, *pts, *lb;
+  if ((s = ensure(c, kBufKeys, n * 4, &keys)) != HD_OK) return s;
+  if ((s = ensure(c, kBufKeysAlt, n * 4, &keys2)) != HD_OK) return s;
+  if ((s = ensure(c, kBufVals, n * 4, &vals)) != HD_OK) return s;
+  if ((s = ensure(c, kBufValsAlt, n * 4, &vals2)) != HD_OK) return s;
+  if ((s = ensure(c, kBufLeft, n * sizeof(float4), &pts)) != HD_OK) return s;
+  if ((s = ensure(c, kBufCodes0, leaves * 2 * sizeof(float4), &lb)) != HD_OK) return s;
+  size_t tb = 0;
+  cub::DeviceRadixSort::SortPairs(nullptr, tb, (const uint32_t*) keys, (uint32_t*) keys2,
+                                  (const uint32_t*) vals, (uint32_t*) vals2, (int64_t) n, 0, 32,
+                                  c.stream);
+  if ((s = ensure(c, kBufCubTemp, tb, &tmp)) != HD_OK) return s;
+  Frame* fr = frame(c, 0);
+  DevScalars* sc = scalars(c, 0);
+  k_frame<<<1, 32, 0, c.stream>>>(&sc->mbr_ord[0][0][0], &sc->mbr_ord[1][0][0], dims, 1, 1, fr);
+  if ((s = after_launch(c, "frame")) != HD_OK) return s;
+  const dim3 grid(grid_for(c, most), 2 * count);
+  if (dims == 2)
+    k_morton_left<2><<<grid, 256, 0, c.stream>>>(l, fr, (uint32_t*) keys, (uint32_t*) vals);
+  else
+    k_morton_left<3><<<grid, 256, 0, c.stream>>>(l, fr, (uint32_t*) keys, (uint32_t*) vals);
+  if ((s = after_launch(c, "morton")) != HD_OK) return s;
+  cudaError_t e = cub::DeviceRadixSort::SortPairs(tmp, tb, (const uint32_t*) keys, (uint32_t*) keys2,
+                                                  (const uint32_t*) vals, (uint32_t*) vals2,
+                                                  (int64_t) n, 0, 32, c.stream);
+  if (e != cudaSuccess) return cuda_fail(c, e, "radix sort");
+  k_gather_left<<<grid, 256, 0, c.stream>>>(l, (const uint32_t*) vals2, (float4*) pts, L,
+                                            (float4*) lb);
+  if ((s = after_launch(c, "gather")) != HD_OK) return s;
+  for (int k = 0; k < 2 * count; ++k)
+    out[k] = SortedSet{(float4*) pts + l.begin[k], (uint32_t*) keys2 + l.begin[k], fr,
+                       (float4*) lb + 2 * (uint64_t) l.leaf0[k], L,
+                       l.begin[k + 1] - l.begin[k], dims, nullptr, 0, sorted_mask(0)};
+  return HD_OK;
+}
+
 size_t scalars_bytes() { return 2 * sizeof(DevScalars) + 2 * sizeof(Frame); }
 
 hd_status spatial_prepare(Ctx& c, const DirInput& in, const SortedSet** q,
                           const SortedSet** t) {
   if (!c.sorted_valid) {
-    // Direction 0 of the call: A is the call's A.
-    hd_status s = spatial_sort(c, in.A, in.nA, in.B, in.nB, in.dims, &c.sorted[0], &c.sorted[1]);
+    // Set 0 is the call's A, whichever direction asks first.
+    const bool ab = in.dir == 0;
+    hd_status s = spatial_sort(c, ab ? in.A : in.B, ab ? in.nA : in.nB, ab ? in.B : in.A,
+                               ab ? in.nB : in.nA, in.dims, &c.sorted[0], &c.sorted[1]);
     if (s != HD_OK) return s;
     c.sorted_valid = true;
   }
