@@ -508,7 +508,15 @@ hd_status hd_solve(hd_ctx* c, const float* A, uint64_t n_a, const float* B,
   const float* dB = B;
   mark_abs(*c, 24);  // start of the whole call (copies included)
   const bool undirected = (flags & HD_UNDIRECTED) != 0;
-  if ((s = init_scalars(*c)) != HD_OK) return s;
+  // Small sets that take the early-break scan by their sizes or by name (with
+  // its deferral cap left to the table).
+  bool small = small_apply(n_a, n_b, n_dims) && c->opt.eb_cap_pairs == 0;
+  if (small && variant != HD_VARIANT_EB) {
+    int va = variant, vb = variant;
+    small = variant == HD_VARIANT_AUTO && select_variant_by_size(*c, n_a, n_b, n_dims, &va) &&
+            va == HD_VARIANT_EB && select_variant_by_size(*c, n_b, n_a, n_dims, &vb);
+  }
+  if (!small && (s = init_scalars(*c)) != HD_OK) return s;
   if (!(flags & HD_DEVICE_PTRS)) {
     // An undirected solve known (from the sizes alone) to take the LBVH in
     // both directions sorts A while B is still being copied.
@@ -551,7 +559,10 @@ hd_status hd_solve(hd_ctx* c, const float* A, uint64_t n_a, const float* B,
     c->boxes_known = cells_state.ran;
     return r;
   };
-  if (variant == HD_VARIANT_AUTO) {
+  if (small) {
+    used[0] = used[1] = HD_VARIANT_EB;
+    cells = false;
+  } else if (variant == HD_VARIANT_AUTO) {
     Selection sel;
     c->ev_base = 0;
     if ((s = select_begin(*c, ins, ndir, used, &sel)) != HD_OK) return s;
@@ -575,6 +586,14 @@ hd_status hd_solve(hd_ctx* c, const float* A, uint64_t n_a, const float* B,
   const bool fused = undirected && used[0] == HD_VARIANT_LBVH && used[1] == HD_VARIANT_LBVH;
   auto run_all = [&]() -> hd_status {
     hd_status r;
+    if (small) {
+      c->ev_base = 0;
+      for (int k = 0; k <= 3; ++k) mark(*c, k);
+      have_result = true;
+      r = small_solve(*c, ins, ndir);
+      for (int k = 4; k <= 6; ++k) mark(*c, k);
+      return r;
+    }
     if (cells) {
       // What the cell filter left: lists go to the LBVH; a direction whose
       // answer is too few cells is filtered on a finer grid; sets that it
@@ -657,7 +676,7 @@ hd_status hd_solve(hd_ctx* c, const float* A, uint64_t n_a, const float* B,
   // a CUDA graph and later ones replay it (no per-kernel launch cost).
   // Timed solves (HD_TIMING) always launch directly.
   auto graphable = [&](int v) { return v == HD_VARIANT_LBVH || v == HD_VARIANT_EB; };
-  const bool eligible = !c->timing && !cells && graphable(used[0]) && (!undirected || graphable(used[1]));
+  const bool eligible = !c->timing && !cells && !small && graphable(used[0]) && (!undirected || graphable(used[1]));
   const uint64_t key[11] = {(uint64_t) dA, (uint64_t) dB, n_a, n_b, (uint64_t) n_dims, flags,
                             (uint64_t) (int64_t) used[0], (uint64_t) (int64_t) used[1],
                             (uint64_t) c->stream, c->buf_gen, 1};
@@ -715,8 +734,9 @@ hd_status hd_solve(hd_ctx* c, const float* A, uint64_t n_a, const float* B,
                         c->stream);
   if (e != cudaSuccess) return cuda_fail(*c, e, "copy result");
   mark_abs(*c, 25);
-  if (!have_result || c->timing) e = cudaStreamSynchronize(c->stream);
+  if (!have_result || small || c->timing) e = cudaStreamSynchronize(c->stream);
   if (e != cudaSuccess) return cuda_fail(*c, e, "solve");
+  c->small_clean |= small;
   if ((s = check_status(*c, *h, ndir)) != HD_OK) return s;
 
   const DevScalars& r0 = h->s[0];
@@ -761,7 +781,7 @@ hd_status hd_solve(hd_ctx* c, const float* A, uint64_t n_a, const float* B,
     const int from[6] = {0, 1, 2, 3, 4, 5};
     const int to[6] = {1, 2, 3, 4, 5, 6};
     // The fused pass records its phases once, on direction 0's events.
-    for (int d = 0; d < (fused ? 1 : ndir); ++d)
+    for (int d = 0; d < (fused || small ? 1 : ndir); ++d)
       for (int p = 0; p < 6; ++p) {
         if (cudaEventElapsedTime(&t, c->ev[12 * d + from[p]], c->ev[12 * d + to[p]]) ==
             cudaSuccess)

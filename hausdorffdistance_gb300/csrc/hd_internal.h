@@ -122,6 +122,7 @@ enum BufSlot {
   kBufF64A,       // FP64 input path: caller's double A / B on the device
   kBufF64B,
   kBufF64Aux,     // FP64 scalars and candidate lists
+  kBufSmall,      // small solves: running minima
   kBufCells,      // cell filter: bitmaps and lists
   kBufLeft,       // sorted points that the cell filter left open
   kBufF64Rows,    // FP64 nearest distance and column of every walked row
@@ -209,6 +210,7 @@ struct Ctx {
   void* sel_pinned = nullptr;    // pinned staging of the selector's samples
   size_t sel_pinned_bytes = 0;
   cudaEvent_t sel_event = nullptr;  // after the samples' copy
+  bool small_clean = false;  // kBufSmall is ready for a small solve
   bool cells_live = false;  // kernels yet to be enqueued read kBufCells
   cudaEvent_t cells_event = nullptr;  // after the copy of the filter's seeds
   void* batch_pinned = nullptr;  // pinned staging of grouped batch results
@@ -329,6 +331,11 @@ hd_status select_finish(Ctx& c, const DirInput* ins, int ndir, int* v, const Sel
 // The selector's choice when the sizes alone decide it (no sampling of the
 // data); false when it needs the sample pass.
 bool select_variant_by_size(const Ctx& c, uint64_t nA, uint64_t nB, int dims, int* variant);
+
+// Small sets (hd_small.cu): the whole solve in one kernel, which writes both
+// DevScalars to the pinned staging; no scalars are needed on the device.
+bool small_apply(uint64_t nA, uint64_t nB, int dims);
+hd_status small_solve(Ctx& c, const DirInput* ins, int ndir);
 
 // FP64 input path (hd_f64.cu) and its hooks into the LBVH solve.
 // A row of a list: the caller's row index and its FP32 nearest squared
