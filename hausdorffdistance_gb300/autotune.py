@@ -267,7 +267,7 @@ def write_table(params, path):
         f.write(f"#define HD_TUNED_EB_SMALL_PAIRS {params['eb_small_pairs']:.6g}\n")
         f.write(f"#define HD_TUNED_INDEX_MIN_PAIRS {params['index_min_pairs']:.6g}\n")
         f.write(f"#define HD_TUNED_EB_RATIO {params['eb_ratio']:.6g}\n")
-        f.write("#define HD_TUNED_BF16_MIN_PAIRS 67108864.0\n")
+        f.write("#define HD_TUNED_BF16_MIN_PAIRS 2000000.0\n")
         f.write(f"#define HD_TUNED_EB_SAMPLE_MAX_PAIRS {params['eb_sample_max_pairs']:.6g}\n")
         f.write(f"#define HD_TUNED_GRID_MAX_OUTSIDE {params['grid_max_outside']:.6g}\n")
         f.write(f"#define HD_TUNED_GRID_MAX_SKEW {params['grid_max_skew']:.6g}\n")

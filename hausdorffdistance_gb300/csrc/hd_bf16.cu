@@ -1,5 +1,6 @@
-// Split-BF16 tensor-core variant for high-dimensional inputs (n_dims a
-// multiple of 16, up to 256).  No counterpart in the reference, which only
+// Split-BF16 tensor-core variant for high-dimensional inputs: n_dims 16, 32, 48
+// or 64 by name, any up to 64 (padded with zeros) when AUTO chooses it.  No
+// counterpart in the reference, which only
 // handles n_dims 2 and 3 (src/main.cpp:134-135).
 //
 // ||a - b||^2 = ||a||^2 + ||b||^2 - 2 a.b.  Each coordinate is split into
@@ -606,11 +607,12 @@ __global__ void k_bf16_values(uint32_t* __restrict__ rowmin, const float* __rest
 // squared distance's bits (non-negative floats order like their bits).
 __global__ void __launch_bounds__(256)
     k_bf16_recheck(const float* __restrict__ A, const float* __restrict__ B, uint64_t nB, int D,
-                   const uint32_t* __restrict__ list, const Bf16Scalars* bs,
+                   const uint32_t* __restrict__ list, const Bf16Scalars* bs, uint32_t limit,
                    uint32_t* __restrict__ cand_min) {
   __shared__ __align__(16) float sa[256];
   __shared__ uint32_t red[8];
   const uint32_t n = bs->cand;
+  if (n > limit) return;
   const bool vec = (D % 4) == 0 && ((reinterpret_cast<uintptr_t>(B) & 15) == 0);
   for (uint32_t e = blockIdx.y; e < n; e += gridDim.y) {
     const uint32_t ia = list[e];
@@ -652,8 +654,10 @@ __global__ void __launch_bounds__(256)
 }
 
 __global__ void k_bf16_recheck_final(const uint32_t* __restrict__ list, const Bf16Scalars* bs,
-                                     const uint32_t* __restrict__ cand_min, DevScalars* sc) {
+                                     uint32_t limit, const uint32_t* __restrict__ cand_min,
+                                     DevScalars* sc) {
   const uint32_t n = bs->cand;
+  if (n > limit) return;
   for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x)
     atomicMax(&sc->max_key, pack_max(__uint_as_float(cand_min[e]), list[e]));
 }
@@ -816,10 +820,17 @@ hd_status run_bf16_k(Ctx& c, const DirInput& in, DirResult* extra, float* rowmin
                                                    (uint32_t*) cand, &bs->cand);
   if ((s = after_launch(c, "bf16_candidates")) != HD_OK) return s;
   DevScalars* sc = scalars(c, in.dir);
+  // A re-scanned row reads all of B; with more candidates than this (rows that
+  // nearly tie, or coordinates so far from the origin that the bound exceeds
+  // their distances) the early-break scan is the cheaper way to the same
+  // answer.
+  const uint32_t limit = (uint32_t) (in.nA / 32 + 256);
   k_bf16_recheck<<<dim3(c.num_sms * 2, 16), 256, 0, c.stream>>>(in.A, in.B, in.nB, in.dims,
-                                                               (const uint32_t*) cand, bs, cand_min);
+                                                               (const uint32_t*) cand, bs, limit,
+                                                               cand_min);
   if ((s = after_launch(c, "bf16_recheck")) != HD_OK) return s;
-  k_bf16_recheck_final<<<c.num_sms, 256, 0, c.stream>>>((const uint32_t*) cand, bs, cand_min, sc);
+  k_bf16_recheck_final<<<c.num_sms, 256, 0, c.stream>>>((const uint32_t*) cand, bs, limit,
+                                                       cand_min, sc);
   if ((s = after_launch(c, "bf16_recheck_final")) != HD_OK) return s;
   // Bound and recheck statistics for the result (small copy, after the work).
   Bf16Scalars h;
@@ -851,13 +862,14 @@ hd_status run_bf16_k(Ctx& c, const DirInput& in, DirResult* extra, float* rowmin
     extra->err_bound = 2.0 * (2.0 * cK * b * b + std::ldexp(1.0, -21) * sq +
                               (Kp + 2.0) * std::ldexp(1.0, -24) * sq);
   }
+  if (h.cand > limit) return run_eb_nd(c, in);
   return certify(c, in);
 }
 
 hd_status run_bf16_impl(Ctx& c, const DirInput& in, DirResult* extra, float* rowmin_host) {
-  if (in.dims % 16 != 0 || in.dims > 256)
-    return fail(c, HD_ERR_UNSUPPORTED, "the BF16 variant needs n_dims % 16 == 0 and <= 256");
-  switch (in.dims) {
+  // Rows are padded with zeros to a multiple of 16; by name (hd_solve checks it)
+  // the variant takes multiples of 16 only.
+  switch ((in.dims + 15) / 16 * 16) {
   case 16: return run_bf16_k<16>(c, in, extra, rowmin_host);
   case 32: return run_bf16_k<32>(c, in, extra, rowmin_host);
   case 48: return run_bf16_k<48>(c, in, extra, rowmin_host);
@@ -873,6 +885,8 @@ hd_status run_bf16(Ctx& c, const DirInput& in, DirResult* extra) {
 }
 
 hd_status bf16_rowmin_debug(Ctx& c, const DirInput& in, float* rowmin_host) {
+  if (in.dims % 16 != 0 || in.dims > 256)
+    return fail(c, HD_ERR_UNSUPPORTED, "the BF16 variant needs n_dims % 16 == 0 and <= 256");
   return run_bf16_impl(c, in, nullptr, rowmin_host);
 }
 

@@ -46,9 +46,10 @@
 //      eb_small_pairs take EB and problems from index_min_pairs up take the
 //      LBVH, both without sampling (at the largest sizes the grid's worst
 //      cases cost tens of times the LBVH while its best cases save ~20%);
-//      inputs with n_dims other than 2 or 3 take the split-BF16 tiles when
-//      n_dims is a multiple of 16 and the pair count is large, else the FP32
-//      scan.
+//      inputs with n_dims other than 2 or 3 take the split-BF16 tiles (padded
+//      with zeros to a multiple of 16) when n_dims is at most 64 and the pair
+//      count is large, else the FP32 scan.  10-D unit rows, 60,000 x 50,000:
+//      7.6 ms by the scan, 0.54 by the tiles; 24-D, 9,000 x 8,000: 0.80 and 0.12.
 //   All thresholds come from the autotuner's table
 //   (hausdorffdistance_gb300/autotune.py fits them over a sweep of
 //   workloads); hd_options.eb_only_threshold overrides eb_ratio.
@@ -246,7 +247,10 @@ bool select_variant_by_size(const Ctx& c, uint64_t nA, uint64_t nB, int dims, in
   const Tuning& tu = tuning();
   const double pairs = (double) nA * (double) nB;
   if (dims != 2 && dims != 3) {
-    *v = (dims % 16 == 0 && pairs >= tu.bf16_min_pairs) ? HD_VARIANT_BF16 : HD_VARIANT_EB;
+    // The tiles take about 95 us per direction at least; the scan passes that at
+    // 1.4e6 pairs in 10-D, 4e6 in 4-D.
+    const double least = tu.bf16_min_pairs * (dims <= 8 ? 2.0 : 1.0);
+    *v = ((dims % 16 == 0 || dims <= 64) && pairs >= least) ? HD_VARIANT_BF16 : HD_VARIANT_EB;
     return true;
   }
   const bool sample = c.opt.always_sample != 0;

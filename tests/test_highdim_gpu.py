@@ -114,3 +114,24 @@ def test_bf16_runs_of_tiles(engine, na, nb, dims, kind):
         d2 = hd_oracle.exact(a, b, 32)[0]
     assert np.float32(r.hd_f32) == np.sqrt(np.float32(d2))
     assert hd_oracle.dist2_f32(a[r.ia], b[r.ib]) == np.float32(d2)
+
+
+# AUTO pads rows to a multiple of 16 for the tiles; rows far from the origin,
+# whose bound exceeds their distances, and rows that all tie go back to the scan.
+@pytest.mark.parametrize("dims", [1, 4, 5, 10, 24, 31, 33, 63])
+@pytest.mark.parametrize("kind", ["plain", "far_from_origin", "all_tie"])
+def test_auto_pads_to_tiles(engine, dims, kind):
+    rng = np.random.default_rng(dims)
+    a = rng.random((2105, dims)).astype(np.float32)
+    b = (rng.random((1999, dims)) * 1.05).astype(np.float32)
+    if kind == "far_from_origin":
+        a, b = a + np.float32(300.0), b + np.float32(300.0)
+    elif kind == "all_tie":
+        a[:] = a[0]
+        b[:] = a[0] + np.float32(0.25)
+    r = engine.solve(a, b, undirected=True)
+    want = hd_oracle.hd_f32(a, b, undirected=True)
+    assert np.float32(r.hd_f32) == want["hd_f32"]
+    src, dst = (a, b) if r.direction == 0 else (b, a)
+    assert hd_oracle.dist2_f32(src[r.ia], dst[r.ib]) == want["d2"]
+    assert r.variant_used == 4
