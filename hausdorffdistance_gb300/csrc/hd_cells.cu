@@ -621,6 +621,21 @@ __global__ void __launch_bounds__(kSearchThreads) k_cell_seed(CellArgs a) {
   if ((threadIdx.x & 31) == 0) raise_level(d.st, lb);
 }
 
+// A direction's running maximum from L: a key of that distance and no row,
+// below the key of any row at h, so that a scan or an index may stop its
+// queries at L from the start.
+template <class Ge>
+__device__ __forceinline__ void start_at_level(const CellDir& d, const CellGrid& g) {
+  const float L2 = __uint_as_float(d.st->L2) * (g.side * g.side) * 0.9999f;
+  if (g.valid && d.soft_r < 0.0f && L2 > 0.0f)
+    atomicMax(&d.sc->max_key, (unsigned long long) __float_as_uint(L2) << 32);
+}
+
+template <class Ge>
+__global__ void k_cell_level(CellArgs a) {
+  if (threadIdx.x < a.count) start_at_level<Ge>(a.d[threadIdx.x], cell_grid<Ge>(a.ord));
+}
+
 // For a cell at each of the 64 places of a block, the cells of neighbour j (of
 // 3^D) that lie within `stop` at the far corner, as masks of its 64 cells; the
 // first 64 threads of a CTA.
@@ -658,11 +673,7 @@ __global__ void __launch_bounds__(256) k_cell_blocks(CellArgs a) {
   if (!(stop >= kMinReach * kMinReach * D)) {
     if (blockIdx.x == 0 && threadIdx.x == 0) {
       d.st->off = 1u;
-      // The index that takes over may stop its queries at L from the start: a
-      // key of that distance and no row, below the key of any row at h.
-      const float L2 = __uint_as_float(d.st->L2) * (g.side * g.side) * 0.9999f;
-      if (g.valid && d.soft_r < 0.0f && L2 > 0.0f)
-        atomicMax(&d.sc->max_key, (unsigned long long) __float_as_uint(L2) << 32);
+      start_at_level<Ge>(d, g);  // for the index that takes over
     }
     return;
   }
@@ -1146,7 +1157,7 @@ namespace {
 
 template <class Ge>
 hd_status enqueue(Ctx& c, const DirInput* ins, int count, const F64Plan* plan, CellArgs& a,
-                  bool boxes_known, bool* no_room) {
+                  bool boxes_known, bool seeds_only, bool* no_room) {
   const uint64_t n[2] = {ins[0].nA, ins[0].nB};
   hd_status s;
   // Zeroed words first: state, occupied cells, U, N, maps of marked blocks.
@@ -1164,7 +1175,8 @@ hd_status enqueue(Ctx& c, const DirInput* ins, int count, const F64Plan* plan, C
     o_any[k] = take(coarse);
     o_top[k] = take(Ge::kShared ? 0 : 32768);
   }
-  for (int k = 0; k < count; ++k) {
+  const int lists = seeds_only ? 0 : count;
+  for (int k = 0; k < lists; ++k) {
     o_U[k] = take(fine);
     o_N[k] = take(fine);
   }
@@ -1174,7 +1186,7 @@ hd_status enqueue(Ctx& c, const DirInput* ins, int count, const F64Plan* plan, C
     o_coarse[k] = take(coarse);
     o_code[k] = take((n[k] + 3) / 4 * 16);
   }
-  for (int k = 0; k < count; ++k) {
+  for (int k = 0; k < lists; ++k) {
     const uint64_t cc = std::min(n[k], kCapCells);
     const uint64_t cq = cap_queries(n[k]), ct = cap_targets(n[1 - k]);
     o_cells[k] = take(cc * 4);
@@ -1211,6 +1223,10 @@ hd_status enqueue(Ctx& c, const DirInput* ins, int count, const F64Plan* plan, C
     d.nQ = ins[k].nA;
     d.nT = ins[k].nB;
     d.qset = k;
+    d.st = (CellDirState*) base + k;
+    d.sc = scalars(c, ins[k].dir);
+    d.soft_r = plan ? plan->soft_r[k] : -1.0f;
+    if (seeds_only) continue;
     d.U = (unsigned long long*) (base + o_U[k]);
     d.N = (unsigned long long*) (base + o_N[k]);
     d.cells = (uint32_t*) (base + o_cells[k]);
@@ -1224,9 +1240,6 @@ hd_status enqueue(Ctx& c, const DirInput* ins, int count, const F64Plan* plan, C
     d.cap_cells = (uint32_t) std::min(ins[k].nA, kCapCells);
     d.cap_q = (uint32_t) cap_queries(ins[k].nA);
     d.cap_t = (uint32_t) cap_targets(ins[k].nB);
-    d.st = (CellDirState*) base + k;
-    d.sc = scalars(c, ins[k].dir);
-    d.soft_r = plan ? plan->soft_r[k] : -1.0f;
   }
   if (count == 1) a.d[1] = a.d[0];
   cudaError_t e = cudaMemsetAsync(base, 0, zero_bytes, c.stream);
@@ -1250,6 +1263,10 @@ hd_status enqueue(Ctx& c, const DirInput* ins, int count, const F64Plan* plan, C
   if ((s = after_launch(c, "cell_coarse")) != HD_OK) return s;
   k_cell_seed<Ge><<<dim3(kSeedWarps / kSearchWarps, dirs), kSearchThreads, 0, c.stream>>>(a);
   if ((s = after_launch(c, "cell_seed")) != HD_OK) return s;
+  if (seeds_only) {
+    k_cell_level<Ge><<<1, 32, 0, c.stream>>>(a);
+    return after_launch(c, "cell_level");
+  }
   // What the seeds found, for the host to act on while the rest runs.
   if (!c.cells_event) {
     if ((e = cudaEventCreateWithFlags(&c.cells_event, cudaEventDisableTiming)) != cudaSuccess)
@@ -1310,7 +1327,7 @@ hd_status cells_begin(Ctx& c, const DirInput* ins, int count, int level, const F
   bool no_room = false;
   *run = CellsRun{};
   auto go = [&](auto grid) {
-    return enqueue<decltype(grid)>(c, ins, count, plan, a, boxes_known, &no_room);
+    return enqueue<decltype(grid)>(c, ins, count, plan, a, boxes_known, false, &no_room);
   };
   hd_status s;
   if (ins[0].dims == 3)
@@ -1328,6 +1345,16 @@ hd_status cells_begin(Ctx& c, const DirInput* ins, int count, int level, const F
     run->cap_t[k] = a.d[k].cap_t;
   }
   return HD_OK;
+}
+
+hd_status cells_seed(Ctx& c, const DirInput* ins, int count, bool* seeded) {
+  CellArgs a{};
+  bool no_room = false;
+  const hd_status s =
+      ins[0].dims == 3 ? enqueue<Geo<3, 8>>(c, ins, count, nullptr, a, false, true, &no_room)
+                       : enqueue<Geo<2, 12>>(c, ins, count, nullptr, a, false, true, &no_room);
+  *seeded = s == HD_OK && !no_room;
+  return s;
 }
 
 hd_status cells_hopeless(Ctx& c, int count, int dims, const CellsRun& run, bool* off,

@@ -352,6 +352,13 @@ hd_status run_direction(Ctx& c, const DirInput& in, int variant, int* used,
   }
 }
 
+// Early-break scans of at least this many points per direction (|A| + |B| over
+// the directions, which share the cost) start from the cell filter's lower
+// bound (35 us): directed 3-D clusters 20,000 x 20,000 125 us without and 140 with
+// it, 40,000 x 30,000 152 and 167, 1M x 1M 2.5 and 1.2 ms; undirected 40,000 x
+// 40,000 306 and 272 us.
+constexpr uint64_t kSeedMinPoints = 80000;
+
 hd_status check_status(Ctx& c, const HostScalars& h, int ndir) {
   for (int d = 0; d < ndir; ++d) {
     uint32_t st = h.s[d].status;
@@ -662,6 +669,13 @@ hd_status hd_solve(hd_ctx* c, const float* A, uint64_t n_a, const float* B,
       if ((r = run_lbvh_pair(*c, ins[0], ins[1])) != HD_OK) return r;
       mark(*c, 6);
     } else {
+      // The early-break scan starts from the cell filter's lower bound.
+      if (used[0] == HD_VARIANT_EB && (n_dims == 2 || n_dims == 3) &&
+          (n_a + n_b) * ndir >= kSeedMinPoints) {
+        bool seeded = false;
+        if ((r = cells_seed(*c, ins, ndir, &seeded)) != HD_OK) return r;
+        for (int d = 0; d < ndir; ++d) c->seeded[d] |= seeded;
+      }
       for (int d = 0; d < ndir; ++d) {
         c->ev_base = 12 * d;
         mark(*c, 0);

@@ -25,7 +25,8 @@
 //    running maximum — and the seeds that start the maximum (the first 152
 //    visited points, before the main pass, so that it never starts from a
 //    zero threshold; the reference's hybrid seeds it with an MBR lower bound
-//    and a sample, hybrid.h:111-142) are finished by the tile-wise list
+//    and a sample, hybrid.h:111-142; larger sets start from the cell filter's
+//    bound instead, hd_cells.cu) are finished by the tile-wise list
 //    scan k_eb_list: groups of up to 256 points against chunks of B's tiles
 //    staged in shared memory; a group raises the running maximum as soon as
 //    its last chunk is done, so later groups break early.
@@ -671,9 +672,16 @@ hd_status run_eb_dim(Ctx& c, const DirInput& in) {
     // clamp(|B| / div, min, max) from the tuning table.  Pausing is not only
     // a tail guard: a paused point resumes under a higher running maximum.
     uint64_t cap = c.opt.eb_cap_pairs;
-    if (cap == 0)
-      cap = std::min<uint64_t>(std::max<uint64_t>(in.nB / tuning().eb_cap_div, tuning().eb_cap_min),
+    if (cap == 0) {
+      // A 3-D scan that starts near its final maximum settles most points in a
+      // tile or two; what is left holds whole CTAs until the cap (1M clusters:
+      // 1.19 ms with the table's cap of 4,096 pairs, 1.03 with half; 2-D points,
+      // which need thousands of pairs, only move from one kernel to the other).
+      const uint64_t half = D == 3 && c.seeded[in.dir] ? 2 : 1;
+      cap = std::min<uint64_t>(std::max<uint64_t>(in.nB / (tuning().eb_cap_div * half),
+                                                  tuning().eb_cap_min / half),
                                tuning().eb_cap_max);
+    }
     uint32_t capTiles = (uint32_t) std::max<uint64_t>(1, cap / kEbTile);
     const float* a_ptr = in.A;
     const PT* b_ptr = (const PT*) pb;

@@ -401,6 +401,9 @@ struct CellsRun {
 };
 hd_status cells_begin(Ctx& c, const DirInput* ins, int count, int level, const F64Plan* plan,
                       bool boxes_known, CellsRun* run);
+// The filter's seeds alone: starts the directions' running maxima at their L
+// (seeded: false when there was no room).  Takes no read-back.
+hd_status cells_seed(Ctx& c, const DirInput* ins, int count, bool* seeded);
 // Waits for the filter's seeds alone: off[k] where it will give direction k up
 // (reach[k]: its L in cells), so that the index can be enqueued behind it.
 hd_status cells_hopeless(Ctx& c, int count, int dims, const CellsRun& run, bool* off,

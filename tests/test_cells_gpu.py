@@ -90,6 +90,19 @@ def test_shapes(engine, kind, d):
     check(b, a, engine.solve(b, a, variant="lbvh", count_pairs=True, timing=True), False)
 
 
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("d", [2, 3])
+def test_early_break_starts_from_the_cells(engine, kind, d):
+    # The scan's running maximum starts at the filter's bound, which no row has;
+    # the third identical solve replays a graph.
+    rng = np.random.default_rng(d * 300 + KINDS.index(kind))
+    a, b = (np.ascontiguousarray(x, np.float32) for x in shapes(kind, d, rng))
+    for _ in range(3):
+        check(a, b, engine.solve(a, b, undirected=True, variant="eb"), True)
+    a, b = np.tile(a, (2, 1)), np.tile(b, (2, 1))
+    check(a, b, engine.solve(a, b, variant="eb", count_pairs=True), False)
+
+
 @pytest.mark.parametrize("kind", [k for k in KINDS if k not in ("huge", "beyond_the_grid")])
 @pytest.mark.parametrize("d", [2, 3])
 def test_shapes_f64(engine, kind, d):
