@@ -179,6 +179,10 @@ struct CellArgs {
   uint32_t* any[2];             // blocks with a cell that U or N marks in this set
   uint32_t* top[2];             // and super-blocks with such a block (large maps only)
   int count;                    // directions
+  CellDirState* seen;           // pinned host memory: state after the listing of cells,
+  CellDirState* left;           // and at the end
+  const DevScalars* sc0;        // DevScalars of direction 0
+  DevScalars* result;           // pinned host memory: results of finished directions
   CellDir d[2];
 };
 
@@ -221,6 +225,7 @@ template <class Ge, bool FIRST>
 __global__ void __launch_bounds__(256) k_cell_occ(CellArgs a, const float* __restrict__ A,
                                                   uint64_t nA, const float* __restrict__ B,
                                                   uint64_t nB, uint32_t every) {
+  chain_wait();
   constexpr int D = Ge::D;
   const CellGrid g = cell_grid<Ge>(a.ord);
   if (!g.valid) return;
@@ -285,6 +290,7 @@ __device__ __forceinline__ uint32_t half_cell(int bx, int by, int bz, int x, int
 // occupied cells of twice the size (a block of them covers 2^3 blocks).
 template <class Ge>
 __global__ void __launch_bounds__(256) k_cell_coarse(CellArgs a) {
+  chain_wait();
   const uint32_t block = blockIdx.x * 256 + threadIdx.x;
   const unsigned long long w = a.occ[blockIdx.y][block];
   const unsigned m = __ballot_sync(0xFFFFFFFFu, w != 0);
@@ -597,6 +603,7 @@ __device__ __forceinline__ const uint32_t* search_map(const uint32_t* __restrict
 // one cell of one of its occupied blocks.
 template <class Ge>
 __global__ void __launch_bounds__(kSearchThreads) k_cell_seed(CellArgs a) {
+  chain_wait();
   const CellDir& d = a.d[blockIdx.y];
   const CellGrid g = cell_grid<Ge>(a.ord);
   if (!g.valid) return;
@@ -666,6 +673,7 @@ __device__ __forceinline__ void near_masks(float stop, int j, unsigned long long
 // are listed.  The first CTAs also write down the masks of k_cell_near.
 template <class Ge>
 __global__ void __launch_bounds__(256) k_cell_blocks(CellArgs a) {
+  chain_wait();
   constexpr int D = Ge::D;
   const CellDir& d = a.d[blockIdx.y];
   const CellGrid g = cell_grid<Ge>(a.ord);
@@ -674,8 +682,14 @@ __global__ void __launch_bounds__(256) k_cell_blocks(CellArgs a) {
     if (blockIdx.x == 0 && threadIdx.x == 0) {
       d.st->off = 1u;
       start_at_level<Ge>(d, g);  // for the index that takes over
+      a.seen[blockIdx.y].L2 = d.st->L2;
+      a.seen[blockIdx.y].off = 1u;
     }
     return;
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    a.seen[blockIdx.y].L2 = d.st->L2;
+    a.seen[blockIdx.y].off = d.st->off;  // a query without a cell
   }
   constexpr int kN = D == 3 ? 27 : 9;
   if (blockIdx.x < kN)
@@ -775,6 +789,7 @@ __global__ void __launch_bounds__(256) k_cell_blocks(CellArgs a) {
 // their nearest target one or two blocks beyond the touching ones.
 template <class Ge, bool HALF>
 __global__ void __launch_bounds__(256) k_cell_near(CellArgs a) {
+  chain_wait();
   constexpr int D = Ge::D;
   constexpr int NB = HALF ? Ge::NB / 2 : Ge::NB;
   constexpr int kN = D == 3 ? 27 : 9;
@@ -829,6 +844,7 @@ constexpr uint32_t kManyFar = 24576;
 
 template <class Ge>
 __global__ void __launch_bounds__(kSearchThreads) k_cell_search(CellArgs a) {
+  chain_wait();
   const CellDir& d = a.d[blockIdx.y];
   if (d.st->off) return;
   const uint32_t n = d.st->n_far;
@@ -894,6 +910,7 @@ __device__ __forceinline__ void mark_block(uint32_t* any, uint32_t* top, uint32_
 
 template <class Ge>
 __global__ void __launch_bounds__(kSearchThreads) k_cell_mark(CellArgs a) {
+  chain_wait();
   constexpr int D = Ge::D;
   __shared__ uint32_t s_cell[kMarkChunk];
   __shared__ float s_ub[kMarkChunk];
@@ -991,6 +1008,7 @@ template <class Ge>
 __global__ void __launch_bounds__(256) k_cell_collect(CellArgs a, const float* __restrict__ A,
                                                       uint64_t nA, const float* __restrict__ B,
                                                       uint64_t nB) {
+  chain_wait();
   constexpr int D = Ge::D;
   const int set = blockIdx.y;
   const bool ask = set < a.count && !a.d[set].st->off;               // direction `set`
@@ -1055,12 +1073,16 @@ __device__ __forceinline__ bool scan_takes(const CellDirState* st, uint32_t cap_
 // finish takes the maximum over the queries and writes the direction's result.
 template <class Ge, bool COUNT>
 __global__ void __launch_bounds__(256) k_cell_solve(CellArgs a) {
+  chain_wait();
   constexpr int D = Ge::D;
   __shared__ float4 s[kScanTile];
   __shared__ unsigned long long red[2][8];
   __shared__ bool s_last;
   const CellDir& d = a.d[blockIdx.y];
-  if (!scan_takes(d.st, d.cap_q, d.cap_t)) return;
+  if (!scan_takes(d.st, d.cap_q, d.cap_t)) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) a.left[blockIdx.y] = *d.st;
+    return;
+  }
   const uint32_t nq = d.st->n_q, nt = d.st->n_t;
   const uint32_t qt = (nq + 255) / 256, tt = (nt + kScanTile - 1) / kScanTile;
   const uint64_t items = (uint64_t) qt * tt;
@@ -1127,6 +1149,19 @@ __global__ void __launch_bounds__(256) k_cell_solve(CellArgs a) {
     if (COUNT) d.sc->pairs += (unsigned long long) nq * nt;
     finalize_scalars(d.Q, d.T, D, d.sc);
     d.st->done = 1u;
+    // The words that the host reads.
+    DevScalars* o = a.result + (d.sc - a.sc0);
+    o->d2_64 = d.sc->d2_64;
+    o->d2 = d.sc->d2;
+    o->ia = d.sc->ia;
+    o->ib = d.sc->ib;
+    o->status = d.sc->status;
+    o->pairs = d.sc->pairs;
+    o->nodes = o->leaves = 0;
+    o->heavy_count = 0;
+    a.left[blockIdx.y].off = 0u;
+    a.left[blockIdx.y].done = 1u;
+    __threadfence_system();
   }
 }
 
@@ -1154,6 +1189,28 @@ bool cells_apply(const Ctx& c, uint64_t nA, uint64_t nB, int dims) {
 }
 
 namespace {
+
+// A launch behind the kernel before it (see chain_wait): its CTAs are on their
+// SMs when that kernel's last ones leave.  Eleven short kernels in a row: 200k
+// uniform 2-D points 144 -> 131 us, 1M clusters 220 -> 204, 10M 368 -> 348.  Not
+// for the kernels below that pass chain = false: the search's waiting CTAs
+// hold shared memory that the level before needs (5M 2-D points 374 -> 439 us),
+// the pass over the points ran slower when it started beside the marking (50M
+// planes 3.94 -> 4.33 ms), and the pair scan delays an index that waits behind
+// it (200k planes directed 294 -> 310 us).
+template <class... P, class... T>
+void launch_next(Ctx& c, bool chain, void (*kernel)(P...), dim3 grid, int threads, T... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3((unsigned) threads);
+  cfg.stream = c.stream;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = chain ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
 
 template <class Ge>
 hd_status enqueue(Ctx& c, const DirInput* ins, int count, const F64Plan* plan, CellArgs& a,
@@ -1216,6 +1273,10 @@ hd_status enqueue(Ctx& c, const DirInput* ins, int count, const F64Plan* plan, C
     a.top[k] = (uint32_t*) (base + o_top[k]);
   }
   a.count = count;
+  a.seen = (CellDirState*) ((char*) c.host_pinned + kStageSeeds);
+  a.left = (CellDirState*) ((char*) c.host_pinned + kStageState);
+  a.sc0 = scalars(c, 0);
+  a.result = (DevScalars*) c.host_pinned;
   for (int k = 0; k < count; ++k) {
     CellDir& d = a.d[k];
     d.Q = ins[k].A;
@@ -1250,58 +1311,60 @@ hd_status enqueue(Ctx& c, const DirInput* ins, int count, const F64Plan* plan, C
   // Passes over points: four points per thread.
   const unsigned gp = (unsigned) std::max<uint64_t>(
       1, std::min<uint64_t>((most / 4 + 255) / 256, (uint64_t) sms * 8));
+  // (Not while a solve is captured: the seeds alone run inside graphs.)
+  const bool chain = !seeds_only;
   const uint32_t every = n[0] + n[1] >= kOccSplit ? kOccFirst : 1u;
-  k_cell_occ<Ge, true><<<dim3(gp, 2), 256, 0, c.stream>>>(a, ins[0].A, ins[0].nA, ins[0].B,
-                                                          ins[0].nB, every);
+  launch_next(c, chain, k_cell_occ<Ge, true>, dim3(gp, 2), 256, a, ins[0].A, ins[0].nA, ins[0].B,
+              ins[0].nB, every);
   if ((s = after_launch(c, "cell_occ")) != HD_OK) return s;
   if (every > 1) {
-    k_cell_occ<Ge, false><<<dim3(gp, 2), 256, 0, c.stream>>>(a, ins[0].A, ins[0].nA, ins[0].B,
-                                                             ins[0].nB, every);
+    launch_next(c, chain, k_cell_occ<Ge, false>, dim3(gp, 2), 256, a, ins[0].A, ins[0].nA,
+                ins[0].B, ins[0].nB, every);
     if ((s = after_launch(c, "cell_occ")) != HD_OK) return s;
   }
-  k_cell_coarse<Ge><<<dim3(Ge::kBlocks / 256, 2), 256, 0, c.stream>>>(a);
+  launch_next(c, chain, k_cell_coarse<Ge>, dim3(Ge::kBlocks / 256, 2), 256, a);
   if ((s = after_launch(c, "cell_coarse")) != HD_OK) return s;
-  k_cell_seed<Ge><<<dim3(kSeedWarps / kSearchWarps, dirs), kSearchThreads, 0, c.stream>>>(a);
+  launch_next(c, chain, k_cell_seed<Ge>, dim3(kSeedWarps / kSearchWarps, dirs), kSearchThreads, a);
   if ((s = after_launch(c, "cell_seed")) != HD_OK) return s;
   if (seeds_only) {
     k_cell_level<Ge><<<1, 32, 0, c.stream>>>(a);
     return after_launch(c, "cell_level");
   }
-  // What the seeds found, for the host to act on while the rest runs.
+  launch_next(c, chain, k_cell_blocks<Ge>,
+              dim3(std::min<unsigned>(Ge::kBlocks / 256, sms * 32), dirs), 256, a);
+  if ((s = after_launch(c, "cell_blocks")) != HD_OK) return s;
+  // What the seeds found is in pinned memory now, for the host to act on while
+  // the rest runs.
   if (!c.cells_event) {
     if ((e = cudaEventCreateWithFlags(&c.cells_event, cudaEventDisableTiming)) != cudaSuccess)
       return cuda_fail(c, e, "filter event");
   }
-  e = cudaMemcpyAsync((char*) c.host_pinned + kStageSeeds, base, 2 * sizeof(CellDirState),
-                      cudaMemcpyDeviceToHost, c.stream);
-  if (e == cudaSuccess) e = cudaEventRecord(c.cells_event, c.stream);
-  if (e != cudaSuccess) return cuda_fail(c, e, "filter seeds");
-  k_cell_blocks<Ge><<<dim3(std::min<unsigned>(Ge::kBlocks / 256, sms * 32), dirs), 256, 0, c.stream>>>(
-      a);
-  if ((s = after_launch(c, "cell_blocks")) != HD_OK) return s;
+  if ((e = cudaEventRecord(c.cells_event, c.stream)) != cudaSuccess)
+    return cuda_fail(c, e, "filter event");
   const dim3 gw(sms * 6 / dirs, dirs);  // searches: six CTAs with the map per SM
   const dim3 gn(sms * 8 / dirs, dirs);
-  k_cell_near<Ge, false><<<gn, 256, 0, c.stream>>>(a);
+  launch_next(c, chain, k_cell_near<Ge, false>, gn, 256, a);
   if ((s = after_launch(c, "cell_near")) != HD_OK) return s;
   if constexpr (Ge::D == 3) {
-    k_cell_near<Ge, true><<<gn, 256, 0, c.stream>>>(a);
+    launch_next(c, chain, k_cell_near<Ge, true>, gn, 256, a);
     if ((s = after_launch(c, "cell_near")) != HD_OK) return s;
   }
-  k_cell_search<Ge><<<gw, kSearchThreads, 0, c.stream>>>(a);
+  launch_next(c, false, k_cell_search<Ge>, gw, kSearchThreads, a);
   if ((s = after_launch(c, "cell_search")) != HD_OK) return s;
-  k_cell_mark<Ge><<<gw, kSearchThreads, 0, c.stream>>>(a);
+  launch_next(c, chain, k_cell_mark<Ge>, gw, kSearchThreads, a);
   if ((s = after_launch(c, "cell_mark")) != HD_OK) return s;
   mark(c, 1);
-  k_cell_collect<Ge><<<dim3(gp, 2), 256, 0, c.stream>>>(a, ins[0].A, ins[0].nA, ins[0].B, ins[0].nB);
+  launch_next(c, false, k_cell_collect<Ge>, dim3(gp, 2), 256, a, ins[0].A, ins[0].nA, ins[0].B,
+              ins[0].nB);
   if ((s = after_launch(c, "cell_collect")) != HD_OK) return s;
   mark(c, 2);
   mark(c, 3);
   if (!plan) {
     const dim3 gs(sms * 4, dirs);
     if (ins[0].count)
-      k_cell_solve<Ge, true><<<gs, 256, 0, c.stream>>>(a);
+      launch_next(c, false, k_cell_solve<Ge, true>, gs, 256, a);
     else
-      k_cell_solve<Ge, false><<<gs, 256, 0, c.stream>>>(a);
+      launch_next(c, false, k_cell_solve<Ge, false>, gs, 256, a);
     if ((s = after_launch(c, "cell_solve")) != HD_OK) return s;
   }
   mark(c, 4);
@@ -1336,6 +1399,7 @@ hd_status cells_begin(Ctx& c, const DirInput* ins, int count, int level, const F
     s = level == 0 ? go(Geo<2, 12>{}) : level == 1 ? go(Geo<2, 13>{}) : go(Geo<2, 14>{});
   if (s != HD_OK || no_room) return s;
   run->ran = true;
+  run->wrote = plan == nullptr;
   c.cells_live = true;
   run->state = a.d[0].st;
   for (int k = 0; k < count; ++k) {
@@ -1378,16 +1442,14 @@ hd_status cells_hopeless(Ctx& c, int count, int dims, const CellsRun& run, bool*
   return HD_OK;
 }
 
-hd_status cells_finish(Ctx& c, int count, bool scalars_too, const CellsRun& run, CellsLeft* left) {
+hd_status cells_finish(Ctx& c, int count, const CellsRun& run, CellsLeft* left) {
   for (int k = 0; k < count; ++k) left[k] = CellsLeft{};
   if (!run.ran) return HD_OK;
   CellDirState* h = reinterpret_cast<CellDirState*>((char*) c.host_pinned + kStageState);
   static_assert(2 * sizeof(CellDirState) <= 512, "pinned staging");
-  cudaError_t e = cudaMemcpyAsync(h, run.state, 2 * sizeof(CellDirState), cudaMemcpyDeviceToHost,
-                                  c.stream);
-  if (e == cudaSuccess && scalars_too)
-    e = cudaMemcpyAsync(c.host_pinned, scalars(c, 0), 2 * sizeof(DevScalars), cudaMemcpyDeviceToHost,
-                        c.stream);
+  cudaError_t e = cudaSuccess;
+  if (!run.wrote)  // no pair scan, which would have written it there
+    e = cudaMemcpyAsync(h, run.state, 2 * sizeof(CellDirState), cudaMemcpyDeviceToHost, c.stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(c.stream);
   if (e != cudaSuccess) return cuda_fail(c, e, "cell filter");
   c.cells_live = false;  // but for the lists below

@@ -146,6 +146,15 @@ __device__ __forceinline__ float soft_stop(float thr, float r) {
   return g > 0.0f ? g : -1.0f;
 }
 
+// A kernel of a chain launched with programmatic stream serialization: lets the
+// next kernel's CTAs take their places now, and waits until the kernels before
+// have finished and their writes are visible.  (No effect in a kernel launched
+// without the attribute.)
+__device__ __forceinline__ void chain_wait() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // Error bits written to the context's device status word.
 enum : uint32_t {
   kErrWaitTimeout = 1u,   // an mbarrier / flag wait hit its iteration cap

@@ -624,7 +624,12 @@ hd_status hd_solve(hd_ctx* c, const float* A, uint64_t n_a, const float* B,
           if (indexed[d] && (r = run_direction(*c, ins[d], used[d], &used[d], &ex[d])) != HD_OK)
             return r;
       }
-      if ((r = cells_finish(*c, ndir, true, cells_state, left)) != HD_OK) return r;
+      if (indexed[0] || indexed[1]) {  // else the filter's kernels write the results there
+        const cudaError_t e = cudaMemcpyAsync(c->host_pinned, c->bufs[kBufScalars].p,
+                                              sizeof(HostScalars), cudaMemcpyDeviceToHost, c->stream);
+        if (e != cudaSuccess) return cuda_fail(*c, e, "copy result");
+      }
+      if ((r = cells_finish(*c, ndir, cells_state, left)) != HD_OK) return r;
       have_result = cells_state.ran;
       for (int d = 0; d < ndir; ++d) left[d].done |= indexed[d];
       for (int d = 0; d < ndir; ++d)
@@ -642,7 +647,7 @@ hd_status hd_solve(hd_ctx* c, const float* A, uint64_t n_a, const float* B,
         if (finer >= 0) {
           CellsRun again;
           if ((r = cells_begin(*c, &ins[d], 1, finer, nullptr, true, &again)) != HD_OK) return r;
-          if ((r = cells_finish(*c, 1, true, again, &fine)) != HD_OK) return r;
+          if ((r = cells_finish(*c, 1, again, &fine)) != HD_OK) return r;
         }
         if (!fine.done && fine.narrowed) {
           if ((r = run_lbvh_left(*c, &ins[d], 1, nullptr, &fine)) != HD_OK) return r;

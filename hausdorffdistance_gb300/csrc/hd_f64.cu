@@ -825,7 +825,7 @@ hd_status hd_solve_f64(hd_ctx* c, const double* A, uint64_t n_a, const double* B
     if (cells_apply(*c, n_a, n_b, n_dims)) {
       CellsRun run;
       if ((s = cells_begin(*c, ins, ndir, cells_level(n_a + n_b, n_dims), &plan, true, &run)) != HD_OK) return s;
-      if ((s = cells_finish(*c, ndir, false, run, left)) != HD_OK) return s;
+      if ((s = cells_finish(*c, ndir, run, left)) != HD_OK) return s;
       narrowed = true;
       for (int k = 0; k < ndir; ++k) narrowed &= left[k].narrowed && left[k].nq <= kListCap;
     }

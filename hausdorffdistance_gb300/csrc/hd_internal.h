@@ -388,12 +388,14 @@ int cells_level(uint64_t points, int dims);
 int cells_finer(uint64_t points, int dims, int level, float reach);
 // Filters `count` directions: the call's (ins[k].dir == k), or one of them.  With a plan, queries are
 // settled by the FP64 listing pass's level, and no direction is finished here.
-// scalars_too: also copies both DevScalars to the pinned staging.  boxes_known:
-// DevScalars[0].mbr_ord already holds the sets' boxes.
+// Without a plan the results of finished directions are in the pinned staging
+// (DevScalars by direction).  boxes_known: DevScalars[0].mbr_ord already holds
+// the sets' boxes.
 //   cells_begin enqueues the filter, cells_finish waits for the stream and
 //   reads what it left (begin's `ran` false: there was no room for its lists).
 struct CellsRun {
   bool ran = false;
+  bool wrote = false;           // the kernels write the state to the pinned staging
   const void* state = nullptr;  // device words to read back
   const float4* q[2];
   const float4* t[2];
@@ -408,7 +410,7 @@ hd_status cells_seed(Ctx& c, const DirInput* ins, int count, bool* seeded);
 // (reach[k]: its L in cells), so that the index can be enqueued behind it.
 hd_status cells_hopeless(Ctx& c, int count, int dims, const CellsRun& run, bool* off,
                          float* reach);
-hd_status cells_finish(Ctx& c, int count, bool scalars_too, const CellsRun& run, CellsLeft* left);
+hd_status cells_finish(Ctx& c, int count, const CellsRun& run, CellsLeft* left);
 // LBVH over what the filter left of `count` directions.
 hd_status run_lbvh_left(Ctx& c, const DirInput* ins, int count, F64Plan* plan,
                         const CellsLeft* left);
