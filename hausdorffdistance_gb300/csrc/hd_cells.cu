@@ -136,19 +136,6 @@ __device__ __forceinline__ uint32_t cell_of(const CellGrid& g, float x, float y,
   }
 }
 
-// One direction of the filter (device words are zeroed before each solve).
-struct CellDirState {
-  uint32_t L2;       // float bits: squared lower bound of h in cell units
-  uint32_t off;      // the filter gave up
-  uint32_t n_cells;  // cells of open blocks,
-  uint32_t n_rim;    // those without a target cell near by (3-D),
-  uint32_t n_far;    // and those without one twice as far
-  uint32_t n_q;      // open queries
-  uint32_t n_t;      // and collected targets (counts may exceed the lists)
-  uint32_t done;     // the pair scan finished the direction
-  uint32_t ticket;   // its CTAs that are through
-};
-
 struct CellDir {
   const float* Q;
   const float* T;
@@ -630,11 +617,11 @@ __global__ void __launch_bounds__(kSearchThreads) k_cell_seed(CellArgs a) {
 
 // A direction's running maximum from L: a key of that distance and no row,
 // below the key of any row at h, so that a scan or an index may stop its
-// queries at L from the start.
+// queries at L from the start (the FP64 listing pass at soft_stop(L)).
 template <class Ge>
 __device__ __forceinline__ void start_at_level(const CellDir& d, const CellGrid& g) {
   const float L2 = __uint_as_float(d.st->L2) * (g.side * g.side) * 0.9999f;
-  if (g.valid && d.soft_r < 0.0f && L2 > 0.0f)
+  if (g.valid && L2 > 0.0f)
     atomicMax(&d.sc->max_key, (unsigned long long) __float_as_uint(L2) << 32);
 }
 
@@ -1070,7 +1057,8 @@ __device__ __forceinline__ bool scan_takes(const CellDirState* st, uint32_t cap_
 // 256 queries (one per thread) by kScanTile targets (through shared memory),
 // each query's nearest target (lowest row among ties: every target at its
 // distance was collected) by one 64-bit atomicMin per item.  The last CTA to
-// finish takes the maximum over the queries and writes the direction's result.
+// finish takes the maximum over the queries and writes the direction's result
+// (with a plan, only that maximum).
 template <class Ge, bool COUNT>
 __global__ void __launch_bounds__(256) k_cell_solve(CellArgs a) {
   chain_wait();
@@ -1144,6 +1132,12 @@ __global__ void __launch_bounds__(256) k_cell_solve(CellArgs a) {
         best = red[0][k];
         pair = red[1][k];
       }
+    if (d.soft_r >= 0.0f) {  // the FP64 path goes on from here
+      d.st->max32 = (uint32_t) (best >> 32);
+      d.st->scanned = 1u;
+      if (COUNT) d.sc->pairs += (unsigned long long) nq * nt;
+      return;
+    }
     d.sc->max_key = best;
     d.sc->min_key = pair;
     if (COUNT) d.sc->pairs += (unsigned long long) nq * nt;
@@ -1359,14 +1353,12 @@ hd_status enqueue(Ctx& c, const DirInput* ins, int count, const F64Plan* plan, C
   if ((s = after_launch(c, "cell_collect")) != HD_OK) return s;
   mark(c, 2);
   mark(c, 3);
-  if (!plan) {
-    const dim3 gs(sms * 4, dirs);
-    if (ins[0].count)
-      launch_next(c, false, k_cell_solve<Ge, true>, gs, 256, a);
-    else
-      launch_next(c, false, k_cell_solve<Ge, false>, gs, 256, a);
-    if ((s = after_launch(c, "cell_solve")) != HD_OK) return s;
-  }
+  const dim3 gs(sms * 4, dirs);
+  if (ins[0].count)
+    launch_next(c, false, k_cell_solve<Ge, true>, gs, 256, a);
+  else
+    launch_next(c, false, k_cell_solve<Ge, false>, gs, 256, a);
+  if ((s = after_launch(c, "cell_solve")) != HD_OK) return s;
   mark(c, 4);
   mark(c, 5);
   return HD_OK;
@@ -1403,6 +1395,7 @@ hd_status cells_begin(Ctx& c, const DirInput* ins, int count, int level, const F
   c.cells_live = true;
   run->state = a.d[0].st;
   for (int k = 0; k < count; ++k) {
+    run->q_min[k] = a.d[k].q_min;
     run->q[k] = a.d[k].q;
     run->t[k] = a.d[k].t;
     run->cap_q[k] = a.d[k].cap_q;
@@ -1448,7 +1441,7 @@ hd_status cells_finish(Ctx& c, int count, const CellsRun& run, CellsLeft* left) 
   CellDirState* h = reinterpret_cast<CellDirState*>((char*) c.host_pinned + kStageState);
   static_assert(2 * sizeof(CellDirState) <= 512, "pinned staging");
   cudaError_t e = cudaSuccess;
-  if (!run.wrote)  // no pair scan, which would have written it there
+  if (!run.wrote)
     e = cudaMemcpyAsync(h, run.state, 2 * sizeof(CellDirState), cudaMemcpyDeviceToHost, c.stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(c.stream);
   if (e != cudaSuccess) return cuda_fail(c, e, "cell filter");

@@ -27,14 +27,17 @@
 //     So that pass stops a row only at or below G(running maximum) and lists
 //     every row that stays open with its FP32 minimum; each row with an FP32
 //     minimum > T is listed.
-//  5. Each listed row with an FP32 minimum > T FP64 nearest neighbour is found by a walk of the
-//     same tree, one warp per row: boxes and points are tested in FP32
+//  5. The FP64 nearest neighbour of each listed row with an FP32 minimum > T is
+//     found by a walk of the same tree, one warp per row: boxes and points are tested in FP32
 //     against a float threshold P derived from the row's best FP64 distance
 //     (anything above P is provably farther in FP64), and only points within
 //     P get an FP64 distance.  A walk stops once its best (an upper bound of
 //     its distance) is strictly below the running FP64 maximum (seeded with
 //     L).  The answer is the largest completed distance, the lowest row
 //     among equal ones, and that row's lowest column.
+// When the cell filter left few queries and targets (hd_cells.cu), its pair
+// scan has the FP32 minima of step 2, and k_f64_left does the rest without an
+// index: rows above G(M), their pairs within P, and the FP64 distances of those.
 // When the list overflows (rows that nearly all tie: a lattice and its
 // translate) step 5 walks every row.  Other n_dims, coordinates beyond
 // +-1e18 and the eb / brute variants use an FP64 scan instead.
@@ -66,6 +69,8 @@ constexpr unsigned long long kRangeBits = 0x43ABC16D674EC800ull;
 constexpr uint32_t kF64NonFinite = 1u, kF64Range = 2u, kF64Tiny = 4u;
 constexpr double kMargin = 0x1p-40;
 constexpr int kScanThreads = 128;
+constexpr uint32_t kPairCap = 16384;   // pairs that one CTA finishes in FP64
+constexpr uint32_t kLeftTile = 1024;   // targets per item
 constexpr int kWalkWarps = 4;
 constexpr int kWalkStack = 2048;  // stack entries per warp (shared memory)
 
@@ -83,6 +88,10 @@ struct F64Dir {
   float thr;                 // T: listed rows at or below it are settled (-1: none)
   uint32_t status;           // kErr* of the FP64 kernels
   uint32_t walked;           // rows whose nearest neighbour was searched in FP64
+  uint32_t n_rows;           // k_f64_left: rows above G(M),
+  uint32_t n_pairs;          // pairs found (may exceed kPairCap),
+  uint32_t ticket;           // its CTAs that are through,
+  uint32_t finished;         // and whether max64 and pick are the answer
 };
 
 // Device layout of kBufF64Aux; the two candidate lists follow it.
@@ -271,6 +280,7 @@ __global__ void k_f64_init(F64Aux* aux) {
     z.thr = -1.0f;
     z.status = 0u;
     z.walked = 0u;
+    z.n_rows = z.n_pairs = z.ticket = z.finished = 0u;
     aux->dir[k] = z;
     aux->round[k].emax = 0u;
     aux->round[k].flags = 0u;
@@ -278,9 +288,9 @@ __global__ void k_f64_init(F64Aux* aux) {
 }
 
 // The seed rows: each direction's FP32-certified row and its FP32 minimum.
-__global__ void k_f64_seed_entries(const DevScalars* sc, F64Aux* aux, int count) {
-  const int k = threadIdx.x;
-  if (k < count) aux->seed[k] = RowEntry{sc[k].ia, __float_as_uint(sc[k].d2)};
+__global__ void k_f64_seed_entries(const DevScalars* sc, F64Aux* aux, int first, int count) {
+  const int k = first + threadIdx.x;
+  if (threadIdx.x < count) aux->seed[k] = RowEntry{sc[k].ia, __float_as_uint(sc[k].d2)};
 }
 
 // Rows walked by one launch (blockIdx.y = direction).
@@ -493,10 +503,9 @@ __global__ void __launch_bounds__(kWalkWarps * 32) k_f64_walk(WalkSets ws) {
 }
 
 // T from the seeds (thread per direction).
-__global__ void k_f64_prepare(F64Aux* aux, int count, int D, double rxy0, double rxy1) {
-  const int k = threadIdx.x;
-  if (k >= count) return;
-  const double rxy = k == 0 ? rxy0 : rxy1;
+__global__ void k_f64_prepare(F64Aux* aux, int first, int count, int D, double rxy) {
+  const int k = first + threadIdx.x;
+  if (threadIdx.x >= count) return;
   F64Dir& f = aux->dir[k];
   const double L = aux->seed_min[k];
   if (L < 0.0) f.status |= kErrInternal;  // a seed walk cannot stop
@@ -573,6 +582,153 @@ __global__ void __launch_bounds__(kScanThreads)
   atomicMax(&f->max64, dbits(best));
 }
 
+// What the cell filter's pair scan left of a direction.
+struct LeftArgs {
+  const double* X;              // query set, caller's rows
+  const double* Y;              // target set, caller's rows
+  const CellDirState* st;
+  const float4* q;              // open queries (cut x, y, z, row)
+  unsigned long long* q_min;    // their (FP32 minimum's bits, target row)
+  const float4* t;              // collected targets
+  struct Pair {
+    uint32_t e, j;              // entry in q, target row
+    double d;
+  }* pairs;                     // kPairCap of them
+  double rxy;
+  float soft_r;
+  F64Dir* f;
+};
+struct LeftSets {
+  LeftArgs d[2];
+};
+
+// The FP64 answer from the FP32 minima of all open queries.  Items of 256
+// queries by kLeftTile targets: queries above G(M) are kept (every other one is
+// below the FP64 distance of the row at M), their targets within P listed; the
+// last CTA computes the listed pairs in FP64, takes each query's minimum (in
+// q_min, whose FP32 minima are no longer needed), the maximum over the queries,
+// and the lowest row and column among ties.  A row's targets at its FP64 minimum are all
+// within P, and all collected.  Nothing is written when a list runs over
+// (rows that tie): the index takes the lists then.
+// Latency: reading the lists, a few FP64 pairs.  In place of the index over the
+// lists (sort, tree, query, two walks; 25 launches and two read-backs), 10M x 10M
+// clusters 907 -> 508 us, 300k x 400k 444 -> 222 (417 with no filter at all).
+template <int D>
+__global__ void __launch_bounds__(256) k_f64_left(LeftSets ls) {
+  __shared__ float4 s_q[256];
+  __shared__ float s_P[256];
+  __shared__ uint32_t s_e[256];
+  __shared__ uint32_t s_n;
+  __shared__ bool s_last, s_over;
+  __shared__ unsigned long long s_red[8];
+  const LeftArgs& a = ls.d[blockIdx.y];
+  if (!a.st->scanned) return;
+  const uint32_t nq = a.st->n_q, nt = a.st->n_t;
+  const uint32_t qt = (nq + 255) / 256, tt = (nt + kLeftTile - 1) / kLeftTile;
+  const uint64_t items = (uint64_t) qt * tt;
+  if (blockIdx.x >= items) return;
+  const float G = soft_stop(__uint_as_float(a.st->max32), a.soft_r);
+  for (uint64_t item = blockIdx.x; item < items; item += gridDim.x) {
+    const uint32_t q0 = (uint32_t) (item % qt) * 256, t0 = (uint32_t) (item / qt) * kLeftTile;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      s_n = 0;
+      s_over = __ldcg(&a.f->n_pairs) > kPairCap;
+    }
+    __syncthreads();
+    if (s_over) break;
+    const uint32_t e = q0 + threadIdx.x;
+    if (e < nq) {
+      const float m32 = __uint_as_float((uint32_t) (a.q_min[e] >> 32));
+      if (m32 > G) {
+        const uint32_t slot = atomicAdd(&s_n, 1u);
+        s_q[slot] = a.q[e];
+        s_P[slot] = prune32<D>(upper_from32<D>(m32, a.rxy), a.rxy);
+        s_e[slot] = e;
+      }
+    }
+    __syncthreads();
+    const uint32_t n = s_n;
+    if (n == 0) continue;
+    if (t0 == 0 && threadIdx.x == 0) atomicAdd(&a.f->n_rows, n);
+    const uint32_t m = min(kLeftTile, nt - t0);
+    bool over = false;
+    for (uint32_t i = threadIdx.x; i < m && !over; i += 256) {
+      const float4 t = a.t[t0 + i];
+      for (uint32_t c = 0; c < n && !over; ++c) {
+        const float q[3] = {s_q[c].x, s_q[c].y, s_q[c].z};
+        if (d2_32<D>(q, t) > s_P[c]) continue;
+        const uint32_t slot = atomicAdd(&a.f->n_pairs, 1u);
+        if (slot < kPairCap) a.pairs[slot] = LeftArgs::Pair{s_e[c], __float_as_uint(t.w), 0.0};
+        over = slot >= kPairCap;
+      }
+    }
+  }
+  __threadfence();
+  __syncthreads();
+  const uint32_t ctas = (uint32_t) min((uint64_t) gridDim.x, items);
+  if (threadIdx.x == 0) s_last = atomicAdd(&a.f->ticket, 1u) == ctas - 1;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  const uint32_t n = __ldcg(&a.f->n_pairs);
+  if (n == 0 || n > kPairCap) return;
+  for (uint32_t k = threadIdx.x; k < n; k += 256) {
+    const uint32_t e = __ldcg(&a.pairs[k].e), j = __ldcg(&a.pairs[k].j);
+    const uint64_t row = __float_as_uint(a.q[e].w);
+    double x[D], y[D];
+#pragma unroll
+    for (int i = 0; i < D; ++i) {
+      x[i] = a.X[row * D + i];
+      y[i] = a.Y[(uint64_t) j * D + i];
+    }
+    __stcg(&a.pairs[k].d, d2_64<D>(x, y));
+    __stcg(a.q_min + e, ~0ull);
+  }
+  __threadfence();
+  __syncthreads();
+  for (uint32_t k = threadIdx.x; k < n; k += 256)
+    atomicMin(a.q_min + __ldcg(&a.pairs[k].e), dbits(__ldcg(&a.pairs[k].d)));
+  __threadfence();
+  __syncthreads();
+  // The least value of the CTA.
+  auto cta_min = [&](unsigned long long v) {
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+      const unsigned long long w = __shfl_xor_sync(0xFFFFFFFFu, v, o);
+      v = w < v ? w : v;
+    }
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) s_red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    v = s_red[0];
+#pragma unroll
+    for (int k = 1; k < 8; ++k) v = s_red[k] < v ? s_red[k] : v;
+    return v;
+  };
+  unsigned long long v = ~0ull;
+  for (uint32_t k = threadIdx.x; k < n; k += 256) {
+    const unsigned long long w = ~__ldcg(a.q_min + __ldcg(&a.pairs[k].e));
+    v = w < v ? w : v;
+  }
+  const unsigned long long top = ~cta_min(v);
+  v = ~0ull;
+  for (uint32_t k = threadIdx.x; k < n; k += 256) {
+    const uint32_t e = __ldcg(&a.pairs[k].e);
+    if (dbits(__ldcg(&a.pairs[k].d)) != top || __ldcg(a.q_min + e) != top) continue;
+    const unsigned long long w =
+        ((unsigned long long) __float_as_uint(a.q[e].w) << 32) | __ldcg(&a.pairs[k].j);
+    v = w < v ? w : v;
+  }
+  v = cta_min(v);
+  if (threadIdx.x == 0) {
+    a.f->max64 = top;
+    a.f->pick = v;
+    a.f->walked = __ldcg(&a.f->n_rows);
+    a.f->finished = 1u;
+  }
+}
+
 // The answer: the lowest row whose completed distance equals the maximum
 // (and its column); the seed row takes part when it has one.
 __global__ void k_f64_pick(const double* __restrict__ row_min, const uint32_t* __restrict__ row_col,
@@ -602,14 +758,41 @@ __global__ void k_f64_pick(const double* __restrict__ row_min, const uint32_t* _
 
 // Per-call host state shared with f64_seed.
 struct F64Call {
-  const double* X[2];
+  const double* X[2];  // by direction
   const double* Y[2];
-  double rxy[2];
+  double rxy;
   int dims;
+  int first;           // direction of the plan's first entry
   F64Aux* aux;
-  double* seed_min;
-  uint32_t* seed_col;
 };
+
+// k_f64_left behind the cell filter; the pairs are kept where an index pass
+// would list its rows.
+hd_status finish_left(Ctx& c, const CellsRun& run, const F64Call& call, const F64Plan& plan,
+                      int count, RowEntry* lists) {
+  static_assert(kPairCap * sizeof(LeftArgs::Pair) <= kListCap * sizeof(RowEntry), "pairs");
+  LeftSets ls;
+  for (int k = 0; k < count; ++k) {
+    LeftArgs& a = ls.d[k];
+    a.X = call.X[k];
+    a.Y = call.Y[k];
+    a.st = run.state + k;
+    a.q = run.q[k];
+    a.q_min = run.q_min[k];
+    a.t = run.t[k];
+    a.pairs = (LeftArgs::Pair*) (lists + (size_t) k * kListCap);
+    a.rxy = call.rxy;
+    a.soft_r = plan.soft_r[k];
+    a.f = &call.aux->dir[k];
+  }
+  if (count == 1) ls.d[1] = ls.d[0];
+  const dim3 grid(c.num_sms * 4, count);
+  if (call.dims == 2)
+    k_f64_left<2><<<grid, 256, 0, c.stream>>>(ls);
+  else
+    k_f64_left<3><<<grid, 256, 0, c.stream>>>(ls);
+  return after_launch(c, "f64_left");
+}
 
 hd_status launch_walks(Ctx& c, const WalkSets& ws, int count, uint64_t max_rows, int dims) {
   if (max_rows == 0) return HD_OK;
@@ -661,27 +844,28 @@ hd_status status_of(Ctx& c, uint32_t st) {
 // directions are certified).
 hd_status f64_seed(Ctx& c, F64Plan& plan, int count) {
   F64Call& call = *reinterpret_cast<F64Call*>(plan.state);
-  k_f64_seed_entries<<<1, 32, 0, c.stream>>>(scalars(c, 0), call.aux, count);
+  const int first = call.first;
+  k_f64_seed_entries<<<1, 32, 0, c.stream>>>(scalars(c, 0), call.aux, first, count);
   hd_status s = after_launch(c, "f64_seed_entries");
   if (s != HD_OK) return s;
   WalkSets ws;
   for (int k = 0; k < count; ++k) {
+    const int d = first + k;
     WalkArgs& w = ws.d[k];
-    w.X = call.X[k];
-    w.Y = call.Y[k];
+    w.X = call.X[d];
+    w.Y = call.Y[d];
     w.t = plan.tree[k];
-    w.list = &call.aux->seed[k];
+    w.list = &call.aux->seed[d];
     w.n_rows = 1;
-    w.rxy = call.rxy[k];
-    w.f = &call.aux->dir[k];
-    w.row_min = call.seed_min + k;
-    w.row_col = call.seed_col + k;
-    w.status = &call.aux->dir[k].status;
+    w.rxy = call.rxy;
+    w.f = &call.aux->dir[d];
+    w.row_min = call.aux->seed_min + d;
+    w.row_col = call.aux->seed_col + d;
+    w.status = &call.aux->dir[d].status;
   }
   if (count == 1) ws.d[1] = ws.d[0];
   if ((s = launch_walks(c, ws, count, 1, call.dims)) != HD_OK) return s;
-  k_f64_prepare<<<1, 32, 0, c.stream>>>(call.aux, count, call.dims, call.rxy[0],
-                                        count > 1 ? call.rxy[1] : 0.0);
+  k_f64_prepare<<<1, 32, 0, c.stream>>>(call.aux, first, count, call.dims, call.rxy);
   return after_launch(c, "f64_prepare");
 }
 
@@ -765,6 +949,15 @@ hd_status hd_solve_f64(hd_ctx* c, const double* A, uint64_t n_a, const double* B
   c->boxes_known = spatial_dims;
   static_assert(sizeof(F64Aux) + 1024 <= 4096, "pinned staging");
   F64Aux* h = reinterpret_cast<F64Aux*>((char*) c->host_pinned + 1024);
+  DevScalars* hs = reinterpret_cast<DevScalars*>(c->host_pinned);
+  static_assert(2 * sizeof(DevScalars) <= 1024, "pinned staging");
+  auto copy_back = [&]() -> hd_status {
+    cudaError_t e = cudaMemcpyAsync(h, aux, sizeof(F64Aux), cudaMemcpyDeviceToHost, c->stream);
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(hs, scalars(*c, 0), 2 * sizeof(DevScalars), cudaMemcpyDeviceToHost,
+                          c->stream);
+    return e == cudaSuccess ? HD_OK : cuda_fail(*c, e, "f64 read-back");
+  };
   auto read_aux = [&]() -> hd_status {
     cudaError_t e = cudaMemcpyAsync(h, aux, sizeof(F64Aux), cudaMemcpyDeviceToHost, c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
@@ -791,91 +984,125 @@ hd_status hd_solve_f64(hd_ctx* c, const double* A, uint64_t n_a, const double* B
 
   int used = lbvh ? HD_VARIANT_LBVH : (variant == HD_VARIANT_BRUTE ? HD_VARIANT_BRUTE : HD_VARIANT_EB);
   uint64_t walked[2] = {0, 0};
+  bool finished = false;  // the answer has been read back already
   if (lbvh) {
     F64Call call;
     call.dims = n_dims;
     call.aux = aux;
-    call.seed_min = aux->seed_min;
-    call.seed_col = aux->seed_col;
+    call.rxy = (rset[0] + rset[1]) * (1.0 + kMargin);
+    // The bound as a float, rounded up.
+    float rf = (float) call.rxy;
+    if ((double) rf < call.rxy) rf = std::nextafter(rf, INFINITY);
     DirInput ins[2];
     for (int k = 0; k < ndir; ++k) {
       call.X[k] = d64[k];
       call.Y[k] = d64[1 - k];
-      call.rxy[k] = (rset[0] + rset[1]) * (1.0 + kMargin);
       ins[k] = DirInput{f32[k], nn[k], f32[1 - k], nn[1 - k], n_dims, k,
                         (flags & HD_COUNT_PAIRS) != 0};
     }
+    // The plan of directions first .. first + count - 1.
     F64Plan plan;
-    std::memset(&plan, 0, sizeof(plan));
-    plan.cand_cap = kListCap;
-    plan.state = &call;
-    for (int k = 0; k < ndir; ++k) {
-      plan.cand[k] = lists + (size_t) k * kListCap;
-      plan.cand_count[k] = &aux->dir[k].cand_count;
-      // The bound as a float, rounded up.
-      float rf = (float) call.rxy[k];
-      if ((double) rf < call.rxy[k]) rf = std::nextafter(rf, INFINITY);
-      plan.soft_r[k] = rf;
-    }
-    // The cell filter first, by the listing pass's level; the lists it leaves
-    // are searched in place of the sets when it narrowed every direction and no
-    // list of rows can overflow (then every row of the set would be walked).
+    auto plan_of = [&](int first, int count) {
+      std::memset(&plan, 0, sizeof(plan));
+      plan.cand_cap = kListCap;
+      plan.state = &call;
+      call.first = first;
+      for (int k = 0; k < count; ++k) {
+        plan.cand[k] = lists + (size_t) (first + k) * kListCap;
+        plan.cand_count[k] = &aux->dir[first + k].cand_count;
+        plan.soft_r[k] = rf;
+      }
+    };
+    // The index's listing pass over those directions' sets (or the filter's
+    // lists), and the walks of the rows that it listed, or of every row when a
+    // list overflowed (after the read-back of their counts).
+    auto index = [&](int first, int count, const CellsLeft* left) {
+      plan_of(first, count);
+      return left ? run_lbvh_left(*c, ins + first, count, &plan, left + first)
+                  : run_lbvh_f64(*c, ins + first, count, &plan);
+    };
+    auto walk = [&](int first, int count) -> hd_status {
+      uint64_t off[2] = {0, 0}, total = 0, most = 0;
+      for (int k = 0; k < count; ++k) {
+        const uint32_t listed = h->dir[first + k].cand_count;
+        walked[k] = listed <= kListCap ? listed : nn[first + k];
+        off[k] = total;
+        total += walked[k];
+        most = std::max(most, walked[k]);
+      }
+      void* rows;
+      hd_status r = ensure(*c, kBufF64Rows, total * (sizeof(double) + sizeof(uint32_t)) + 16, &rows);
+      if (r != HD_OK) return r;
+      double* row_min = (double*) rows;
+      uint32_t* row_col = (uint32_t*) (row_min + total);
+      WalkSets ws;
+      for (int k = 0; k < count; ++k) {
+        const int d = first + k;
+        WalkArgs& w = ws.d[k];
+        w.X = call.X[d];
+        w.Y = call.Y[d];
+        w.t = plan.tree[k];
+        w.list = h->dir[d].cand_count <= kListCap ? plan.cand[k] : nullptr;
+        w.n_rows = walked[k];
+        w.rxy = call.rxy;
+        w.f = &aux->dir[d];
+        w.row_min = row_min + off[k];
+        w.row_col = row_col + off[k];
+        w.status = &aux->dir[d].status;
+      }
+      if (count == 1) ws.d[1] = ws.d[0];
+      if ((r = launch_walks(*c, ws, count, most, n_dims)) != HD_OK) return r;
+      for (int k = 0; k < count; ++k)
+        if ((r = pick(*c, ws.d[k].row_min, ws.d[k].row_col, ws.d[k].list, walked[k],
+                      ws.d[k].f)) != HD_OK)
+          return r;
+      return HD_OK;
+    };
+    // The cell filter first, by the listing pass's level.  Short lists are
+    // finished pair by pair; others go to the index in place of the sets when
+    // no list of rows can overflow (then every row of the set would be walked).
+    // A direction that the filter's seeds rule out starts on the index behind
+    // the filter's other kernels.
+    bool open[2] = {true, undirected}, off[2] = {false, false};
     CellsLeft left[2];
-    bool narrowed = false;
     if (cells_apply(*c, n_a, n_b, n_dims)) {
       CellsRun run;
-      if ((s = cells_begin(*c, ins, ndir, cells_level(n_a + n_b, n_dims), &plan, true, &run)) != HD_OK) return s;
-      if ((s = cells_finish(*c, ndir, run, left)) != HD_OK) return s;
-      narrowed = true;
-      for (int k = 0; k < ndir; ++k) narrowed &= left[k].narrowed && left[k].nq <= kListCap;
+      float reach[2];
+      plan_of(0, ndir);
+      const int level = cells_level(n_a + n_b, n_dims);
+      if ((s = cells_begin(*c, ins, ndir, level, &plan, true, &run)) != HD_OK) return s;
+      if (run.ran) {
+        if ((s = finish_left(*c, run, call, plan, ndir, lists)) != HD_OK) return s;
+        if ((s = cells_hopeless(*c, ndir, n_dims, run, off, reach)) != HD_OK) return s;
+        const int first = off[0] ? 0 : 1, count = (off[0] ? 1 : 0) + (ndir > 1 && off[1] ? 1 : 0);
+        if (count && (s = index(first, count, nullptr)) != HD_OK) return s;
+        if ((s = copy_back()) != HD_OK) return s;
+        if ((s = cells_finish(*c, ndir, run, left)) != HD_OK) return s;
+        if (count && (s = walk(first, count)) != HD_OK) return s;
+        for (int k = 0; k < ndir; ++k) open[k] = !off[k] && !h->dir[k].finished;
+        finished = !count;
+      }
     }
-    if (!narrowed) c->cells_live = false;
-    s = narrowed ? run_lbvh_left(*c, ins, ndir, &plan, left) : run_lbvh_f64(*c, ins, ndir, &plan);
-    if (s != HD_OK) return s;
-    if ((s = read_aux()) != HD_OK) return s;
-    DevScalars hs[2];
-    cudaError_t e = cudaMemcpy(hs, scalars(*c, 0), sizeof(hs), cudaMemcpyDeviceToHost);
-    if (e != cudaSuccess) return cuda_fail(*c, e, "f64 read-back");
+    const int first = open[0] ? 0 : 1, count = (int) open[0] + (int) open[1];
+    if (count) {
+      bool narrowed = true;
+      for (int k = first; k < first + count; ++k)
+        narrowed &= left[k].narrowed && left[k].nq <= kListCap;
+      if (!narrowed) c->cells_live = false;
+      if ((s = index(first, count, narrowed ? left : nullptr)) != HD_OK) return s;
+      if ((s = copy_back()) != HD_OK) return s;
+      const cudaError_t e = cudaStreamSynchronize(c->stream);
+      if (e != cudaSuccess) return cuda_fail(*c, e, "f64 read-back");
+      if ((s = walk(first, count)) != HD_OK) return s;
+      finished = false;
+    }
+    c->cells_live = false;
     for (int k = 0; k < ndir; ++k) {
       if ((s = status_of(*c, hs[k].status | h->dir[k].status)) != HD_OK) return s;
       out->visited_pairs += hs[k].pairs;
       out->visited_nodes += hs[k].nodes;
       out->visited_leaves += hs[k].leaves;
     }
-    // Walk the listed rows, or every row when a list overflowed.
-    uint64_t off[2] = {0, 0}, total = 0;
-    for (int k = 0; k < ndir; ++k) {
-      walked[k] = h->dir[k].cand_count <= kListCap ? h->dir[k].cand_count : nn[k];
-      off[k] = total;
-      total += walked[k];
-    }
-    void* rows;
-    if ((s = ensure(*c, kBufF64Rows, total * (sizeof(double) + sizeof(uint32_t)) + 16, &rows)) !=
-        HD_OK)
-      return s;
-    double* row_min = (double*) rows;
-    uint32_t* row_col = (uint32_t*) (row_min + total);
-    WalkSets ws;
-    for (int k = 0; k < ndir; ++k) {
-      WalkArgs& w = ws.d[k];
-      w.X = call.X[k];
-      w.Y = call.Y[k];
-      w.t = plan.tree[k];
-      w.list = h->dir[k].cand_count <= kListCap ? plan.cand[k] : nullptr;
-      w.n_rows = walked[k];
-      w.rxy = call.rxy[k];
-      w.f = &aux->dir[k];
-      w.row_min = row_min + off[k];
-      w.row_col = row_col + off[k];
-      w.status = &aux->dir[k].status;
-    }
-    if (ndir == 1) ws.d[1] = ws.d[0];
-    if ((s = launch_walks(*c, ws, ndir, std::max(walked[0], walked[1]), n_dims)) != HD_OK)
-      return s;
-    for (int k = 0; k < ndir; ++k)
-      if ((s = pick(*c, ws.d[k].row_min, ws.d[k].row_col, ws.d[k].list, walked[k],
-                    &aux->dir[k])) != HD_OK)
-        return s;
   } else {
     void* rows;
     const uint64_t total = n_a + (undirected ? n_b : 0);
@@ -903,7 +1130,7 @@ hd_status hd_solve_f64(hd_ctx* c, const double* A, uint64_t n_a, const double* B
     }
   }
   if (c->timing) cudaEventRecord(c->ev[25], c->stream);
-  if ((s = read_aux()) != HD_OK) return s;
+  if ((!finished || c->timing) && (s = read_aux()) != HD_OK) return s;
   if (lbvh)
     for (int k = 0; k < ndir; ++k)
       if ((s = status_of(*c, h->dir[k].status)) != HD_OK) return s;

@@ -387,17 +387,33 @@ bool cells_apply(const Ctx& c, uint64_t nA, uint64_t nB, int dims);
 int cells_level(uint64_t points, int dims);
 int cells_finer(uint64_t points, int dims, int level, float reach);
 // Filters `count` directions: the call's (ins[k].dir == k), or one of them.  With a plan, queries are
-// settled by the FP64 listing pass's level, and no direction is finished here.
+// settled by the FP64 listing pass's level, and the pair scan leaves the open
+// queries' FP32 minima; no direction is finished here.
 // Without a plan the results of finished directions are in the pinned staging
 // (DevScalars by direction).  boxes_known: DevScalars[0].mbr_ord already holds
 // the sets' boxes.
 //   cells_begin enqueues the filter, cells_finish waits for the stream and
 //   reads what it left (begin's `ran` false: there was no room for its lists).
+// One direction of the filter, on the device (zeroed before each solve).
+struct CellDirState {
+  uint32_t L2;       // float bits: squared lower bound of h in cell units
+  uint32_t off;      // the filter gave up
+  uint32_t n_cells;  // cells of open blocks,
+  uint32_t n_rim;    // those without a target cell near by (3-D),
+  uint32_t n_far;    // and those without one twice as far
+  uint32_t n_q;      // open queries
+  uint32_t n_t;      // and collected targets (counts may exceed the lists)
+  uint32_t done;     // the pair scan finished the direction
+  uint32_t ticket;   // its CTAs that are through
+  uint32_t scanned;  // with a plan: q_min holds every open query's FP32 minimum
+  uint32_t max32;    // and this is the largest (float bits)
+};
 struct CellsRun {
   bool ran = false;
-  bool wrote = false;           // the kernels write the state to the pinned staging
-  const void* state = nullptr;  // device words to read back
+  bool wrote = false;  // the kernels write the state to the pinned staging
+  const CellDirState* state = nullptr;  // device words to read back
   const float4* q[2];
+  unsigned long long* q_min[2];  // per open query: (FP32 minimum's bits, target row)
   const float4* t[2];
   uint32_t cap_q[2], cap_t[2];
 };

@@ -115,6 +115,24 @@ def test_shapes_f64(engine, kind, d):
     assert (int(r.ia), int(r.ib)) == (win[1], win[2])
 
 
+@pytest.mark.parametrize("rows,cols", [(1, 1), (255, 64), (300, 20), (129, 127), (129, 128),
+                                       (3000, 2)])
+@pytest.mark.parametrize("d", [2, 3])
+def test_f64_rows_that_floats_cannot_order(engine, d, rows, cols):
+    # rows x cols pairs at the maximum to within float precision: finished pair
+    # by pair up to 16,384 of them, by the index beyond; half are exact copies.
+    rng = np.random.default_rng(d * 1000 + rows + cols)
+    a, b = rng.random((30_011, d)), rng.random((25_007, d)) * 1.05
+    a[rng.permutation(len(a))[:rows]] = 3.0 + 1e-10 * (np.arange(rows) // 2)[:, None]
+    b[rng.permutation(len(b))[:cols]] = 1.2 + 1e-10 * (np.arange(cols) // 2)[:, None]
+    for x, y in ((a, b), (b, a)):
+        r = engine.solve_f64(x, y, undirected=x is a)
+        want = [hd_oracle.exact_f64(x, y)] + ([hd_oracle.exact_f64(y, x)] if x is a else [])
+        assert r.hd_ab == np.sqrt(want[0][0])
+        win = max(want, key=lambda w: w[0])
+        assert (r.hd, int(r.ia), int(r.ib)) == (np.sqrt(win[0]), win[1], win[2])
+
+
 def test_nan_points_leave_their_direction_to_the_index(engine):
     # Targets with NaN coordinates are nobody's nearest neighbour, as before.
     rng = np.random.default_rng(4)
