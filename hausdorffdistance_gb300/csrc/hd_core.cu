@@ -99,6 +99,16 @@ hd_status ensure_side(Ctx& c) {
   return HD_OK;
 }
 
+hd_status ensure_index_side(Ctx& c) {
+  if (c.index_side) return HD_OK;
+  cudaError_t e;
+  if ((!c.index_join &&
+       (e = cudaEventCreateWithFlags(&c.index_join, cudaEventDisableTiming)) != cudaSuccess) ||
+      (e = cudaStreamCreateWithFlags(&c.index_side, cudaStreamNonBlocking)) != cudaSuccess)
+    return cuda_fail(c, e, "index stream");
+  return HD_OK;
+}
+
 DevScalars* scalars(Ctx& c, int dir) {
   return reinterpret_cast<DevScalars*>(c.bufs[kBufScalars].p) + dir;
 }
@@ -463,6 +473,8 @@ hd_status hd_destroy(hd_ctx* c) {
   if (c->sel_pinned) cudaFreeHost(c->sel_pinned);
   if (c->sel_event) cudaEventDestroy(c->sel_event);
   if (c->cells_event) cudaEventDestroy(c->cells_event);
+  if (c->index_side) cudaStreamDestroy(c->index_side);
+  if (c->index_join) cudaEventDestroy(c->index_join);
   if (c->batch_pinned) cudaFreeHost(c->batch_pinned);
   if (c->own_stream) cudaStreamDestroy(c->own_stream);
   delete c;
@@ -611,18 +623,27 @@ hd_status hd_solve(hd_ctx* c, const float* A, uint64_t n_a, const float* B,
       CellsLeft rest_left[2];
       int n = 0;
       // A direction that the filter's seeds already rule out (and that no finer
-      // grid takes) starts on its index behind the filter's other kernels.
+      // grid takes) starts on its index beside the filter's other kernels.
       bool off[2], indexed[2] = {false, false};
       float reach[2];
       if ((r = cells_hopeless(*c, ndir, n_dims, cells_state, off, reach)) != HD_OK) return r;
       for (int d = 0; d < ndir; ++d)
         indexed[d] = off[d] && cells_finer(n_a + n_b, n_dims, level, reach[d]) < 0;
-      if (indexed[0] && indexed[1] && fused) {
-        if ((r = run_lbvh_pair(*c, ins[0], ins[1])) != HD_OK) return r;
-      } else {
+      auto index = [&]() -> hd_status {
+        if (indexed[0] && indexed[1] && fused) return run_lbvh_pair(*c, ins[0], ins[1]);
         for (int d = 0; d < ndir; ++d)
           if (indexed[d] && (r = run_direction(*c, ins[d], used[d], &used[d], &ex[d])) != HD_OK)
             return r;
+        return HD_OK;
+      };
+      if (indexed[0] || indexed[1]) {
+        r = index_beside(*c, index);
+        if (r == HD_ERR_OOM) {  // after the filter then, with its room
+          c->last_error.clear();
+          indexed[0] = indexed[1] = false;
+        } else if (r != HD_OK) {
+          return r;
+        }
       }
       if (indexed[0] || indexed[1]) {  // else the filter's kernels write the results there
         const cudaError_t e = cudaMemcpyAsync(c->host_pinned, c->bufs[kBufScalars].p,

@@ -1061,7 +1061,7 @@ hd_status hd_solve_f64(hd_ctx* c, const double* A, uint64_t n_a, const double* B
     // The cell filter first, by the listing pass's level.  Short lists are
     // finished pair by pair; others go to the index in place of the sets when
     // no list of rows can overflow (then every row of the set would be walked).
-    // A direction that the filter's seeds rule out starts on the index behind
+    // A direction that the filter's seeds rule out starts on the index beside
     // the filter's other kernels.
     bool open[2] = {true, undirected}, off[2] = {false, false};
     CellsLeft left[2];
@@ -1074,8 +1074,18 @@ hd_status hd_solve_f64(hd_ctx* c, const double* A, uint64_t n_a, const double* B
       if (run.ran) {
         if ((s = finish_left(*c, run, call, plan, ndir, lists)) != HD_OK) return s;
         if ((s = cells_hopeless(*c, ndir, n_dims, run, off, reach)) != HD_OK) return s;
-        const int first = off[0] ? 0 : 1, count = (off[0] ? 1 : 0) + (ndir > 1 && off[1] ? 1 : 0);
-        if (count && (s = index(first, count, nullptr)) != HD_OK) return s;
+        const int first = off[0] ? 0 : 1;
+        int count = (off[0] ? 1 : 0) + (ndir > 1 && off[1] ? 1 : 0);
+        if (count) {
+          s = index_beside(*c, [&]() { return index(first, count, nullptr); });
+          if (s == HD_ERR_OOM) {  // after the filter then, with its room
+            c->last_error.clear();
+            off[0] = off[1] = false;
+            count = 0;
+          } else if (s != HD_OK) {
+            return s;
+          }
+        }
         if ((s = copy_back()) != HD_OK) return s;
         if ((s = cells_finish(*c, ndir, run, left)) != HD_OK) return s;
         if (count && (s = walk(first, count)) != HD_OK) return s;

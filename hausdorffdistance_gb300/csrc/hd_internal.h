@@ -212,7 +212,10 @@ struct Ctx {
   cudaEvent_t sel_event = nullptr;  // after the samples' copy
   bool small_clean = false;  // kBufSmall is ready for a small solve
   bool cells_live = false;  // kernels yet to be enqueued read kBufCells
-  cudaEvent_t cells_event = nullptr;  // after the copy of the filter's seeds
+  cudaEvent_t cells_event = nullptr;  // when the filter's seeds are in pinned memory
+  // A direction's index beside the rest of the filter (index_beside).
+  cudaStream_t index_side = nullptr;
+  cudaEvent_t index_join = nullptr;
   void* batch_pinned = nullptr;  // pinned staging of grouped batch results
   size_t batch_pinned_bytes = 0;
   std::string last_error;
@@ -299,6 +302,7 @@ hd_status ensure(Ctx& c, BufSlot slot, size_t bytes, void** out);
 hd_status after_launch(Ctx& c, const char* what);
 // Creates the context's side stream and fork/join events on first use.
 hd_status ensure_side(Ctx& c);
+hd_status ensure_index_side(Ctx& c);
 
 DevScalars* scalars(Ctx& c, int dir);
 
@@ -426,6 +430,24 @@ hd_status cells_seed(Ctx& c, const DirInput* ins, int count, bool* seeded);
 // (reach[k]: its L in cells), so that the index can be enqueued behind it.
 hd_status cells_hopeless(Ctx& c, int count, int dims, const CellsRun& run, bool* off,
                          float* reach);
+// Runs `index` on a stream of its own behind the filter's seeds, beside the
+// filter's other kernels (which work on the other direction, or return at once);
+// the call's stream waits for it.  Planes undirected, 300k x 500k 470 -> 442 us
+// against the same behind those kernels, FP64 200k x 300k 524 -> 469.
+template <class F>
+hd_status index_beside(Ctx& c, F index) {
+  hd_status s = ensure_index_side(c);
+  if (s != HD_OK) return s;
+  cudaError_t e = cudaStreamWaitEvent(c.index_side, c.cells_event, 0);
+  if (e != cudaSuccess) return cuda_fail(c, e, "index stream");
+  const cudaStream_t main = c.stream;
+  c.stream = c.index_side;
+  s = index();
+  c.stream = main;
+  e = cudaEventRecord(c.index_join, c.index_side);
+  if (e == cudaSuccess) e = cudaStreamWaitEvent(main, c.index_join, 0);
+  return s == HD_OK && e != cudaSuccess ? cuda_fail(c, e, "index stream") : s;
+}
 hd_status cells_finish(Ctx& c, int count, const CellsRun& run, CellsLeft* left);
 // LBVH over what the filter left of `count` directions.
 hd_status run_lbvh_left(Ctx& c, const DirInput* ins, int count, F64Plan* plan,
