@@ -178,6 +178,7 @@ struct BatchArgs {
   float* wb_b;                     // window bound per row of B (direction B->A)
   LongRow* longq;
   unsigned long long* long_count;
+  unsigned long long* taken;       // directions taken by the CTA and the one-warp path
   uint64_t long_cap;
   uint32_t small_rows;             // one-warp path: directions up to this many rows
   uint32_t pipe_rows;              // CTA path up to this many rows; multi-pass pipeline above
@@ -267,10 +268,69 @@ __device__ __forceinline__ float scan_run(const float* __restrict__ X, uint32_t 
   return cmin;
 }
 
+// A row's window bound: its minimum over the w0 points of its window.  The
+// tuned window of 5 points, away from the ends, takes its loads at once.
+template <int D>
+__device__ __forceinline__ float window_bound(const float* __restrict__ X, uint32_t row,
+                                              const float* __restrict__ Y, float ratio,
+                                              uint32_t ny, uint32_t w0) {
+  uint32_t j = scan_start(row, ratio, ny, w0 >> 1);
+  if (w0 != 5 || j > ny - 5) return scan_run<D>(X, row, Y, j, ny, w0, INFINITY);
+  float x[D], y[5][D];
+  load_pt<D>(X, row, x);
+#pragma unroll
+  for (int u = 0; u < 5; ++u) load_pt<D>(Y + (uint64_t) j * D, u, y[u]);
+  float m = d2_of<D>(x, y[0]);
+#pragma unroll
+  for (int u = 1; u < 5; ++u) m = fminf(m, d2_of<D>(x, y[u]));
+  return fminf(m, INFINITY);
+}
+
+// A lane's largest bound above `floor` so far and its row (the first among
+// equal ones when rows come in ascending order).
+struct TopRow {
+  float u;
+  uint32_t row;
+  __device__ __forceinline__ void add(float v, uint32_t r) {
+    if (v > u) {
+      u = v;
+      row = r;
+    }
+  }
+  __device__ __forceinline__ unsigned long long key(float floor) const {
+    return u > floor ? pack_max(u, row) : 0ull;
+  }
+};
+
+// A lane's nearest point so far, the lowest index among ties (ascending j).
+struct NearPoint {
+  float d;
+  uint32_t j;
+  __device__ __forceinline__ void add(float v, uint32_t at) {
+    if (v < d) {
+      d = v;
+      j = at;
+    }
+  }
+};
+
 __device__ __forceinline__ float warp_min(float v) {
 #pragma unroll
   for (int o = 16; o; o >>= 1) v = fminf(v, __shfl_xor_sync(0xFFFFFFFFu, v, o));
   return v;
+}
+
+__device__ __forceinline__ unsigned long long warp_max_key(unsigned long long v) {
+#pragma unroll
+  for (int o = 16; o; o >>= 1) {
+    const unsigned long long w = __shfl_xor_sync(0xFFFFFFFFu, v, o);
+    v = w > v ? w : v;
+  }
+  return v;
+}
+
+__device__ __forceinline__ unsigned long long warp_min_key(unsigned long long v) {
+  return ~warp_max_key(~v);
 }
 
 // Window pass, one item: each row's minimum over 2*window+1 points of the
@@ -526,9 +586,15 @@ __global__ void __launch_bounds__(kBatchThreads) k_batch_long(BatchArgs a) {
 // One-warp path: a warp solves a whole problem-direction of at most
 // small_rows query rows with the same steps as the multi-pass pipeline —
 // window bounds (stored per row and read back by the lane that wrote them),
-// the 8 residue-class seeds, the sweep with early break, open rows scanned by
-// the whole warp — with no pass boundary in between.  Warps take
-// problem-directions in plan order.
+// the rows of the largest bounds, the sweep with early break, open rows scanned
+// by the whole warp — with no pass boundary in between.  Warps take
+// problem-directions in plan order from a queue: with fixed shares 40 % of the
+// SMs' time went by idle at 30,000 polylines, behind the blocks with the longest
+// ones.  Bound by latency (L1 hits 75 %, 0.5 instructions per cycle and
+// scheduler; more warps or more loads in flight measured slower): what counts is
+// the number of passes over the rows.  The window pass finds the first row by
+// itself, and an exact scan keeps the nearest point, which spares the pass that
+// certifies.  100,000 polylines (41M points a side) 1024 -> 735 us.
 template <int D>
 __device__ __forceinline__ void small_direction(const BatchArgs& a, uint32_t p, int d,
                                                 const hd_problem& pr, float* wb, int lane) {
@@ -542,9 +608,12 @@ __device__ __forceinline__ void small_direction(const BatchArgs& a, uint32_t p, 
 
   // Window bounds, one per row (an upper bound on the row's nearest-neighbour
   // distance); each row is read back only by the lane that wrote it.
+  TopRow top{-1.0f, 0u};
+#pragma unroll 1
   for (uint32_t row = lane; row < nx; row += 32) {
-    uint32_t j = scan_start(row, ratio, ny, half);
-    wb[row] = scan_run<D>(X, row, Y, j, ny, w0, INFINITY);
+    const float u = window_bound<D>(X, row, Y, ratio, ny, w0);
+    wb[row] = u;
+    top.add(u, row);
   }
   __syncwarp();
 
@@ -552,24 +621,20 @@ __device__ __forceinline__ void small_direction(const BatchArgs& a, uint32_t p, 
   // split the other set, early break once the row cannot raise the maximum),
   // then the next, until no bound exceeds the maximum — every other row is
   // then settled by its bound alone.  A scanned row's bound is set to -1.
-  // After kBestFirst rows the sweep below settles the rest.
+  // After kBestFirst rows the sweep below settles the rest.  The scan keeps
+  // the nearest point as well, which certifies the row.
   unsigned long long best = 0;
+  uint32_t near = kInvalid;  // nearest point of best's row, once known
   float thr = -1.0f;
   bool all_settled = false;
   for (int it = 0; it < kBestFirst; ++it) {
-    unsigned long long cand = 0;
-    for (uint32_t row = lane; row < nx; row += 32) {
-      const float u = wb[row];
-      if (u > thr) {
-        const unsigned long long kk = pack_max(u, row);
-        cand = kk > cand ? kk : cand;
-      }
+    if (it > 0) {
+      top = TopRow{thr, 0u};
+#pragma unroll 4
+      for (uint32_t row = lane; row < nx; row += 32) top.add(wb[row], row);
     }
-#pragma unroll
-    for (int o = 16; o; o >>= 1) {
-      const unsigned long long v = __shfl_xor_sync(0xFFFFFFFFu, cand, o);
-      cand = v > cand ? v : cand;
-    }
+    unsigned long long cand = top.key(thr);
+    cand = warp_max_key(cand);
     if (cand == 0) {
       all_settled = true;
       break;
@@ -578,41 +643,46 @@ __device__ __forceinline__ void small_direction(const BatchArgs& a, uint32_t p, 
     float xr[D];
 #pragma unroll
     for (int t = 0; t < D; ++t) xr[t] = X[(uint64_t) r * D + t];
-    float cm = __uint_as_float((uint32_t) (cand >> 32));  // its bound: a real distance
+    NearPoint np{INFINITY, kInvalid};
     bool broke = false;
-    for (uint64_t t0 = 0; t0 < ny; t0 += 32 * kLongIlp) {
+    for (uint64_t at = 0; at < ny; at += 32 * kLongIlp) {
+      const uint32_t t0 = (uint32_t) at, rem = ny - t0;
       float y[kLongIlp][D];
 #pragma unroll
       for (int u = 0; u < kLongIlp; ++u) {
-        const uint64_t jj = t0 + (uint64_t) u * 32 + lane;
+        const uint32_t v = u * 32 + lane;
+        if (v < rem) {
+          load_pt<D>(Y, (uint64_t) t0 + v, y[u]);
+        } else {
 #pragma unroll
-        for (int k = 0; k < D; ++k) y[u][k] = jj < ny ? Y[jj * D + k] : INFINITY;
+          for (int k = 0; k < D; ++k) y[u][k] = INFINITY;
+        }
       }
 #pragma unroll
-      for (int u = 0; u < kLongIlp; ++u) {
-        const uint64_t jj = t0 + (uint64_t) u * 32 + lane;
-        float d2;
-        if constexpr (D == 2)
-          d2 = d2_2(xr[0], xr[1], y[u][0], y[u][1]);
-        else
-          d2 = d2_3(xr[0], xr[1], xr[2], y[u][0], y[u][1], y[u][2]);
-        if (jj < ny) cm = fminf(cm, d2);
-      }
-      if (warp_min(cm) <= thr) {
+      for (int u = 0; u < kLongIlp; ++u)
+        np.add(d2_of<D>(xr, y[u]), t0 + u * 32 + lane);  // infinite past the end: no nearer
+      if (__any_sync(0xFFFFFFFFu, np.d <= thr)) {
         broke = true;
         break;
       }
     }
     if (!broke) {
-      const unsigned long long kr = pack_max(warp_min(cm), r);
+      unsigned long long am = np.j == kInvalid ? ~0ull : pack_min(np.d, np.j);
+      am = warp_min_key(am);
+      // No distance below infinity: the minimum is infinite, the nearest
+      // point left to the scan at the end.
+      const float m = am == ~0ull ? INFINITY : __uint_as_float((uint32_t) (am >> 32));
+      const unsigned long long kr = pack_max(m, r);
       if (kr > best) {
         best = kr;
+        near = (uint32_t) am;
         thr = threshold_of(best);
       }
     }
     if (lane == (int) (r & 31)) wb[r] = -1.0f;
     __syncwarp();
   }
+  const unsigned long long certified = near == kInvalid ? 0ull : best;
 
   // Sweep.
   const uint32_t limit = ny < (uint32_t) kShortScan ? ny : (uint32_t) kShortScan;
@@ -637,11 +707,7 @@ __device__ __forceinline__ void small_direction(const BatchArgs& a, uint32_t p, 
     const bool pending = !broke && step < ny;
     // Rows that completed their scan raise the maximum.
     unsigned long long kk = (!broke && !pending) ? pack_max(cmin, row) : 0ull;
-#pragma unroll
-    for (int o = 16; o; o >>= 1) {
-      const unsigned long long v = __shfl_xor_sync(0xFFFFFFFFu, kk, o);
-      kk = v > kk ? v : kk;
-    }
+    kk = warp_max_key(kk);
     if (kk > best) {
       best = kk;
       thr = threshold_of(best);
@@ -697,22 +763,21 @@ __device__ __forceinline__ void small_direction(const BatchArgs& a, uint32_t p, 
   }
   // Certification here, where the rows are at hand: the argmin of the
   // certifying row (lowest index among ties), as k_batch_certify does for
-  // the pipeline's directions.
+  // the pipeline's directions, unless the row's own scan found it.
   const uint32_t rc = unpack_max_index(best);
-  float xc[D];
-  load_pt<D>(X, rc, xc);
-  unsigned long long am = ~0ull;
+  unsigned long long am = (best & 0xFFFFFFFF00000000ull) | near;
+  if (best != certified) {
+    float xc[D];
+    load_pt<D>(X, rc, xc);
+    am = ~0ull;
 #pragma unroll 4
-  for (uint32_t j = lane; j < ny; j += 32) {
-    float y[D];
-    load_pt<D>(Y, j, y);
-    const unsigned long long k = pack_min(d2_of<D>(xc, y), j);
-    am = k < am ? k : am;
-  }
-#pragma unroll
-  for (int o = 16; o; o >>= 1) {
-    const unsigned long long v = __shfl_xor_sync(0xFFFFFFFFu, am, o);
-    am = v < am ? v : am;
+    for (uint32_t j = lane; j < ny; j += 32) {
+      float y[D];
+      load_pt<D>(Y, j, y);
+      const unsigned long long k = pack_min(d2_of<D>(xc, y), j);
+      am = k < am ? k : am;
+    }
+    am = warp_min_key(am);
   }
   if (lane == 0) {
     a.keys[2 * (uint64_t) p + d] = best;
@@ -726,11 +791,7 @@ __device__ __forceinline__ void small_direction(const BatchArgs& a, uint32_t p, 
 // thread).  `red` is shared scratch of one word per warp.
 __device__ __forceinline__ unsigned long long block_max_u64(unsigned long long v,
                                                             unsigned long long* red) {
-#pragma unroll
-  for (int o = 16; o; o >>= 1) {
-    const unsigned long long w = __shfl_xor_sync(0xFFFFFFFFu, v, o);
-    v = w > v ? w : v;
-  }
+  v = warp_max_key(v);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
   __syncthreads();
   v = red[0];
@@ -770,25 +831,26 @@ __device__ __forceinline__ void cta_direction(const BatchArgs& a, uint32_t p, in
   const float ratio = (float) ny / (float) nx;
   const uint32_t w0 = ny > 2 * a.window + 1 ? 2 * a.window + 1 : ny;
   const uint32_t half = w0 >> 1;
+  TopRow top{-1.0f, 0u};
+#pragma unroll 1
   for (uint32_t row = tid; row < nx; row += kBatchThreads) {
-    uint32_t j = scan_start(row, ratio, ny, half);
-    wb[row] = scan_run<D>(X, row, Y, j, ny, w0, INFINITY);
+    const float u = window_bound<D>(X, row, Y, ratio, ny, w0);
+    wb[row] = u;
+    top.add(u, row);
   }
   __syncthreads();
 
   unsigned long long best = 0;
+  uint32_t near = kInvalid;  // nearest point of best's row, once known
   float thr = -1.0f;
   bool settled = false;
   for (int it = 0; it < kBestFirst; ++it) {
-    unsigned long long cand = 0;
-    for (uint32_t row = tid; row < nx; row += kBatchThreads) {
-      const float u = wb[row];
-      if (u > thr) {
-        const unsigned long long kk = pack_max(u, row);
-        cand = kk > cand ? kk : cand;
-      }
+    if (it > 0) {
+      top = TopRow{thr, 0u};
+#pragma unroll 4
+      for (uint32_t row = tid; row < nx; row += kBatchThreads) top.add(wb[row], row);
     }
-    cand = block_max_u64(cand, s_red);
+    const unsigned long long cand = block_max_u64(top.key(thr), s_red);
     if (cand == 0) {
       settled = true;
       break;
@@ -796,37 +858,44 @@ __device__ __forceinline__ void cta_direction(const BatchArgs& a, uint32_t p, in
     const uint32_t r = unpack_max_index(cand);
     float xr[D];
     load_pt<D>(X, r, xr);
-    float cm = __uint_as_float((uint32_t) (cand >> 32));  // its bound: a real distance
+    NearPoint np{INFINITY, kInvalid};
     bool broke = false;
-    for (uint64_t t0 = 0; t0 < ny; t0 += (uint64_t) kBatchThreads * kLongIlp) {
+    for (uint64_t at = 0; at < ny; at += kBatchThreads * kLongIlp) {
+      const uint32_t t0 = (uint32_t) at, rem = ny - t0;
       float y[kLongIlp][D];
 #pragma unroll
       for (int u = 0; u < kLongIlp; ++u) {
-        const uint64_t jj = t0 + (uint64_t) u * kBatchThreads + tid;
+        const uint32_t v = u * kBatchThreads + tid;
+        if (v < rem) {
+          load_pt<D>(Y, (uint64_t) t0 + v, y[u]);
+        } else {
 #pragma unroll
-        for (int k = 0; k < D; ++k) y[u][k] = jj < ny ? Y[jj * D + k] : INFINITY;
+          for (int k = 0; k < D; ++k) y[u][k] = INFINITY;
+        }
       }
 #pragma unroll
-      for (int u = 0; u < kLongIlp; ++u) {
-        const uint64_t jj = t0 + (uint64_t) u * kBatchThreads + tid;
-        const float d2 = d2_of<D>(xr, y[u]);
-        if (jj < ny) cm = fminf(cm, d2);
-      }
-      if (__syncthreads_or(cm <= thr)) {
+      for (int u = 0; u < kLongIlp; ++u)
+        np.add(d2_of<D>(xr, y[u]), t0 + u * kBatchThreads + tid);
+      if (__syncthreads_or(np.d <= thr)) {
         broke = true;
         break;
       }
     }
     if (!broke) {
-      const unsigned long long kr = pack_max(block_min_f(cm, s_redf), r);
+      const unsigned long long am =
+          ~block_max_u64(np.j == kInvalid ? 0ull : ~pack_min(np.d, np.j), s_red);
+      const float m = am == ~0ull ? INFINITY : __uint_as_float((uint32_t) (am >> 32));
+      const unsigned long long kr = pack_max(m, r);
       if (kr > best) {
         best = kr;
+        near = (uint32_t) am;
         thr = threshold_of(best);
       }
     }
     if (tid == 0) wb[r] = -1.0f;
     __syncthreads();
   }
+  const unsigned long long certified = near == kInvalid ? 0ull : best;
   if (!settled) {
     // Rows still above the maximum: one warp per row, lanes over the other
     // set; the block's maximum is shared through s_best.
@@ -868,19 +937,23 @@ __device__ __forceinline__ void cta_direction(const BatchArgs& a, uint32_t p, in
     best = s_best;
     __syncthreads();
   }
-  // Certification (block-wide argmin of the certifying row).
+  // Certification (block-wide argmin of the certifying row, unless its own
+  // scan found it).
   const uint32_t rc = unpack_max_index(best);
-  float xc[D];
-  load_pt<D>(X, rc, xc);
-  unsigned long long am = ~0ull;
+  unsigned long long am = (best & 0xFFFFFFFF00000000ull) | near;
+  if (best != certified) {
+    float xc[D];
+    load_pt<D>(X, rc, xc);
+    am = ~0ull;
 #pragma unroll 4
-  for (uint32_t j = tid; j < ny; j += kBatchThreads) {
-    float y[D];
-    load_pt<D>(Y, j, y);
-    const unsigned long long k = pack_min(d2_of<D>(xc, y), j);
-    am = k < am ? k : am;
+    for (uint32_t j = tid; j < ny; j += kBatchThreads) {
+      float y[D];
+      load_pt<D>(Y, j, y);
+      const unsigned long long k = pack_min(d2_of<D>(xc, y), j);
+      am = k < am ? k : am;
+    }
+    am = ~block_max_u64(~am, s_red);  // min via the complement
   }
-  am = ~block_max_u64(~am, s_red);  // min via the complement
   if (tid == 0) {
     a.keys[2 * (uint64_t) p + d] = best;
     const bool ok = (uint32_t) (am >> 32) == (uint32_t) (best >> 32);
@@ -894,7 +967,13 @@ __global__ void __launch_bounds__(kBatchThreads) k_batch_small(BatchArgs a) {
   const int lane = threadIdx.x & 31;
   // First the CTA-path directions, one per block: they sit among the first
   // n_big ranks of the plan, largest first.
-  for (uint64_t q = blockIdx.x; q < (uint64_t) a.n_big * a.ndir; q += gridDim.x) {
+  __shared__ unsigned long long s_q;
+  for (;;) {
+    __syncthreads();
+    if (threadIdx.x == 0) s_q = atomicAdd(a.taken, 1ull);
+    __syncthreads();
+    const uint64_t q = s_q;
+    if (q >= (uint64_t) a.n_big * a.ndir) break;
     const uint32_t r = (uint32_t) (q / a.ndir);
     const int d = (int) (q % a.ndir);
     const uint32_t p = a.order[r];
@@ -903,11 +982,15 @@ __global__ void __launch_bounds__(kBatchThreads) k_batch_small(BatchArgs a) {
     if (nx <= (uint64_t) a.small_rows || nx > (uint64_t) a.pipe_rows) continue;
     cta_direction<D>(a, p, d, pr, d == 0 ? a.wb_a + pr.offset_a : a.wb_b + pr.offset_b);
   }
-  // Then the one-warp directions, one per warp.
-  const uint64_t nw = (uint64_t) gridDim.x * (kBatchThreads / 32);
+  // Then the one-warp directions, one per warp; the next one is asked for
+  // before this one's work.
   const uint64_t npd = (uint64_t) a.nprob * a.ndir;
-  for (uint64_t q = (uint64_t) blockIdx.x * (kBatchThreads / 32) + (threadIdx.x >> 5); q < npd;
-       q += nw) {
+  unsigned long long mine = 0;
+  if (lane == 0) mine = atomicAdd(a.taken + 1, 1ull);
+  for (;;) {
+    const uint64_t q = __shfl_sync(0xFFFFFFFFu, mine, 0);
+    if (q >= npd) break;
+    if (lane == 0) mine = atomicAdd(a.taken + 1, 1ull);
     const uint32_t r = (uint32_t) (q / a.ndir);
     const int d = (int) (q % a.ndir);
     const uint32_t p = a.order[r];
@@ -1067,7 +1150,7 @@ struct BatchGraph {
   uint64_t n, maxpairs;
   char* base;             // the batch buffer; reset region starts here
   size_t zero_bytes;      // keys and window bounds per class (reset to 0)
-  unsigned long long* ctr;    // long-row count, certification mismatch count
+  unsigned long long* ctr;    // long-row count, mismatch count, directions taken (two)
   size_t o_smin, smin_bytes;  // seed minima (reset to 0xFF bytes)
   size_t o_pkeys, o_pkeys2, o_pvals, o_cnt, o_tmp, cub_tmp;
   PD* pd;
@@ -1079,14 +1162,14 @@ struct BatchGraph {
 
 // Resets the graph's per-call words with a kernel (no memset node that could
 // queue behind copies): keys and window bounds to 0, seed minima to all ones,
-// the two counters to 0.
+// the four counters to 0.
 __global__ void k_batch_reset(uint4* __restrict__ zero, size_t zero16, uint4* __restrict__ ones,
                               size_t ones16, unsigned long long* __restrict__ ctr) {
   const size_t stride = (size_t) gridDim.x * blockDim.x;
   const size_t t = blockIdx.x * (size_t) blockDim.x + threadIdx.x;
   for (size_t i = t; i < zero16; i += stride) zero[i] = make_uint4(0u, 0u, 0u, 0u);
   for (size_t i = t; i < ones16; i += stride) ones[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
-  if (t < 2) ctr[t] = 0ull;
+  if (t < 4) ctr[t] = 0ull;
 }
 
 hd_status capture_batch_graph(Ctx& c, const BatchGraph& g, cudaGraphExec_t* out) {
@@ -1100,7 +1183,7 @@ hd_status capture_batch_graph(Ctx& c, const BatchGraph& g, cudaGraphExec_t* out)
   {
     // Both regions are whole multiples of 256 bytes (Layout pieces).
     const size_t z16 = g.zero_bytes / 16, o16 = g.smin_bytes / 16;
-    const size_t work = std::max<size_t>(std::max(z16, o16), 2);
+    const size_t work = std::max<size_t>(std::max(z16, o16), 4);
     const unsigned rb = (unsigned) std::min<size_t>((work + 255) / 256, (size_t) c.num_sms * 8);
     k_batch_reset<<<rb, 256, 0, c.stream>>>((uint4*) g.base, z16, (uint4*) at(g.o_smin), o16,
                                             g.ctr);
@@ -1237,7 +1320,7 @@ hd_status batch_solve(Ctx& c, const float* A, uint64_t total_a, const float* B, 
   g.zero_bytes = L.off;
   g.o_smin = L.take(n * 2 * kSlots * 4);
   g.smin_bytes = L.off - g.o_smin;
-  const size_t o_ctr = L.take(2 * 8);  // long-row count, mismatch count
+  const size_t o_ctr = L.take(4 * 8);  // see BatchGraph::ctr
   const size_t o_wb_a = L.take(total_a * 4);
   const size_t o_wb_b = L.take(ndir == 2 ? total_b * 4 : 0);
   const size_t o_probs = L.take(n * sizeof(hd_problem));
@@ -1315,6 +1398,7 @@ hd_status batch_solve(Ctx& c, const float* A, uint64_t total_a, const float* B, 
   args.wb_b = (float*) at(o_wb_b);
   args.longq = (LongRow*) at(o_long);
   args.long_count = d_ctr;
+  args.taken = d_ctr + 2;
   args.long_cap = long_cap;
   args.small_rows = small_rows;
   args.pipe_rows = pipe_rows;

@@ -90,6 +90,42 @@ def test_batch_incoherent_sets(dims, small_rows):
             assert out["hd_f32"][p] == want["hd_f32"], (p, undirected)
 
 
+@pytest.mark.parametrize("dims", [2, 3])
+@pytest.mark.parametrize("small_rows", [0, 32])
+def test_batch_nearest_points(dims, small_rows):
+    """The certifying column comes from the winning row's own scan: the lowest
+    one at the row's distance, at sizes around the window (5 points), a scan
+    step (256, 2048 points) and with copies; infinite distances included."""
+    import hausdorffdistance_gb300 as hd
+    sizes = [(1, 1), (3, 4), (40, 5), (40, 6), (33, 255), (300, 256), (300, 257), (50, 2048),
+             (50, 2049), (700, 4097), (20, 9), (64, 300)]
+    rng = np.random.default_rng(31 + dims)
+    a, b = [], []
+    for k, (n, m) in enumerate(sizes):
+        x, y = rng.random((n, dims)), rng.random((m, dims))
+        if k % 2:  # few distinct points: many ties
+            x, y = np.round(x * 4), np.round(y * 4) + 0.25
+        if k == 10:  # squared distances overflow
+            x, y = x * 1e20, -1e20 * (1 + y)
+        a.append(x.astype(np.float32))
+        b.append(y.astype(np.float32))
+    oa = np.concatenate([[0], np.cumsum([len(x) for x in a])])
+    ob = np.concatenate([[0], np.cumsum([len(y) for y in b])])
+    with hd.Engine(batch_small_rows=small_rows) as engine:
+        out = engine.solve_batch(np.concatenate(a), np.concatenate(b), oa, ob)
+    for p, (x, y) in enumerate(zip(a, b)):
+        with np.errstate(over="ignore"):
+            d2 = np.zeros((len(x), len(y)), np.float32)
+            for k in range(dims):
+                diff = x[:, None, k] - y[None, :, k]
+                d2 = diff * diff if k == 0 else d2 + diff * diff
+        near = d2.min(1)
+        assert out["hd_f32"][p] == np.sqrt(near.max()), p
+        row = int(out["ia"][p])
+        assert near[row] == near.max(), p
+        assert int(out["ib"][p]) == int(np.argmin(d2[row])), p
+
+
 def test_batch_rejects_out_of_range_offsets(engine):
     import hausdorffdistance_gb300 as hd
     a = np.ones((4, 2), np.float32)
