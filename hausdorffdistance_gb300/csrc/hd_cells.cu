@@ -166,6 +166,7 @@ struct CellArgs {
   uint32_t* any[2];             // blocks with a cell that U or N marks in this set
   uint32_t* top[2];             // and super-blocks with such a block (large maps only)
   int count;                    // directions
+  int seeds_only;               // the seeds set the running maxima, nothing follows
   CellDirState* seen;           // pinned host memory: state after the listing of cells,
   CellDirState* left;           // and at the end
   const DevScalars* sc0;        // DevScalars of direction 0
@@ -586,6 +587,16 @@ __device__ __forceinline__ const uint32_t* search_map(const uint32_t* __restrict
   }
 }
 
+// A direction's running maximum from L: a key of that distance and no row,
+// below the key of any row at h, so that a scan or an index may stop its
+// queries at L from the start (the FP64 listing pass at soft_stop(L)).
+template <class Ge>
+__device__ __forceinline__ void start_at_level(const CellDir& d, const CellGrid& g, float cells2) {
+  const float L2 = cells2 * (g.side * g.side) * 0.9999f;
+  if (g.valid && L2 > 0.0f)
+    atomicMax(&d.sc->max_key, (unsigned long long) __float_as_uint(L2) << 32);
+}
+
 // Seeds (a warp per sampled word, 64 blocks, of the query set's coarse map):
 // one cell of one of its occupied blocks.
 template <class Ge>
@@ -612,22 +623,10 @@ __global__ void __launch_bounds__(kSearchThreads) k_cell_seed(CellArgs a) {
   const float stop = __uint_as_float(ld_relaxed_u32(&d.st->L2));
   float lb, ub;
   cell_search<Ge, true>(p, a.occ[1 - d.qset], map, stop, &lb, &ub);
-  if ((threadIdx.x & 31) == 0) raise_level(d.st, lb);
-}
-
-// A direction's running maximum from L: a key of that distance and no row,
-// below the key of any row at h, so that a scan or an index may stop its
-// queries at L from the start (the FP64 listing pass at soft_stop(L)).
-template <class Ge>
-__device__ __forceinline__ void start_at_level(const CellDir& d, const CellGrid& g) {
-  const float L2 = __uint_as_float(d.st->L2) * (g.side * g.side) * 0.9999f;
-  if (g.valid && L2 > 0.0f)
-    atomicMax(&d.sc->max_key, (unsigned long long) __float_as_uint(L2) << 32);
-}
-
-template <class Ge>
-__global__ void k_cell_level(CellArgs a) {
-  if (threadIdx.x < a.count) start_at_level<Ge>(a.d[threadIdx.x], cell_grid<Ge>(a.ord));
+  if ((threadIdx.x & 31) == 0) {
+    raise_level(d.st, lb);
+    if (a.seeds_only && lb < INFINITY) start_at_level<Ge>(d, g, lb / kSlack);
+  }
 }
 
 // For a cell at each of the 64 places of a block, the cells of neighbour j (of
@@ -668,7 +667,7 @@ __global__ void __launch_bounds__(256) k_cell_blocks(CellArgs a) {
   if (!(stop >= kMinReach * kMinReach * D)) {
     if (blockIdx.x == 0 && threadIdx.x == 0) {
       d.st->off = 1u;
-      start_at_level<Ge>(d, g);  // for the index that takes over
+      start_at_level<Ge>(d, g, __uint_as_float(d.st->L2));  // for the index that takes over
       a.seen[blockIdx.y].L2 = d.st->L2;
       a.seen[blockIdx.y].off = 1u;
     }
@@ -1184,28 +1183,13 @@ bool cells_apply(const Ctx& c, uint64_t nA, uint64_t nB, int dims) {
 
 namespace {
 
-// A launch behind the kernel before it (see chain_wait): its CTAs are on their
-// SMs when that kernel's last ones leave.  Eleven short kernels in a row: 200k
-// uniform 2-D points 144 -> 131 us, 1M clusters 220 -> 204, 10M 368 -> 348.  Not
-// for the kernels below that pass chain = false: the search's waiting CTAs
-// hold shared memory that the level before needs (5M 2-D points 374 -> 439 us),
-// the pass over the points ran slower when it started beside the marking (50M
-// planes 3.94 -> 4.33 ms), and the pair scan delays an index that waits behind
-// it (200k planes directed 294 -> 310 us).
-template <class... P, class... T>
-void launch_next(Ctx& c, bool chain, void (*kernel)(P...), dim3 grid, int threads, T... args) {
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3((unsigned) threads);
-  cfg.stream = c.stream;
-  cudaLaunchAttribute at{};
-  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at.val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = &at;
-  cfg.numAttrs = chain ? 1 : 0;
-  cudaLaunchKernelEx(&cfg, kernel, P(args)...);
-}
-
+// The filter's launches: eleven short kernels in a row (200k uniform 2-D points
+// 144 -> 131 us with them chained, 1M clusters 220 -> 204, 10M 368 -> 348).  Not
+// chained are the search, whose waiting CTAs hold shared memory that the level
+// before needs (5M 2-D points 374 -> 439 us), the pass over the points, which ran
+// slower when it started beside the marking (50M planes 3.94 -> 4.33 ms), and the
+// pair scan, which delays an index that waits behind it (200k planes directed
+// 294 -> 310 us).
 template <class Ge>
 hd_status enqueue(Ctx& c, const DirInput* ins, int count, const F64Plan* plan, CellArgs& a,
                   bool boxes_known, bool seeds_only, bool* no_room) {
@@ -1267,6 +1251,7 @@ hd_status enqueue(Ctx& c, const DirInput* ins, int count, const F64Plan* plan, C
     a.top[k] = (uint32_t*) (base + o_top[k]);
   }
   a.count = count;
+  a.seeds_only = seeds_only;
   a.seen = (CellDirState*) ((char*) c.host_pinned + kStageSeeds);
   a.left = (CellDirState*) ((char*) c.host_pinned + kStageState);
   a.sc0 = scalars(c, 0);
@@ -1305,26 +1290,22 @@ hd_status enqueue(Ctx& c, const DirInput* ins, int count, const F64Plan* plan, C
   // Passes over points: four points per thread.
   const unsigned gp = (unsigned) std::max<uint64_t>(
       1, std::min<uint64_t>((most / 4 + 255) / 256, (uint64_t) sms * 8));
-  // (Not while a solve is captured: the seeds alone run inside graphs.)
-  const bool chain = !seeds_only;
+  constexpr bool chain = true;
   const uint32_t every = n[0] + n[1] >= kOccSplit ? kOccFirst : 1u;
-  launch_next(c, chain, k_cell_occ<Ge, true>, dim3(gp, 2), 256, a, ins[0].A, ins[0].nA, ins[0].B,
+  launch_next(c.stream, chain, k_cell_occ<Ge, true>, dim3(gp, 2), 256, a, ins[0].A, ins[0].nA, ins[0].B,
               ins[0].nB, every);
   if ((s = after_launch(c, "cell_occ")) != HD_OK) return s;
   if (every > 1) {
-    launch_next(c, chain, k_cell_occ<Ge, false>, dim3(gp, 2), 256, a, ins[0].A, ins[0].nA,
+    launch_next(c.stream, chain, k_cell_occ<Ge, false>, dim3(gp, 2), 256, a, ins[0].A, ins[0].nA,
                 ins[0].B, ins[0].nB, every);
     if ((s = after_launch(c, "cell_occ")) != HD_OK) return s;
   }
-  launch_next(c, chain, k_cell_coarse<Ge>, dim3(Ge::kBlocks / 256, 2), 256, a);
+  launch_next(c.stream, chain, k_cell_coarse<Ge>, dim3(Ge::kBlocks / 256, 2), 256, a);
   if ((s = after_launch(c, "cell_coarse")) != HD_OK) return s;
-  launch_next(c, chain, k_cell_seed<Ge>, dim3(kSeedWarps / kSearchWarps, dirs), kSearchThreads, a);
+  launch_next(c.stream, chain, k_cell_seed<Ge>, dim3(kSeedWarps / kSearchWarps, dirs), kSearchThreads, a);
   if ((s = after_launch(c, "cell_seed")) != HD_OK) return s;
-  if (seeds_only) {
-    k_cell_level<Ge><<<1, 32, 0, c.stream>>>(a);
-    return after_launch(c, "cell_level");
-  }
-  launch_next(c, chain, k_cell_blocks<Ge>,
+  if (seeds_only) return HD_OK;
+  launch_next(c.stream, chain, k_cell_blocks<Ge>,
               dim3(std::min<unsigned>(Ge::kBlocks / 256, sms * 32), dirs), 256, a);
   if ((s = after_launch(c, "cell_blocks")) != HD_OK) return s;
   // What the seeds found is in pinned memory now, for the host to act on while
@@ -1337,27 +1318,27 @@ hd_status enqueue(Ctx& c, const DirInput* ins, int count, const F64Plan* plan, C
     return cuda_fail(c, e, "filter event");
   const dim3 gw(sms * 6 / dirs, dirs);  // searches: six CTAs with the map per SM
   const dim3 gn(sms * 8 / dirs, dirs);
-  launch_next(c, chain, k_cell_near<Ge, false>, gn, 256, a);
+  launch_next(c.stream, chain, k_cell_near<Ge, false>, gn, 256, a);
   if ((s = after_launch(c, "cell_near")) != HD_OK) return s;
   if constexpr (Ge::D == 3) {
-    launch_next(c, chain, k_cell_near<Ge, true>, gn, 256, a);
+    launch_next(c.stream, chain, k_cell_near<Ge, true>, gn, 256, a);
     if ((s = after_launch(c, "cell_near")) != HD_OK) return s;
   }
-  launch_next(c, false, k_cell_search<Ge>, gw, kSearchThreads, a);
+  launch_next(c.stream, false, k_cell_search<Ge>, gw, kSearchThreads, a);
   if ((s = after_launch(c, "cell_search")) != HD_OK) return s;
-  launch_next(c, chain, k_cell_mark<Ge>, gw, kSearchThreads, a);
+  launch_next(c.stream, chain, k_cell_mark<Ge>, gw, kSearchThreads, a);
   if ((s = after_launch(c, "cell_mark")) != HD_OK) return s;
   mark(c, 1);
-  launch_next(c, false, k_cell_collect<Ge>, dim3(gp, 2), 256, a, ins[0].A, ins[0].nA, ins[0].B,
+  launch_next(c.stream, false, k_cell_collect<Ge>, dim3(gp, 2), 256, a, ins[0].A, ins[0].nA, ins[0].B,
               ins[0].nB);
   if ((s = after_launch(c, "cell_collect")) != HD_OK) return s;
   mark(c, 2);
   mark(c, 3);
   const dim3 gs(sms * 4, dirs);
   if (ins[0].count)
-    launch_next(c, false, k_cell_solve<Ge, true>, gs, 256, a);
+    launch_next(c.stream, false, k_cell_solve<Ge, true>, gs, 256, a);
   else
-    launch_next(c, false, k_cell_solve<Ge, false>, gs, 256, a);
+    launch_next(c.stream, false, k_cell_solve<Ge, false>, gs, 256, a);
   if ((s = after_launch(c, "cell_solve")) != HD_OK) return s;
   mark(c, 4);
   mark(c, 5);

@@ -155,6 +155,7 @@ __global__ void k_init_scalars(DevScalars* sc, int n) {
 // distances the lowest index wins (atomicMin on (d2 bits, index)).
 __global__ void k_argmin(const float* __restrict__ A, const float* __restrict__ B,
                          uint64_t nB, int D, DevScalars* sc) {
+  chain_wait();
   const unsigned long long key = sc->max_key;
   const uint32_t ia = unpack_max_index(key);
   if (key == 0 || ia == kInvalid) return;  // no row has completed
@@ -237,6 +238,7 @@ __global__ void k_argmin(const float* __restrict__ A, const float* __restrict__ 
 
 __global__ void k_finalize(const float* __restrict__ A, const float* __restrict__ B,
                            int D, DevScalars* sc) {
+  chain_wait();
   finalize_scalars(A, B, D, sc);
 }
 
@@ -247,10 +249,10 @@ hd_status certify(Ctx& c, const DirInput& in) {
   DevScalars* sc = scalars(c, in.dir);
   int grid = (int) std::min<uint64_t>((in.nB + 255) / 256, (uint64_t) c.num_sms * 4);
   grid = std::max(grid, 1);
-  k_argmin<<<grid, 256, 0, c.stream>>>(in.A, in.B, in.nB, in.dims, sc);
+  launch_next(c.stream, true, k_argmin, grid, 256, in.A, in.B, in.nB, in.dims, sc);
   hd_status s = after_launch(c, "argmin");
   if (s != HD_OK) return s;
-  k_finalize<<<1, 1, 0, c.stream>>>(in.A, in.B, in.dims, sc);
+  launch_next(c.stream, true, k_finalize, 1, 1, in.A, in.B, in.dims, sc);
   return after_launch(c, "finalize");
 }
 
@@ -291,7 +293,7 @@ hd_status certify_left(Ctx& c, const DirInput& in, const CellsLeft& left) {
     k_argmin_left<3><<<grid, 256, 0, c.stream>>>(in.A, left.t, (uint32_t) left.nt, sc);
   hd_status s = after_launch(c, "argmin");
   if (s != HD_OK) return s;
-  k_finalize<<<1, 1, 0, c.stream>>>(in.A, in.B, in.dims, sc);
+  launch_next(c.stream, true, k_finalize, 1, 1, in.A, in.B, in.dims, sc);
   return after_launch(c, "finalize");
 }
 
@@ -362,12 +364,14 @@ hd_status run_direction(Ctx& c, const DirInput& in, int variant, int* used,
   }
 }
 
-// Early-break scans of at least this many points per direction (|A| + |B| over
-// the directions, which share the cost) start from the cell filter's lower
-// bound (35 us): directed 3-D clusters 20,000 x 20,000 125 us without and 140 with
-// it, 40,000 x 30,000 152 and 167, 1M x 1M 2.5 and 1.2 ms; undirected 40,000 x
-// 40,000 306 and 272 us.
-constexpr uint64_t kSeedMinPoints = 80000;
+// Early-break scans of at least this many points (|A| + |B|, times the
+// directions, which share the cost) start from the cell filter's lower bound (30
+// us) instead of 152 seed rows scanned in full (20 us).  Without it and with it,
+// us: directed 3-D planes 20,000 x 15,000 184 and 163, 2-D uniform 19,000 x 18,000
+// 146 and 115, clusters 20,000 x 20,000 125 and 130, 60,000 x 50,000 251 and 188,
+// 1M x 1M 2500 and 1025; undirected clusters 15,000 x 15,000 216 and 185; below,
+// directed clusters 13,000 x 13,000 108 and 132.
+constexpr uint64_t kSeedMinPoints = 35000;
 
 hd_status check_status(Ctx& c, const HostScalars& h, int ndir) {
   for (int d = 0; d < ndir; ++d) {

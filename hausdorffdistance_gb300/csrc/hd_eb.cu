@@ -96,6 +96,7 @@ __device__ __forceinline__ void load_a(const float* __restrict__ A, uint64_t i,
 template <int D>
 __global__ void k_eb_pack(const float* __restrict__ B, uint64_t nB, Perm perm,
                           typename EbPt<D>::T* __restrict__ out, uint64_t nPad) {
+  chain_wait();
   for (uint64_t j = blockIdx.x * (uint64_t) blockDim.x + threadIdx.x; j < nPad;
        j += (uint64_t) gridDim.x * blockDim.x) {
     if constexpr (D == 2) {
@@ -131,6 +132,7 @@ __global__ void __launch_bounds__(kEbThreads)
               uint64_t a_end, const typename EbPt<D>::T* __restrict__ Bp,
               uint32_t nTiles, uint32_t capTiles, DevScalars* sc,
               HeavyEntry* heavy, uint32_t heavy_cap) {
+  chain_wait();
   using PT = typename EbPt<D>::T;
   constexpr uint32_t kTileBytes = kEbTile * sizeof(PT);
   __shared__ __align__(128) PT tile[2][kEbTile];
@@ -332,6 +334,7 @@ __global__ void __launch_bounds__(kEbThreads)
     k_eb_list(const float* __restrict__ A, const typename EbPt<D>::T* __restrict__ Bp,
               uint32_t nTiles, HeavyEntry* list, uint32_t* group_done, uint32_t n_host,
               const uint32_t* n_dev, uint32_t cap, DevScalars* sc) {
+  chain_wait();
   using PT = typename EbPt<D>::T;
   constexpr uint32_t kTileBytes = kEbTile * sizeof(PT);
   __shared__ __align__(128) PT tile[2][kEbTile];
@@ -463,6 +466,7 @@ __global__ void __launch_bounds__(kEbThreads)
     k_eb_heavy(const float* __restrict__ A, const typename EbPt<D>::T* __restrict__ Bp,
                uint32_t nTiles, DevScalars* sc, const HeavyEntry* __restrict__ list,
                const uint32_t* n_dev, uint32_t cap, const uint32_t* first_dev) {
+  chain_wait();
   constexpr int P = kHeavySlots;
   __shared__ float red[kEbThreads / 32][P];
   __shared__ float s_thr;
@@ -575,12 +579,14 @@ __global__ void __launch_bounds__(kEbThreads)
 // entries listed so far are finished, and the bulk's visit counter starts
 // again at zero.
 __global__ void k_eb_mark_heavy(DevScalars* sc) {
+  chain_wait();
   sc->heavy_mark = sc->heavy_count;
   sc->next = 0;
 }
 
 // The seed list: the first n visit positions of A, nothing scanned yet.
 __global__ void k_eb_seed_list(Perm permA, uint32_t n, uint32_t nTiles, HeavyEntry* list) {
+  chain_wait();
   const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e < n) list[e] = HeavyEntry{(uint32_t) permA(e), 0u, nTiles, FLT_MAX};
 }
@@ -624,7 +630,7 @@ hd_status run_eb_dim(Ctx& c, const DirInput& in) {
 
   {
     int grid = (int) std::min<uint64_t>((nPad + 255) / 256, (uint64_t) c.num_sms * 16);
-    k_eb_pack<D><<<grid, 256, 0, c.stream>>>(in.B, in.nB, pB, (PT*) pb, nPad);
+    launch_next(c.stream, true, k_eb_pack<D>, grid, 256, in.B, in.nB, pB, (PT*) pb, nPad);
     if ((s = after_launch(c, "eb_pack")) != HD_OK) return s;
   }
   mark(c, 1);
@@ -650,8 +656,8 @@ hd_status run_eb_dim(Ctx& c, const DirInput& in) {
     // Slots per thread: the most (4, 2, 1) that still fill every resident CTA
     // of a full grid, so that a small set spreads over all SMs instead of
     // leaving most of them idle (every slot of a thread is computed).
-    const void* fns[3] = {(const void*) k_eb_main<D, 4>, (const void*) k_eb_main<D, 2>,
-                          (const void*) k_eb_main<D, 1>};
+    constexpr decltype(&k_eb_main<D, 4>) fns[3] = {k_eb_main<D, 4>, k_eb_main<D, 2>,
+                                                   k_eb_main<D, 1>};
     const int slots[3] = {4, 2, 1};
     const uint64_t rest = in.nA - n_seed;
     int pick = 2, occ = 1;
@@ -682,11 +688,8 @@ hd_status run_eb_dim(Ctx& c, const DirInput& in) {
                                                   tuning().eb_cap_min / half),
                                tuning().eb_cap_max);
     }
-    uint32_t capTiles = (uint32_t) std::max<uint64_t>(1, cap / kEbTile);
-    const float* a_ptr = in.A;
-    const PT* b_ptr = (const PT*) pb;
-    HeavyEntry* h_ptr = (HeavyEntry*) ph;
-    uint32_t heavy_cap = (uint32_t) (in.nA - n_seed);
+    const uint32_t capTiles = (uint32_t) std::max<uint64_t>(1, cap / kEbTile);
+    const uint32_t heavy_cap = (uint32_t) (in.nA - n_seed);
     // Checkpoints: the main pass runs in parts; after each part the points
     // it deferred are finished before the next part starts.  Deferred points
     // include the outliers, whose distances are the ones that lift the
@@ -714,14 +717,13 @@ hd_status run_eb_dim(Ctx& c, const DirInput& in) {
         k_eb_mark_heavy<<<1, 1, 0, c.stream>>>(sc);
         if ((s = after_launch(c, "eb_mark")) != HD_OK) return s;
       }
-      void* args[] = {&a_ptr, &pA, &a_begin, &a_end, &b_ptr, (void*) &nTiles, &capTiles, &sc,
-                      &h_ptr, &heavy_cap};
-      cudaLaunchKernel(fns[pick], dim3(grid), dim3(kEbThreads), args, 0, c.stream);
+      launch_next(c.stream, true, fns[pick], grid, kEbThreads, in.A, pA, a_begin, a_end,
+                  (const PT*) pb, nTiles, capTiles, sc, (HeavyEntry*) ph, heavy_cap);
       if ((s = after_launch(c, "eb_main")) != HD_OK) return s;
       if (part == parts - 1) mark(c, 4);
-      k_eb_heavy<D><<<c.num_sms * 4, kEbThreads, 0, c.stream>>>(
-          in.A, (const PT*) pb, nTiles, sc, (const HeavyEntry*) ph, &sc->heavy_count, heavy_cap,
-          part > 0 ? &sc->heavy_mark : nullptr);
+      launch_next(c.stream, true, k_eb_heavy<D>, c.num_sms * 4, kEbThreads, in.A, (const PT*) pb,
+                  nTiles, sc, (const HeavyEntry*) ph, &sc->heavy_count, heavy_cap,
+                  part > 0 ? &sc->heavy_mark : nullptr);
       if ((s = after_launch(c, "eb_deferred")) != HD_OK) return s;
       a_begin = a_end;
     }

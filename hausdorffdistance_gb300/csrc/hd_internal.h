@@ -54,6 +54,23 @@ struct DevScalars {
 };
 
 #ifdef __CUDACC__
+// A launch behind the kernel before it on the stream: chained, its CTAs are on
+// their SMs when that kernel's last ones leave, if both begin with chain_wait.
+template <class... P, class... T>
+cudaError_t launch_next(cudaStream_t st, bool chain, void (*kernel)(P...), dim3 grid, int threads,
+                        T... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3((unsigned) threads);
+  cfg.stream = st;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = chain ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 // The result words of a direction from its running maximum and argmin.
 __device__ __forceinline__ void finalize_scalars(const float* __restrict__ A,
                                                  const float* __restrict__ B, int D,
