@@ -866,7 +866,9 @@ __global__ void __launch_bounds__(kSearchThreads) k_cell_search(CellArgs a) {
 // Cells whose upper distance exceeds the L that the search ended with, and the
 // target cells within that distance of them.  Few cells get here: a CTA looks
 // for them among kMarkChunk far cells at a time and takes each with all its
-// warps.  Of more than kManyFar far cells many may be marked: then a thread per
+// warps.  They sit together in the list, so that a CTA's chunk is taken from all
+// over it (10M clusters 53 -> 43 us against chunks of neighbours, two thirds of
+// the SMs idle then; the call 350 -> 345, 1M 203 -> 195).  Of more than kManyFar far cells many may be marked: then a thread per
 // cell marks whole blocks within the distance.
 constexpr uint32_t kMarkChunk = 8;
 
@@ -944,10 +946,11 @@ __global__ void __launch_bounds__(kSearchThreads) k_cell_mark(CellArgs a) {
     }
     return;
   }
-  for (uint32_t e0 = blockIdx.x * kMarkChunk; e0 < n; e0 += gridDim.x * kMarkChunk) {
+  const uint32_t chunks = (n + kMarkChunk - 1) / kMarkChunk;
+  for (uint32_t at = blockIdx.x; at < chunks; at += gridDim.x) {
     if (threadIdx.x == 0) s_n = 0;
     __syncthreads();
-    const uint32_t e = e0 + threadIdx.x;
+    const uint32_t e = at + threadIdx.x * chunks;  // from all over the list
     if (threadIdx.x < kMarkChunk && e < n && !(d.far_ub[e] * kSlack < stop)) {
       const uint32_t cell = d.far[e], i = atomicAdd(&s_n, 1u);
       s_cell[i] = cell;
