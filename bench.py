@@ -370,6 +370,9 @@ def _fp32_issue_peak(local, sm_mhz):
     return sms * 128 * (sm_mhz or 2070.0) * 1e6
 
 
+CELL_FILTER_MIN_POINTS = 40000  # |A| + |B|: csrc/hd_internal.h, kCellsMinPoints
+
+
 def _lbvh_phases(n_a, n_b, dims, undirected, rc, phase):
     """Roofline entries of the LBVH path's three phases, algorithmic bytes as
     the measurement plan defines them: sort (per set: read the points twice,
@@ -454,7 +457,18 @@ def bench_single(eng, name, n, steps, warmup, args, ctx):
     used = (hd._lib.VARIANT_NAMES.get(res.variant_used),
             hd._lib.VARIANT_NAMES.get(res.variant_used_ba) if undirected else None)
     roof, phases = None, []
-    if res.variant_used == hd._lib.VARIANT_LBVH:
+    if res.variant_used == hd._lib.VARIANT_LBVH and 2 * n >= CELL_FILTER_MIN_POINTS:
+        # The cell filter (and the LBVH over what it leaves): the points are read
+        # for the boxes and for the occupied cells, their cell codes written and
+        # read; the rest of the chain works on the maps and on short lists.
+        alg = 2 * n * (2 * dims * 4 + 8)
+        t_ms = float(sum(phase))
+        ach = alg / (t_ms / 1e3) / 1e9
+        roof = {"bound": "hbm", "kernel": "cell_filter", "achieved": ach,
+                "peak": peaks["hbm_gbs"], "unit": "GB/s", "frac": ach / peaks["hbm_gbs"],
+                "traffic": None, "algorithmic_bytes": alg, "ms": t_ms,
+                "issue_active_ncu": None, "peak_source": pkind + " hbm_gbs"}
+    elif res.variant_used == hd._lib.VARIANT_LBVH:
         for tag, alg, t_ms in _lbvh_phases(n, n, dims, undirected, rc, phase):
             if t_ms <= 0:
                 continue
