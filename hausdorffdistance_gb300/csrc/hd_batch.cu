@@ -1198,7 +1198,8 @@ struct BatchGraph {
   int dims, ndir;
   uint64_t n;
   char* base;             // the batch buffer; reset region starts here
-  size_t zero_bytes;      // keys and window bounds per class (reset to 0)
+  size_t zero_bytes;      // keys and window bounds per class (reset to 0),
+  size_t key_bytes;       // the keys alone
   unsigned long long* ctr;    // long-row count, mismatch count, directions taken (two)
   size_t o_smin, smin_bytes;  // seed minima (reset to 0xFF bytes)
   size_t o_pkeys, o_pkeys2, o_pvals, o_cnt, o_tmp, cub_tmp;
@@ -1226,12 +1227,18 @@ hd_status capture_batch_graph(Ctx& c, const BatchGraph& g, cudaGraphExec_t* out)
   const BatchArgs& a = g.args;
   const uint32_t n = (uint32_t) g.n;
   const unsigned pblocks = (unsigned) ((g.n + 1 + 255) / 256);
+  // Without a direction in the multi-pass pipeline its part of the plan, its
+  // passes and its certification are left out (nine launches; 100,000 polylines
+  // 933 -> 893 us a call, 30,000 in 3-D 415 -> 395).
+  const bool pipeline = a.total > 0;
   cudaGraph_t graph = nullptr;
   cudaError_t e = cudaStreamBeginCapture(c.stream, cudaStreamCaptureModeThreadLocal);
   if (e != cudaSuccess) return cuda_fail(c, e, "begin capture");
   {
-    // Both regions are whole multiples of 256 bytes (Layout pieces).
-    const size_t z16 = g.zero_bytes / 16, o16 = g.smin_bytes / 16;
+    // Both regions are whole multiples of 256 bytes (Layout pieces); the window
+    // bounds and seed minima are the pipeline's.
+    const size_t z16 = (pipeline ? g.zero_bytes : g.key_bytes) / 16;
+    const size_t o16 = pipeline ? g.smin_bytes / 16 : 0;
     const size_t work = std::max<size_t>(std::max(z16, o16), 4);
     const unsigned rb = (unsigned) std::min<size_t>((work + 255) / 256, (size_t) c.num_sms * 8);
     k_batch_reset<<<rb, 256, 0, c.stream>>>((uint4*) g.base, z16, (uint4*) at(g.o_smin), o16,
@@ -1244,11 +1251,13 @@ hd_status capture_batch_graph(Ctx& c, const BatchGraph& g, cudaGraphExec_t* out)
                                   (uint32_t*) at(g.o_pkeys2), (const uint32_t*) at(g.o_pvals),
                                   const_cast<uint32_t*>(a.order), (int64_t) n, 0, kPlanBits,
                                   c.stream);
-  k_plan_counts<<<pblocks, 256, 0, c.stream>>>(a.probs, a.order, n, g.ndir, a.pipe_rows,
-                                              (uint64_t*) at(g.o_cnt));
-  tb = g.cub_tmp;
-  cub::DeviceScan::ExclusiveSum(at(g.o_tmp), tb, (const uint64_t*) at(g.o_cnt),
-                                const_cast<uint64_t*>(a.prefix), (int64_t) (g.n + 1), c.stream);
+  if (pipeline) {
+    k_plan_counts<<<pblocks, 256, 0, c.stream>>>(a.probs, a.order, n, g.ndir, a.pipe_rows,
+                                                (uint64_t*) at(g.o_cnt));
+    tb = g.cub_tmp;
+    cub::DeviceScan::ExclusiveSum(at(g.o_tmp), tb, (const uint64_t*) at(g.o_cnt),
+                                  const_cast<uint64_t*>(a.prefix), (int64_t) (g.n + 1), c.stream);
+  }
   BatchArgs kernel_args = a;
   void* kargs[] = {&kernel_args};
   // Fork: the one-warp path runs on a side branch of the graph, beside the
@@ -1258,7 +1267,7 @@ hd_status capture_batch_graph(Ctx& c, const BatchGraph& g, cudaGraphExec_t* out)
   cudaLaunchKernel(g.fns[4], dim3(g.grids[4]), dim3(kBatchThreads), kargs, 0, c.batch_side);
   cudaEventRecord(c.batch_join, c.batch_side);
   const uint64_t npd = g.n * g.ndir;
-  for (int k = 0; k < 4; ++k) {
+  for (int k = 0; k < 4 && pipeline; ++k) {
     if (k == 2)  // between seed and sweep
       k_batch_fold<<<(unsigned) ((npd + 255) / 256), 256, 0, c.stream>>>(a.ubound, a.smin, npd,
                                                                          a.keys);
@@ -1266,10 +1275,10 @@ hd_status capture_batch_graph(Ctx& c, const BatchGraph& g, cudaGraphExec_t* out)
   }
   cudaStreamWaitEvent(c.stream, c.batch_join, 0);
   const unsigned cblocks = (unsigned) ((g.n * g.ndir * 32 + 255) / 256);
-  if (g.dims == 2)
+  if (pipeline && g.dims == 2)
     k_batch_certify<2><<<cblocks, 256, 0, c.stream>>>(a.A, a.B, a.probs, n, g.ndir, a.keys, g.pd,
                                                       a.pipe_rows);
-  else
+  else if (pipeline)
     k_batch_certify<3><<<cblocks, 256, 0, c.stream>>>(a.A, a.B, a.probs, n, g.ndir, a.keys, g.pd,
                                                       a.pipe_rows);
   k_batch_finalize<<<(unsigned) ((g.n + 255) / 256), 256, 0, c.stream>>>(g.pd, n, g.ndir, g.out,
@@ -1358,6 +1367,7 @@ hd_status batch_solve(Ctx& c, const float* A, uint64_t total_a, const float* B, 
   // first: keys and window bounds (zero), seed minima (0xFF bytes).
   Layout L;
   const size_t o_keys = L.take(n * 2 * 8);
+  g.key_bytes = L.off;
   const size_t o_ub = L.take(n * 2 * kSlots * 8);
   g.zero_bytes = L.off;
   g.o_smin = L.take(n * 2 * kSlots * 4);
@@ -1485,8 +1495,9 @@ hd_status batch_solve(Ctx& c, const float* A, uint64_t total_a, const float* B, 
   cudaGraphExec_t exec = nullptr;
   if ((s = batch_graph_for(c, g, key, &exec)) != HD_OK) return s;
   e = cudaGraphLaunch(exec, c.stream);
-  c.launches += 11;  // own kernels: reset, plan keys, plan counts, one-warp path, window, seed,
-                     // fold, sweep, long, certify, finalize
+  // Own kernels: reset, plan keys, one-warp path, finalize; and the pipeline's plan
+  // counts, window, seed, fold, sweep, long, certify.
+  c.launches += total ? 11 : 4;
   if (e != cudaSuccess) return cuda_fail(c, e, "graph launch");
   if (stage_bad) {
     if ((e = cudaMemcpyAsync(out, g.out, n * sizeof(hd_batch_result), cudaMemcpyDeviceToHost,

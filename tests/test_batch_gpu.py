@@ -126,6 +126,26 @@ def test_batch_nearest_points(dims, small_rows):
         assert int(out["ib"][p]) == int(np.argmin(d2[row])), p
 
 
+@pytest.mark.parametrize("dims", [2, 3])
+def test_batch_with_and_without_the_pipeline(engine, dims):
+    """Directions of more than 65,536 rows bring the multi-pass pipeline into
+    the graph; the same engine takes batches with and without them in turn."""
+    rng = np.random.default_rng(77 + dims)
+    for na, nb in (([65_536, 40, 3], [300, 64, 5]), ([65_537, 100, 3], [300, 66_000, 5]),
+                   ([50, 40], [300, 64])):
+        a = rng.random((sum(na), dims)).astype(np.float32)
+        b = rng.random((sum(nb), dims)).astype(np.float32)
+        oa, ob = np.concatenate([[0], np.cumsum(na)]), np.concatenate([[0], np.cumsum(nb)])
+        for undirected in (False, True):
+            out = engine.solve_batch(a, b, oa, ob, undirected=undirected)
+            for p in range(len(na)):
+                x, y = a[oa[p]:oa[p + 1]], b[ob[p]:ob[p + 1]]
+                want = hd_oracle.hd_f32(x, y, undirected=undirected)
+                assert out["hd_f32"][p] == want["hd_f32"], (p, undirected)
+                src, dst = (x, y) if out["direction"][p] == 0 else (y, x)
+                assert hd_oracle.dist2_f32(src[out["ia"][p]], dst[out["ib"][p]]) == want["d2"]
+
+
 def test_batch_rejects_out_of_range_offsets(engine):
     import hausdorffdistance_gb300 as hd
     a = np.ones((4, 2), np.float32)
