@@ -189,6 +189,50 @@ __device__ __forceinline__ float prune32(double best, double rxy) {
   return p >= (double) FLT_MAX ? INFINITY : __double2float_ru(p);
 }
 
+// A thread's findings to the set's: exponent, flags, box.
+template <int D>
+__device__ __forceinline__ void round_findings(uint32_t emax, uint32_t fl, float (&lo)[D ? D : 1],
+                                               float (&hi)[D ? D : 1], RoundStats* st,
+                                               uint32_t* ord) {
+  constexpr int kStep = D ? D : 1;
+#pragma unroll
+  for (int o = 16; o; o >>= 1) {
+    emax = max(emax, __shfl_xor_sync(0xFFFFFFFFu, emax, o));
+    fl |= __shfl_xor_sync(0xFFFFFFFFu, fl, o);
+    if (D) {
+#pragma unroll
+      for (int k = 0; k < kStep; ++k) {
+        lo[k] = fminf(lo[k], __shfl_xor_sync(0xFFFFFFFFu, lo[k], o));
+        hi[k] = fmaxf(hi[k], __shfl_xor_sync(0xFFFFFFFFu, hi[k], o));
+      }
+    }
+  }
+  if ((threadIdx.x & 31) == 0) {
+    if (emax) atomicMax(&st->emax, emax);
+    if (fl) atomicOr(&st->flags, fl);
+  }
+  if constexpr (D > 0) {
+    __shared__ uint32_t s_lo[D], s_hi[D];
+    if (threadIdx.x < D) {
+      s_lo[threadIdx.x] = 0xFFFFFFFFu;
+      s_hi[threadIdx.x] = 0u;
+    }
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) {
+#pragma unroll
+      for (int k = 0; k < D; ++k) {
+        atomicMin(&s_lo[k], f2ord(lo[k]));
+        atomicMax(&s_hi[k], f2ord(hi[k]));
+      }
+    }
+    __syncthreads();
+    if (threadIdx.x < D) {
+      atomicMin(&ord[threadIdx.x], s_lo[threadIdx.x]);
+      atomicMax(&ord[4 + threadIdx.x], s_hi[threadIdx.x]);
+    }
+  }
+}
+
 // Cuts a set to float (Xf may be null: check only); records the largest
 // exponent, non-finite and out-of-range values, and tiny magnitudes.
 // Integer operations only, but for D = 2 or 3: there the box of the cut
@@ -230,42 +274,64 @@ __global__ void k_f64_round(const double* __restrict__ X, uint64_t total, float*
       }
     }
   }
+  round_findings<D>(emax, fl, lo, hi, st, ord);
+}
+
+// The same with two points per step by 16-byte loads, for sets of 2-D or 3-D
+// points that begin on a 16-byte boundary.  HBM bound (24 or 36 bytes a point,
+// 0.75 of the copy rate at 10M); half as many steps: the call on 300k x 400k
+// points 216 -> 208 us, 2M x 3M in 2-D 433 -> 427, 4M x 5M 372 -> 370, but 10M x 10M
+// 505 -> 510: so not for sets of kRoundPairsBelow points and more.
+constexpr uint64_t kRoundPairsBelow = 7000000;
+template <int D>
+__global__ void k_f64_round_pairs(const double* __restrict__ X, uint64_t total,
+                                  float* __restrict__ Xf, RoundStats* st,
+                                  uint32_t* __restrict__ ord) {
+  uint32_t emax = 0, fl = 0;
+  float lo[D], hi[D];
 #pragma unroll
-  for (int o = 16; o; o >>= 1) {
-    emax = max(emax, __shfl_xor_sync(0xFFFFFFFFu, emax, o));
-    fl |= __shfl_xor_sync(0xFFFFFFFFu, fl, o);
-    if (D) {
+  for (int k = 0; k < D; ++k) {
+    lo[k] = FLT_MAX;
+    hi[k] = -FLT_MAX;
+  }
+  auto cut = [&](double x, int k) {
+    const unsigned long long a = dbits(x) & 0x7FFFFFFFFFFFFFFFull;
+    const uint32_t ex = (uint32_t) (a >> 52);
+    if (ex == 0x7FFu)
+      fl |= kF64NonFinite;
+    else if (a > kRangeBits)
+      fl |= kF64Range;
+    if (ex >= 1023u - 126u)
+      emax = max(emax, ex);
+    else if (a != 0ull)
+      fl |= kF64Tiny;
+    const float f = cut_to_float(x);
+    lo[k] = fminf(lo[k], f);
+    hi[k] = fmaxf(hi[k], f);
+    return f;
+  };
+  const uint64_t stride = (uint64_t) gridDim.x * blockDim.x;
+  const uint64_t me = blockIdx.x * (uint64_t) blockDim.x + threadIdx.x;
+  const uint64_t pairs = total / (2 * D);
+  for (uint64_t t = me; t < pairs; t += stride) {
+    double2 v[D];
 #pragma unroll
-      for (int k = 0; k < kStep; ++k) {
-        lo[k] = fminf(lo[k], __shfl_xor_sync(0xFFFFFFFFu, lo[k], o));
-        hi[k] = fmaxf(hi[k], __shfl_xor_sync(0xFFFFFFFFu, hi[k], o));
-      }
+    for (int i = 0; i < D; ++i) v[i] = reinterpret_cast<const double2*>(X)[t * D + i];
+#pragma unroll
+    for (int i = 0; i < D; ++i) {
+      const float2 f = make_float2(cut(v[i].x, (2 * i) % D), cut(v[i].y, (2 * i + 1) % D));
+      if (Xf) reinterpret_cast<float2*>(Xf)[t * D + i] = f;
     }
   }
-  if ((threadIdx.x & 31) == 0) {
-    if (emax) atomicMax(&st->emax, emax);
-    if (fl) atomicOr(&st->flags, fl);
-  }
-  if constexpr (D > 0) {
-    __shared__ uint32_t s_lo[D], s_hi[D];
-    if (threadIdx.x < D) {
-      s_lo[threadIdx.x] = 0xFFFFFFFFu;
-      s_hi[threadIdx.x] = 0u;
-    }
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0) {
+  if (me == 0 && total % (2 * D)) {  // the last of an odd number of points
 #pragma unroll
-      for (int k = 0; k < D; ++k) {
-        atomicMin(&s_lo[k], f2ord(lo[k]));
-        atomicMax(&s_hi[k], f2ord(hi[k]));
-      }
-    }
-    __syncthreads();
-    if (threadIdx.x < D) {
-      atomicMin(&ord[threadIdx.x], s_lo[threadIdx.x]);
-      atomicMax(&ord[4 + threadIdx.x], s_hi[threadIdx.x]);
+    for (int k = 0; k < D; ++k) {
+      const uint64_t i = 2 * D * pairs + k;
+      const float f = cut(X[i], k);
+      if (Xf) Xf[i] = f;
     }
   }
+  round_findings<D>(emax, fl, lo, hi, st, ord);
 }
 
 __global__ void k_f64_init(F64Aux* aux) {
@@ -943,6 +1009,8 @@ hd_status hd_solve_f64(hd_ctx* c, const double* A, uint64_t n_a, const double* B
         (int) std::max<uint64_t>(1, std::min<uint64_t>((total + 255) / 256, (uint64_t) c->num_sms * 8));
     uint32_t* ord = &scalars(*c, 0)->mbr_ord[k][0][0];
     auto kern = n_dims == 2 ? k_f64_round<2> : n_dims == 3 ? k_f64_round<3> : k_f64_round<0>;
+    if (spatial_dims && nn[k] < kRoundPairsBelow && ((uintptr_t) d64[k] & 15) == 0)
+      kern = n_dims == 2 ? k_f64_round_pairs<2> : k_f64_round_pairs<3>;
     kern<<<grid, 256, 0, c->stream>>>(d64[k], total, (float*) p, &aux->round[k], ord);
     if ((s = after_launch(*c, "f64_round")) != HD_OK) return s;
   }

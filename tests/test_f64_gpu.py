@@ -230,3 +230,22 @@ def test_f64_matches_reference_double_golden(engine, case):
     a, b = rd(case["a"]).copy(), rd(case["b"]).copy()
     r = engine.solve_f64(a, b)
     assert int(np.float64(r.hd).view(np.uint64)) == case["hd_bits"]
+
+
+@pytest.mark.parametrize("dims", [2, 3])
+@pytest.mark.parametrize("skip,n", [(0, 1000), (0, 1001), (1, 1000), (1, 1001), (0, 1), (1, 2),
+                                    (0, 50_001), (1, 50_000)])
+def test_cut_by_pairs_of_points(engine, dims, skip, n):
+    """Two points per step where the set begins on a 16-byte boundary, one
+    elsewhere; odd numbers leave one over.  The far row is the last one."""
+    import torch
+    rng = np.random.default_rng(dims * 10 + skip + n)
+    a, b = rng.random((n + skip, dims)), rng.random((n + skip, dims))
+    a[-1] = 7.0
+    ta, tb = torch.from_numpy(a).cuda()[skip:], torch.from_numpy(b).cuda()[skip:]
+    r = engine.solve_f64(ta, tb, undirected=True)
+    a, b = a[skip:], b[skip:]
+    ab, ba = hd_oracle.exact_f64(a, b), hd_oracle.exact_f64(b, a)
+    assert r.hd_ab == np.sqrt(ab[0]) and r.hd_ba == np.sqrt(ba[0])
+    win = ba if ba[0] > ab[0] else ab
+    assert (int(r.ia), int(r.ib)) == (win[1], win[2])
