@@ -331,6 +331,7 @@ hd_status run_lbvh(Ctx& c, const DirInput& in);
 // Both directions of an undirected solve with shared launches.
 hd_status run_lbvh_pair(Ctx& c, const DirInput& ab, const DirInput& ba);
 hd_status run_grid(Ctx& c, const DirInput& in);
+constexpr int kBf16MaxDims = 64;  // tiles are built for rows of 16, 32, 48 and 64
 hd_status run_bf16(Ctx& c, const DirInput& in, DirResult* extra);
 // Test hook: the BF16 kernel's approximate row minima (no certification).
 hd_status bf16_rowmin_debug(Ctx& c, const DirInput& in, float* rowmin_host);

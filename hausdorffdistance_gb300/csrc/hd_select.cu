@@ -250,7 +250,7 @@ bool select_variant_by_size(const Ctx& c, uint64_t nA, uint64_t nB, int dims, in
     // The tiles take about 95 us per direction at least; the scan passes that at
     // 1.4e6 pairs in 10-D, 4e6 in 4-D.
     const double least = tu.bf16_min_pairs * (dims <= 8 ? 2.0 : 1.0);
-    *v = ((dims % 16 == 0 || dims <= 64) && pairs >= least) ? HD_VARIANT_BF16 : HD_VARIANT_EB;
+    *v = dims <= kBf16MaxDims && pairs >= least ? HD_VARIANT_BF16 : HD_VARIANT_EB;
     return true;
   }
   const bool sample = c.opt.always_sample != 0;

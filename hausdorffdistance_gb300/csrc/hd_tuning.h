@@ -8,7 +8,7 @@ struct Tuning {
   double eb_small_pairs;  // |A|*|B| at or below which AUTO takes EB unsampled
   double index_min_pairs; // |A|*|B| from which AUTO takes the index unsampled
   double eb_ratio;        // EB when |A| * p80 / (|A| + |B|) is below this
-  double bf16_min_pairs;  // n_dims % 16 == 0: BF16 tiles from this |A|*|B| up
+  double bf16_min_pairs;  // n_dims to 64 but 2, 3: BF16 tiles from this |A|*|B| up
   double eb_sample_max_pairs;  // the EB sample runs up to this |A|*|B|
   double grid_max_outside;     // grid only when at most this query fraction is outside
   double grid_max_skew;        // grid only when the target's occupancy skew is at most this

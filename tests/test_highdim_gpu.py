@@ -135,3 +135,18 @@ def test_auto_pads_to_tiles(engine, dims, kind):
     src, dst = (a, b) if r.direction == 0 else (b, a)
     assert hd_oracle.dist2_f32(src[r.ia], dst[r.ib]) == want["d2"]
     assert r.variant_used == 4
+
+
+# No tiles are built past 64 dimensions: AUTO scans there at any size.
+@pytest.mark.parametrize("dims", [65, 80, 96, 100, 112, 127, 128])
+@pytest.mark.parametrize("na,nb", [(2011, 1501), (300, 7001)])
+def test_auto_scans_beyond_the_tiles(engine, dims, na, nb):
+    rng = np.random.default_rng(dims + na)
+    a = rng.standard_normal((na, dims)).astype(np.float32)
+    b = rng.standard_normal((nb, dims)).astype(np.float32)
+    r = engine.solve(a, b, undirected=True)
+    want = hd_oracle.hd_f32(a, b, undirected=True)
+    assert np.float32(r.hd_f32) == want["hd_f32"]
+    src, dst = (a, b) if r.direction == 0 else (b, a)
+    assert hd_oracle.dist2_f32(src[r.ia], dst[r.ib]) == want["d2"]
+    assert r.variant_used == 1 and r.variant_used_ba == 1
