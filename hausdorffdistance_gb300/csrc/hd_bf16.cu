@@ -110,29 +110,34 @@ __global__ void k_bf16_pack(const float* __restrict__ X, uint64_t n, int D, int 
   }
 }
 
-// B's norms: their maximum, and +inf for the padded rows, which then never win
-// a minimum.  The same launch starts A's row minima and candidate minima at
-// their largest.
+// B's norms: their maximum (rows with a NaN, nobody's nearest, aside), and +inf
+// for the padded rows, which then never win a minimum.  The same launch starts
+// A's row minima and candidate minima at their largest, and notes whether A has
+// norms that are NaN (1) or infinite (2).
 __global__ void k_bf16_norm_finish(float* __restrict__ norms, uint64_t n, uint64_t nPad,
                                    uint32_t* __restrict__ maxnorm_ord,
                                    uint32_t* __restrict__ rowmin, uint32_t* __restrict__ cand_min,
-                                   uint64_t nA) {
-  uint32_t local = 0;
+                                   uint64_t nA, const float* __restrict__ anorm,
+                                   uint32_t* __restrict__ odd) {
+  uint32_t local = 0, fl = 0;
   const uint64_t t = blockIdx.x * (uint64_t) blockDim.x + threadIdx.x;
   const uint64_t stride = (uint64_t) gridDim.x * blockDim.x;
   for (uint64_t i = t; i < nPad; i += stride) {
-    if (i < n)
-      local = max(local, f2ord(sqrtf(norms[i])));
-    else
+    if (i >= n)
       norms[i] = INFINITY;
+    else if (norms[i] >= 0.0f)
+      local = max(local, f2ord(sqrtf(norms[i])));
   }
   for (uint64_t i = t; i < nA; i += stride) {
+    const float a = anorm[i];
+    if (!(a < INFINITY)) fl |= a == INFINITY ? 2u : 1u;
     rowmin[i] = 0xFFFFFFFFu;
     cand_min[i] = 0xFFFFFFFFu;
   }
 #pragma unroll
   for (int o = 16; o; o >>= 1) local = max(local, __shfl_xor_sync(0xFFFFFFFFu, local, o));
   if ((threadIdx.x & 31) == 0) atomicMax(maxnorm_ord, local);
+  if (fl) atomicOr(odd, fl);
 }
 
 // ---- tcgen05 / mbarrier helpers (inline PTX) --------------------------------
@@ -249,6 +254,7 @@ struct Bf16Scalars {
   uint32_t lo_ord;     // L: max over completed rows of (m_i - E_i) (order-preserving bits)
   uint32_t cand;       // candidate count
   uint32_t status;
+  uint32_t odd_a;      // A has norms that are NaN (1) or infinite (2)
   uint32_t live[kMaxRounds];   // rows still open after each round
   uint32_t seeds[kMaxRounds];  // rows completed ahead of their turn after each round
   float seed_level;            // rows with a partial minimum above it are taken as seeds
@@ -743,7 +749,8 @@ hd_status run_bf16_k(Ctx& c, const DirInput& in, DirResult* extra, float* rowmin
   if ((s = after_launch(c, "bf16_pack_b")) != HD_OK) return s;
   // A's norm maximum is not needed; B's gives the bound.
   k_bf16_norm_finish<<<c.num_sms * 4, 256, 0, c.stream>>>(nb, in.nB, padB, &bs->bmax_ord,
-                                                          (uint32_t*) rm, cand_min, in.nA);
+                                                          (uint32_t*) rm, cand_min, in.nA, na,
+                                                          &bs->odd_a);
   if ((s = after_launch(c, "bf16_norms")) != HD_OK) return s;
   mark(c, 1);
   mark(c, 2);
@@ -862,7 +869,13 @@ hd_status run_bf16_k(Ctx& c, const DirInput& in, DirResult* extra, float* rowmin
     extra->err_bound = 2.0 * (2.0 * cK * b * b + std::ldexp(1.0, -21) * sq +
                               (Kp + 2.0) * std::ldexp(1.0, -24) * sq);
   }
-  if (h.cand > limit) return run_eb_nd(c, in);
+  // Where norms or approximate minima overflow (coordinates whose squares leave
+  // the FP32 range) the bounds say nothing; the scan compares the differences
+  // themselves.  Rows with a NaN drop out here and are an error there: AUTO
+  // leaves them to the scan whatever its choice by size.
+  const bool bounded = std::isfinite(ord2f(h.bmax_ord)) && std::isfinite(ord2f(h.lo_ord)) &&
+                       !(h.odd_a & 2u);
+  if (!bounded || (in.chosen && h.odd_a) || h.cand == 0 || h.cand > limit) return run_eb_nd(c, in);
   return certify(c, in);
 }
 

@@ -563,7 +563,7 @@ hd_status hd_solve(hd_ctx* c, const float* A, uint64_t n_a, const float* B,
   DirInput ins[2];
   for (int d = 0; d < ndir; ++d) {
     ins[d] = DirInput{d == 0 ? dA : dB, d == 0 ? n_a : n_b, d == 0 ? dB : dA,
-                      d == 0 ? n_b : n_a, n_dims, d, count};
+                      d == 0 ? n_b : n_a, n_dims, d, count, variant == HD_VARIANT_AUTO};
     used[d] = variant;
   }
   // The cell filter runs before the indexes (not before an early-break scan,

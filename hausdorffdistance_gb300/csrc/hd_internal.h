@@ -306,6 +306,7 @@ struct DirInput {
   int dims;
   int dir;      // 0: A->B, 1: B->A (selects the DevScalars slot)
   bool count;
+  bool chosen = false;  // AUTO chose the variant
 };
 
 // Records the first failure on the context and returns its status.

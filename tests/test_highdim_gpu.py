@@ -150,3 +150,41 @@ def test_auto_scans_beyond_the_tiles(engine, dims, na, nb):
     src, dst = (a, b) if r.direction == 0 else (b, a)
     assert hd_oracle.dist2_f32(src[r.ia], dst[r.ib]) == want["d2"]
     assert r.variant_used == 1 and r.variant_used_ba == 1
+
+
+# Inputs that leave the tiles' bounds without a value: AUTO answers what the scan
+# by name answers, or fails as it does (a row with a NaN has no nearest point).
+# The sizes are below and above those of runs of tiles.
+@pytest.mark.parametrize("kind", ["nan_targets", "huge_targets", "all_huge", "nan_row",
+                                  "huge_row", "huge_row_and_products"])
+@pytest.mark.parametrize("dims,na,nb", [(10, 2105, 1999), (16, 2105, 1999), (64, 200, 15_001),
+                                        (16, 50_001, 40_003)])
+def test_auto_where_bounds_have_no_value(engine, kind, dims, na, nb):
+    import hausdorffdistance_gb300 as hd
+    rng = np.random.default_rng(dims + na)
+    a = rng.random((na, dims)).astype(np.float32)
+    b = (rng.random((nb, dims)) * 1.05).astype(np.float32)
+    keep = np.ones(nb, bool)
+    if kind == "all_huge":  # FP32 values near 2e19 lie 2e12 apart
+        a = (2e19 + 1e16 * a.astype(np.float64)).astype(np.float32)
+        b = (2e19 + 1e16 * b.astype(np.float64)).astype(np.float32)
+    elif kind in ("nan_targets", "huge_targets"):
+        keep[::700] = False
+        b[~keep, dims // 2] = 1e25 if kind == "huge_targets" else np.nan
+        a[7] = 0.0
+    else:
+        if kind == "huge_row_and_products":
+            b += np.float32(4.0)
+        a[7, 1] = np.nan if kind == "nan_row" else 1e38
+    got = []
+    for variant in ("auto", "eb"):
+        try:
+            r = engine.solve(a, b, variant=variant)
+            got.append((np.float32(r.hd_f32), r.hd, int(r.ia), int(r.ib)))
+        except hd.HDError as e:
+            got.append(e.status)
+    assert got[0] == got[1]
+    if keep.sum() < nb or kind == "all_huge":
+        d2 = hd_oracle.exact(a, b[keep], 32)[0]
+        assert got[0][0] == np.sqrt(np.float32(d2)) and keep[got[0][3]]
+        assert hd_oracle.dist2_f32(a[got[0][2]], b[got[0][3]]) == np.float32(d2)
