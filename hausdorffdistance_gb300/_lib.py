@@ -36,7 +36,9 @@ EXPORTED = ["hd_default_options", "hd_create", "hd_destroy", "hd_set_stream",
             "hd_solve", "hd_solve_f64", "hd_solve_batch", "hd_solve_batch_offsets", "hd_solve_batch_plain",
             "hd_last_error",
             "hd_status_string", "hd_kernel_launches", "hd_version", "hd_solve_eb_noalloc",
-            "hd_debug_bf16_rowmin", "hd_compute_stats"]
+            "hd_debug_bf16_rowmin", "hd_debug_no_room", "hd_compute_stats"]
+
+DEBUG_FILTER = 0
 
 HD_STATS_HIST_ROWS = 96
 
@@ -141,6 +143,8 @@ def load(path: str = LIB_PATH) -> ctypes.CDLL:
     lib.hd_solve_eb_noalloc.restype = ctypes.c_int
     lib.hd_debug_bf16_rowmin.argtypes = [P, P, ctypes.c_uint64, P, ctypes.c_uint64, ctypes.c_int, P]
     lib.hd_debug_bf16_rowmin.restype = ctypes.c_int
+    lib.hd_debug_no_room.argtypes = [P, ctypes.c_int, ctypes.c_uint32]
+    lib.hd_debug_no_room.restype = ctypes.c_int
     lib.hd_compute_stats.argtypes = [P, P, ctypes.c_uint64, ctypes.c_int, ctypes.c_uint32,
                                      ctypes.c_uint32, ctypes.POINTER(PointStats)]
     lib.hd_compute_stats.restype = ctypes.c_int

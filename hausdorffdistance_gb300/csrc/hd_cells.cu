@@ -1401,7 +1401,7 @@ hd_status cells_seed(Ctx& c, const DirInput* ins, int count, bool* seeded) {
 hd_status cells_hopeless(Ctx& c, int count, int dims, const CellsRun& run, bool* off,
                          float* reach) {
   for (int k = 0; k < count; ++k) {
-    off[k] = !run.ran;
+    off[k] = false;
     reach[k] = 0.0f;
   }
   if (!run.ran) return HD_OK;

@@ -53,10 +53,13 @@ hd_status ensure(Ctx& c, BufSlot slot, size_t bytes, void** out) {
     // do not reallocate every call.
     size_t want = std::max(bytes, b.bytes + b.bytes / 4);
     ++c.buf_gen;
-    cudaError_t e = cudaMalloc(&b.p, want);
+    auto grow = [&](size_t n) {
+      return c.no_room[slot] ? cudaErrorMemoryAllocation : cudaMalloc(&b.p, n);
+    };
+    cudaError_t e = grow(want);
     if (e != cudaSuccess) {
       (void) cudaGetLastError();
-      e = cudaMalloc(&b.p, bytes);
+      e = grow(bytes);
       DevBuf& filter = c.bufs[kBufCells];
       if (e != cudaSuccess && slot != kBufCells && !c.cells_live && filter.p) {
         // The cell filter's bitmaps and lists are not needed any more: their
@@ -66,11 +69,12 @@ hd_status ensure(Ctx& c, BufSlot slot, size_t bytes, void** out) {
           return cuda_fail(c, e, "sync before realloc");
         cudaFree(filter.p);
         filter = DevBuf{};
-        e = cudaMalloc(&b.p, bytes);
+        e = grow(bytes);
       }
       if (e != cudaSuccess) {
         (void) cudaGetLastError();
         b.p = nullptr;
+        if (c.no_room[slot]) --c.no_room[slot];
         return fail(c, HD_ERR_OOM,
                     "device allocation of " + std::to_string(bytes) + " bytes failed");
       }
@@ -853,6 +857,14 @@ hd_status hd_debug_bf16_rowmin(hd_ctx* c, const float* A, uint64_t n_a, const fl
   if ((s = init_scalars(*c)) != HD_OK) return s;
   DirInput in{dA, n_a, dB, n_b, n_dims, 0, false};
   return bf16_rowmin_debug(*c, in, rowmin_out);
+}
+
+hd_status hd_debug_no_room(hd_ctx* c, int buffer, uint32_t times) {
+  if (!c) return HD_ERR_INVALID_ARG;
+  switch (buffer) {
+  case HD_DEBUG_FILTER: c->no_room[kBufCells] = times; return HD_OK;
+  default: return HD_ERR_INVALID_ARG;
+  }
 }
 
 const char* hd_last_error(hd_ctx* c) {

@@ -222,6 +222,7 @@ struct Ctx {
   cudaStream_t own_stream = nullptr;
   cudaStream_t stream = nullptr;
   DevBuf bufs[kNumBufs];
+  uint32_t no_room[kNumBufs] = {};  // growths yet to be refused (hd_debug_no_room)
   void* host_pinned = nullptr;   // pinned result staging
   size_t host_pinned_bytes = 0;
   void* sel_pinned = nullptr;    // pinned staging of the selector's samples
@@ -446,7 +447,8 @@ hd_status cells_begin(Ctx& c, const DirInput* ins, int count, int level, const F
 // (seeded: false when there was no room).  Takes no read-back.
 hd_status cells_seed(Ctx& c, const DirInput* ins, int count, bool* seeded);
 // Waits for the filter's seeds alone: off[k] where it will give direction k up
-// (reach[k]: its L in cells), so that the index can be enqueued behind it.
+// (reach[k]: its L in cells), so that the index can be enqueued behind it.  False
+// when the filter did not run: there are no seeds to wait behind.
 hd_status cells_hopeless(Ctx& c, int count, int dims, const CellsRun& run, bool* off,
                          float* reach);
 // Runs `index` on a stream of its own behind the filter's seeds, beside the

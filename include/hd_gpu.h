@@ -286,6 +286,15 @@ HD_API hd_status hd_debug_bf16_rowmin(hd_ctx* ctx, const float* A, uint64_t n_a,
                                       const float* B, uint64_t n_b, int n_dims,
                                       float* rowmin_out);
 
+/* Test hook for the ways out when device memory runs short: the next `times`
+ * growths of a buffer of this context find no room, as if the device were full
+ * (nothing is allocated or held for it).  0 lifts it.  No counterpart in the
+ * reference. */
+typedef enum hd_debug_buffer {
+  HD_DEBUG_FILTER = 0  /* the cell filter's maps and lists                     */
+} hd_debug_buffer;
+HD_API hd_status hd_debug_no_room(hd_ctx* ctx, int buffer, uint32_t times);
+
 /* Bounding box, density and the occupancy of the reference's statistics
  * grid (n_points_cell points per cell on average) of one 2-D or 3-D point set,
  * host or device pointer (HD_DEVICE_PTRS), computed on the device.  Replaces
