@@ -154,6 +154,12 @@ __global__ void k_init_scalars(DevScalars* sc, int n) {
   }
 }
 
+__global__ void k_restart(DevScalars* sc) {
+  sc->min_key = ~0ull;
+  sc->next = sc->pairs = sc->nodes = sc->leaves = 0ull;
+  sc->heavy_count = sc->heavy_mark = 0u;
+}
+
 // Exact argmin over B for the certifying A point.  Scans the caller's B in
 // its own order so that ib is the caller's index; among equal squared
 // distances the lowest index wins (atomicMin on (d2 bits, index)).
@@ -325,6 +331,11 @@ hd_status init_scalars(Ctx& c) {
   if (s != HD_OK) return s;
   k_init_scalars<<<1, 32, 0, c.stream>>>((DevScalars*) p, 2);
   return after_launch(c, "init_scalars");
+}
+
+hd_status restart_direction(Ctx& c, int dir) {
+  k_restart<<<1, 1, 0, c.stream>>>(scalars(c, dir));
+  return after_launch(c, "restart");
 }
 
 }  // namespace hdg
@@ -648,6 +659,8 @@ hd_status hd_solve(hd_ctx* c, const float* A, uint64_t n_a, const float* B,
         r = index_beside(*c, index);
         if (r == HD_ERR_OOM) {  // after the filter then, with its room
           c->last_error.clear();
+          for (int d = 0; d < ndir; ++d)
+            if (indexed[d] && (r = restart_direction(*c, d)) != HD_OK) return r;
           indexed[0] = indexed[1] = false;
         } else if (r != HD_OK) {
           return r;
@@ -863,6 +876,7 @@ hd_status hd_debug_no_room(hd_ctx* c, int buffer, uint32_t times) {
   if (!c) return HD_ERR_INVALID_ARG;
   switch (buffer) {
   case HD_DEBUG_FILTER: c->no_room[kBufCells] = times; return HD_OK;
+  case HD_DEBUG_TREE: c->no_room[kBufNodes0] = times; return HD_OK;
   default: return HD_ERR_INVALID_ARG;
   }
 }

@@ -455,6 +455,9 @@ hd_status cells_hopeless(Ctx& c, int count, int dims, const CellsRun& run, bool*
 // filter's other kernels (which work on the other direction, or return at once);
 // the call's stream waits for it.  Planes undirected, 300k x 500k 470 -> 442 us
 // against the same behind those kernels, FP64 200k x 300k 524 -> 469.
+// When it fails (it may find no room while the filter holds its own) nothing of
+// it is left running, and the sorted sets it may have made count for nothing:
+// whoever tries again will use their buffers.
 template <class F>
 hd_status index_beside(Ctx& c, F index) {
   hd_status s = ensure_index_side(c);
@@ -465,10 +468,19 @@ hd_status index_beside(Ctx& c, F index) {
   c.stream = c.index_side;
   s = index();
   c.stream = main;
+  if (s != HD_OK) {
+    c.sorted_valid = false;
+    cudaStreamSynchronize(c.index_side);
+    if (c.batch_side) cudaStreamSynchronize(c.batch_side);
+    return s;
+  }
   e = cudaEventRecord(c.index_join, c.index_side);
   if (e == cudaSuccess) e = cudaStreamWaitEvent(main, c.index_join, 0);
-  return s == HD_OK && e != cudaSuccess ? cuda_fail(c, e, "index stream") : s;
+  return e != cudaSuccess ? cuda_fail(c, e, "index stream") : HD_OK;
 }
+// Readies a direction's scalars for another try at it (its running maximum and
+// the sets' boxes hold).
+hd_status restart_direction(Ctx& c, int dir);
 hd_status cells_finish(Ctx& c, int count, const CellsRun& run, CellsLeft* left);
 // LBVH over what the filter left of `count` directions.
 hd_status run_lbvh_left(Ctx& c, const DirInput* ins, int count, F64Plan* plan,

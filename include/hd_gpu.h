@@ -291,7 +291,8 @@ HD_API hd_status hd_debug_bf16_rowmin(hd_ctx* ctx, const float* A, uint64_t n_a,
  * (nothing is allocated or held for it).  0 lifts it.  No counterpart in the
  * reference. */
 typedef enum hd_debug_buffer {
-  HD_DEBUG_FILTER = 0  /* the cell filter's maps and lists                     */
+  HD_DEBUG_FILTER = 0, /* the cell filter's maps and lists                     */
+  HD_DEBUG_TREE = 1    /* the index's nodes, allocated behind its sorts        */
 } hd_debug_buffer;
 HD_API hd_status hd_debug_no_room(hd_ctx* ctx, int buffer, uint32_t times);
 
