@@ -38,7 +38,7 @@ EXPORTED = ["hd_default_options", "hd_create", "hd_destroy", "hd_set_stream",
             "hd_status_string", "hd_kernel_launches", "hd_version", "hd_solve_eb_noalloc",
             "hd_debug_bf16_rowmin", "hd_debug_no_room", "hd_compute_stats"]
 
-DEBUG_FILTER, DEBUG_TREE = range(2)
+DEBUG_FILTER, DEBUG_TREE, DEBUG_TILES = range(3)
 
 HD_STATS_HIST_ROWS = 96
 

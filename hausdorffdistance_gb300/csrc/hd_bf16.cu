@@ -894,7 +894,16 @@ hd_status run_bf16_impl(Ctx& c, const DirInput& in, DirResult* extra, float* row
 }  // namespace
 
 hd_status run_bf16(Ctx& c, const DirInput& in, DirResult* extra) {
-  return run_bf16_impl(c, in, extra, nullptr);
+  const std::string before = c.last_error;
+  const hd_status s = run_bf16_impl(c, in, extra, nullptr);
+  if (s != HD_ERR_OOM || !in.chosen) return s;
+  // The packed sets take 4 bytes per padded coordinate each (a 1-D set 16 times its
+  // size), the scan a copy of B alone: what AUTO chose goes there when they don't
+  // fit, with their room.
+  c.last_error = before;
+  for (BufSlot b : {kBufBf16A, kBufBf16B, kBufBf16Open, kBufNorms, kBufRowMin, kBufCand})
+    release(c, b);
+  return run_eb_nd(c, in);
 }
 
 hd_status bf16_rowmin_debug(Ctx& c, const DirInput& in, float* rowmin_host) {

@@ -86,6 +86,15 @@ hd_status ensure(Ctx& c, BufSlot slot, size_t bytes, void** out) {
   return HD_OK;
 }
 
+void release(Ctx& c, BufSlot slot) {
+  DevBuf& b = c.bufs[slot];
+  if (!b.p) return;
+  cudaStreamSynchronize(c.stream);
+  cudaFree(b.p);
+  b = DevBuf{};
+  ++c.buf_gen;
+}
+
 hd_status after_launch(Ctx& c, const char* what) {
   ++c.launches;
   cudaError_t e = cudaGetLastError();
@@ -877,6 +886,7 @@ hd_status hd_debug_no_room(hd_ctx* c, int buffer, uint32_t times) {
   switch (buffer) {
   case HD_DEBUG_FILTER: c->no_room[kBufCells] = times; return HD_OK;
   case HD_DEBUG_TREE: c->no_room[kBufNodes0] = times; return HD_OK;
+  case HD_DEBUG_TILES: c->no_room[kBufBf16B] = times; return HD_OK;
   default: return HD_ERR_INVALID_ARG;
   }
 }

@@ -316,6 +316,8 @@ hd_status cuda_fail(Ctx& c, cudaError_t e, const char* what);
 
 // Returns the buffer, growing it (contents not kept) when smaller than bytes.
 hd_status ensure(Ctx& c, BufSlot slot, size_t bytes, void** out);
+// Gives a buffer back once the stream is through with it.
+void release(Ctx& c, BufSlot slot);
 
 // Counts a kernel launch and checks for launch errors.
 hd_status after_launch(Ctx& c, const char* what);

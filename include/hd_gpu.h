@@ -292,7 +292,8 @@ HD_API hd_status hd_debug_bf16_rowmin(hd_ctx* ctx, const float* A, uint64_t n_a,
  * reference. */
 typedef enum hd_debug_buffer {
   HD_DEBUG_FILTER = 0, /* the cell filter's maps and lists                     */
-  HD_DEBUG_TREE = 1    /* the index's nodes, allocated behind its sorts        */
+  HD_DEBUG_TREE = 1,   /* the index's nodes, allocated behind its sorts        */
+  HD_DEBUG_TILES = 2   /* the BF16 variant's packed copy of B                  */
 } hd_debug_buffer;
 HD_API hd_status hd_debug_no_room(hd_ctx* ctx, int buffer, uint32_t times);
 

@@ -121,3 +121,24 @@ def test_no_room_for_the_index_of_sets_given_up(undirected):
             engine.solve(a, b, undirected=undirected, variant="lbvh")
         assert e.value.status == 2
         check(a, b, engine.solve(a, b, undirected=undirected, variant="lbvh"), undirected)
+
+
+@pytest.mark.parametrize("refused", [1, 2])
+@pytest.mark.parametrize("undirected", [False, True])
+def test_no_room_for_the_tiles(refused, undirected):
+    """AUTO scans where the packed sets don't fit; by name the variant says so."""
+    import hausdorffdistance_gb300 as hd
+    from hausdorffdistance_gb300 import _lib
+    rng = np.random.default_rng(6)
+    a = rng.random((2105, 16)).astype(np.float32)
+    b = (rng.random((1999, 16)) * 1.05).astype(np.float32)
+    with hd.Engine() as engine:
+        no_room(engine, _lib.DEBUG_TILES, refused)
+        for _ in range(2):
+            check(a, b, engine.solve(a, b, undirected=undirected), undirected)
+    with hd.Engine() as engine:
+        no_room(engine, _lib.DEBUG_TILES, 1)
+        with pytest.raises(hd.HDError) as e:
+            engine.solve(a, b, undirected=undirected, variant="bf16")
+        assert e.value.status == 2
+        check(a, b, engine.solve(a, b, undirected=undirected, variant="bf16"), undirected)
