@@ -188,6 +188,15 @@ __device__ __forceinline__ uint32_t ld_relaxed_u32(const uint32_t* p) {
   return v;
 }
 
+// A plain load that the compiler knows to be of global memory: through a pointer
+// out of CellArgs it takes it for a generic one (the rows of k_cell_blocks at
+// 1024^3 cells 397 us, so 360).
+__device__ __forceinline__ unsigned long long ld_global_u64(const unsigned long long* p) {
+  unsigned long long v;
+  asm volatile("ld.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+
 // One slot per active lane from a counter, with one atomic per warp.
 __device__ __forceinline__ uint32_t take_slot(uint32_t* counter) {
   const unsigned act = __activemask();
@@ -412,7 +421,7 @@ struct RowWalk {
 // Several warps may share a visit: `j` is the lane's first row, `stride` the
 // number of lanes.  WARP = false: each thread visits alone (j = 0, stride = 1).
 template <class Ge, bool WARP, class Reach, class F, class Step>
-__device__ __forceinline__ void visit_blocks(const Probe<Ge>& p, const uint32_t* __restrict__ coarse,
+__device__ __forceinline__ void visit_blocks(const Probe<Ge>& p, const uint32_t* coarse,
                                              int j, int stride, Reach reach, F f, Step step) {
   constexpr int D = Ge::D;
   const unsigned long long* rows = reinterpret_cast<const unsigned long long*>(coarse);
@@ -456,7 +465,7 @@ __device__ __forceinline__ void visit_blocks(const Probe<Ge>& p, const uint32_t*
 // +inf when nothing lies there.
 template <class Ge>
 __device__ __forceinline__ float nearest_block(const Probe<Ge>& p,
-                                               const uint32_t* __restrict__ coarse, float stop) {
+                                               const uint32_t* coarse, float stop) {
   constexpr int D = Ge::D;
   const unsigned long long* rows = reinterpret_cast<const unsigned long long*>(coarse);
   const int lane = threadIdx.x & 31;
@@ -516,8 +525,8 @@ __device__ __forceinline__ float nearest_block(const Probe<Ge>& p,
 // settled against `stop`.  lb2 is +inf when it stopped, or found no cell.
 template <class Ge, bool WARP>
 __device__ __forceinline__ void cell_search(const Probe<Ge>& p,
-                                            const unsigned long long* __restrict__ occ,
-                                            const uint32_t* __restrict__ coarse, float stop,
+                                            const unsigned long long* occ,
+                                            const uint32_t* coarse, float stop,
                                             float* lb2, float* ub2) {
   constexpr int D = Ge::D;
   float lb = INFINITY, ub = INFINITY;
@@ -540,7 +549,7 @@ __device__ __forceinline__ void cell_search(const Probe<Ge>& p,
   visit_blocks<Ge, WARP>(
       p, coarse, WARP ? threadIdx.x & 31 : 0, WARP ? 32 : 1, [&]() { return fminf(lb, cap); },
       [&](uint32_t block, int bx, int by, int bz) {
-        unsigned long long m = __ldg(occ + block);
+        unsigned long long m = occ[block];
         while (m) {
           const int t = __ffsll((long long) m) - 1;
           m &= m - 1;
@@ -575,11 +584,11 @@ __device__ __forceinline__ void raise_level(CellDirState* st, float lb2) {
 // The target's coarse map for a CTA's searches: copied to shared memory (a
 // search is a chain of reads of it) unless it is too large.
 template <class Ge>
-__device__ __forceinline__ const uint32_t* search_map(const uint32_t* __restrict__ map) {
+__device__ __forceinline__ const uint32_t* search_map(const uint32_t* map) {
   if constexpr (Ge::kShared) {
     __shared__ uint4 s[Ge::kCoarse / 4];
     for (uint32_t i = threadIdx.x; i < Ge::kCoarse / 4; i += blockDim.x)
-      s[i] = __ldg(reinterpret_cast<const uint4*>(map) + i);
+      s[i] = reinterpret_cast<const uint4*>(map)[i];
     __syncthreads();
     return reinterpret_cast<const uint32_t*>(s);
   } else {
@@ -612,13 +621,13 @@ __global__ void __launch_bounds__(kSearchThreads) k_cell_seed(CellArgs a) {
   const uint32_t w = (blockIdx.x * kSearchWarps + (threadIdx.x >> 5)) *
                      ((uint32_t) (kMapWords * 0.618) | 1u) & (kMapWords - 1);
   const unsigned long long m =
-      __ldg(reinterpret_cast<const unsigned long long*>(a.coarse[d.qset]) + w);
+      reinterpret_cast<const unsigned long long*>(a.coarse[d.qset])[w];
   if (!m) return;
   // The last occupied block of the word's row but one in four takes the
   // first: clusters' edges, where the far points are.
   const int bit = (w & 3) ? 63 - __clzll((long long) m) : __ffsll((long long) m) - 1;
   const uint32_t block = w * 64 + bit;
-  const unsigned long long cells = __ldg(a.occ[d.qset] + block);
+  const unsigned long long cells = a.occ[d.qset][block];
   const Probe<Ge> p = probe_cell<Ge>(block * 64 + __ffsll((long long) cells) - 1);
   const float stop = __uint_as_float(ld_relaxed_u32(&d.st->L2));
   float lb, ub;
@@ -633,7 +642,7 @@ __global__ void __launch_bounds__(kSearchThreads) k_cell_seed(CellArgs a) {
 // 3^D) that lie within `stop` at the far corner, as masks of its 64 cells; the
 // first 64 threads of a CTA.
 template <class Ge>
-__device__ __forceinline__ void near_masks(float stop, int j, unsigned long long* __restrict__ out) {
+__device__ __forceinline__ void near_masks(float stop, int j, unsigned long long* out) {
   constexpr int D = Ge::D, S = Ge::S;
   const int sub = threadIdx.x;
   if (sub >= 64) return;
@@ -700,7 +709,7 @@ __global__ void __launch_bounds__(256) k_cell_blocks(CellArgs a) {
   __shared__ uint32_t s_sum[8], s_base;
   for (uint32_t block = blockIdx.x * 256 + threadIdx.x; block < Ge::kBlocks;
        block += gridDim.x * 256) {
-  const bool some = (__ldg(a.coarse[d.qset] + (block >> 5)) >> (block & 31)) & 1u;
+  const bool some = (a.coarse[d.qset][block >> 5] >> (block & 31)) & 1u;
   if (!__syncthreads_or(some)) continue;
   const unsigned long long m = some ? a.occ[d.qset][block] : 0ull;
   bool open = m != 0;
@@ -718,7 +727,7 @@ __global__ void __launch_bounds__(256) k_cell_blocks(CellArgs a) {
       const int x0 = max(bx - far, 0), x1 = min(bx + far, Ge::NB - 1);
       unsigned long long any = 0;
       for (int k = x0 >> 6; k <= x1 >> 6; ++k) {
-        unsigned long long bits = __ldg(w + k);
+        unsigned long long bits = ld_global_u64(w + k);
         if (k == x0 >> 6) bits &= ~0ull << (x0 & 63);
         if (k == x1 >> 6) bits &= ~0ull >> (63 - (x1 & 63));
         any |= bits;
@@ -788,7 +797,7 @@ __global__ void __launch_bounds__(256) k_cell_near(CellArgs a) {
   }
   const uint32_t n = HALF ? d.st->n_rim : d.st->n_cells;
   if (blockIdx.x * 256 >= n) return;
-  for (int i = threadIdx.x; i < kN * 64; i += 256) mask[i] = __ldg(d.masks + (HALF ? kN * 64 : 0) + i);
+  for (int i = threadIdx.x; i < kN * 64; i += 256) mask[i] = d.masks[(HALF ? kN * 64 : 0) + i];
   __syncthreads();
   const unsigned long long* occ = HALF ? a.half[1 - d.qset] : a.occ[1 - d.qset];
   // 3-D: listed cells -> rim -> far; 2-D: listed cells -> far.
@@ -807,16 +816,16 @@ __global__ void __launch_bounds__(256) k_cell_near(CellArgs a) {
       bz >>= 1;
       block = (uint32_t) ((bz * NB + by) * NB + bx);
     }
-    bool open = !(__ldg(occ + block) & mask[kN / 2 * 64 + sub]);
+    bool open = !(occ[block] & mask[kN / 2 * 64 + sub]);
     if (open) {
 #pragma unroll
       for (int r = 0; r < kN / 3; ++r) {
         const int y = by + r % 3 - 1, z = D == 3 ? bz + r / 3 - 1 : 0;
         if (!open || (uint32_t) y >= (uint32_t) NB || (uint32_t) z >= (uint32_t) NB) continue;
         const unsigned long long* w = occ + ((size_t) (D == 3 ? z * NB + y : y) * NB + bx);
-        unsigned long long hit = __ldg(w) & mask[(3 * r + 1) * 64 + sub];
-        if (bx > 0) hit |= __ldg(w - 1) & mask[3 * r * 64 + sub];
-        if (bx < NB - 1) hit |= __ldg(w + 1) & mask[(3 * r + 2) * 64 + sub];
+        unsigned long long hit = w[0] & mask[(3 * r + 1) * 64 + sub];
+        if (bx > 0) hit |= w[-1] & mask[3 * r * 64 + sub];
+        if (bx < NB - 1) hit |= w[1] & mask[(3 * r + 2) * 64 + sub];
         if (hit) open = false;
       }
     }
@@ -965,7 +974,7 @@ __global__ void __launch_bounds__(kSearchThreads) k_cell_mark(CellArgs a) {
       visit_blocks<Ge, true>(
           p, map, threadIdx.x, kSearchThreads, [&]() { return r2; },
           [&](uint32_t block, int bx, int by, int bz) {
-            unsigned long long m = __ldg(occ + block), hit = 0ull;
+            unsigned long long m = occ[block], hit = 0ull;
             while (m) {
               const int t = __ffsll((long long) m) - 1;
               m &= m - 1;
@@ -992,12 +1001,12 @@ __global__ void __launch_bounds__(kSearchThreads) k_cell_mark(CellArgs a) {
 
 // The points in marked cells, as (x, y, z, row): queries of the direction that
 // asks for the set's points, targets of the other (blockIdx.y = set).  Four
-// points per thread and step; the set's map of blocks turns most away.
+// points per thread and step; the set's map of blocks turns most away.  Not
+// chained, so that the marks are constant here.
 template <class Ge>
 __global__ void __launch_bounds__(256) k_cell_collect(CellArgs a, const float* __restrict__ A,
                                                       uint64_t nA, const float* __restrict__ B,
                                                       uint64_t nB) {
-  chain_wait();
   constexpr int D = Ge::D;
   const int set = blockIdx.y;
   const bool ask = set < a.count && !a.d[set].st->off;               // direction `set`
@@ -1063,7 +1072,6 @@ __device__ __forceinline__ bool scan_takes(const CellDirState* st, uint32_t cap_
 // (with a plan, only that maximum).
 template <class Ge, bool COUNT>
 __global__ void __launch_bounds__(256) k_cell_solve(CellArgs a) {
-  chain_wait();
   constexpr int D = Ge::D;
   __shared__ float4 s[kScanTile];
   __shared__ unsigned long long red[2][8];

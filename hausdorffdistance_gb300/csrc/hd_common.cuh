@@ -149,7 +149,9 @@ __device__ __forceinline__ float soft_stop(float thr, float r) {
 // A kernel of a chain launched with programmatic stream serialization: lets the
 // next kernel's CTAs take their places now, and waits until the kernels before
 // have finished and their writes are visible.  (No effect in a kernel launched
-// without the attribute.)
+// without the attribute.)  What the kernels before wrote is read by plain loads
+// behind it: the read-only path (__ldg, const __restrict__) wants data that stays
+// as it is for a kernel's whole life, which here begins beside their writes.
 __device__ __forceinline__ void chain_wait() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");

@@ -95,7 +95,7 @@ __device__ __forceinline__ void load_a(const float* __restrict__ A, uint64_t i,
 
 template <int D>
 __global__ void k_eb_pack(const float* __restrict__ B, uint64_t nB, Perm perm,
-                          typename EbPt<D>::T* __restrict__ out, uint64_t nPad) {
+                          typename EbPt<D>::T* out, uint64_t nPad) {
   chain_wait();
   for (uint64_t j = blockIdx.x * (uint64_t) blockDim.x + threadIdx.x; j < nPad;
        j += (uint64_t) gridDim.x * blockDim.x) {
@@ -129,7 +129,7 @@ __device__ __forceinline__ float tile_d2(float ax, float ay, float az,
 template <int D, int S = kEbSlots>
 __global__ void __launch_bounds__(kEbThreads)
     k_eb_main(const float* __restrict__ A, Perm permA, uint64_t a_begin,
-              uint64_t a_end, const typename EbPt<D>::T* __restrict__ Bp,
+              uint64_t a_end, const typename EbPt<D>::T* Bp,
               uint32_t nTiles, uint32_t capTiles, DevScalars* sc,
               HeavyEntry* heavy, uint32_t heavy_cap) {
   chain_wait();
@@ -331,7 +331,7 @@ __global__ void __launch_bounds__(kEbThreads)
 // raise it, and the partial minimum it records is at or below it too.
 template <int D>
 __global__ void __launch_bounds__(kEbThreads)
-    k_eb_list(const float* __restrict__ A, const typename EbPt<D>::T* __restrict__ Bp,
+    k_eb_list(const float* __restrict__ A, const typename EbPt<D>::T* Bp,
               uint32_t nTiles, HeavyEntry* list, uint32_t* group_done, uint32_t n_host,
               const uint32_t* n_dev, uint32_t cap, DevScalars* sc) {
   chain_wait();
@@ -463,8 +463,8 @@ __global__ void __launch_bounds__(kEbThreads)
 // tiles through L2.
 template <int D>
 __global__ void __launch_bounds__(kEbThreads)
-    k_eb_heavy(const float* __restrict__ A, const typename EbPt<D>::T* __restrict__ Bp,
-               uint32_t nTiles, DevScalars* sc, const HeavyEntry* __restrict__ list,
+    k_eb_heavy(const float* __restrict__ A, const typename EbPt<D>::T* Bp,
+               uint32_t nTiles, DevScalars* sc, const HeavyEntry* list,
                const uint32_t* n_dev, uint32_t cap, const uint32_t* first_dev) {
   chain_wait();
   constexpr int P = kHeavySlots;
