@@ -84,6 +84,8 @@ struct Geo {
   static constexpr float kPad = (float) G / (1 << 21);     // see the head of this file
   // Searches read the coarse map from shared memory when it is small.
   static constexpr bool kShared = kCoarse * 4 <= 32768;
+  // Rings of rows that a seed looks through at most (it may stop at a lower bound).
+  static constexpr int kSeedRings = D == 3 ? 16 : 128;
   // Blocks per axis of a super-block, when it is not.
   static constexpr int kTop = D == 3 ? NB / 64 : NB / 512;
 };
@@ -159,6 +161,7 @@ struct CellDir {
 
 struct CellArgs {
   const uint32_t (*ord)[2][4];
+  int swapped;                  // the sets' boxes are in ord in the other order
   unsigned long long* occ[2];
   uint32_t* coarse[2];
   unsigned long long* half[2];  // 3-D: occupied cells of twice the size
@@ -284,7 +287,9 @@ __device__ __forceinline__ uint32_t half_cell(int bx, int by, int bz, int x, int
 }
 
 // The coarse maps, one bit per block with an occupied cell, and in 3-D the
-// occupied cells of twice the size (a block of them covers 2^3 blocks).
+// occupied cells of twice the size (a block of them covers 2^3 blocks).  The
+// query set's cells are counted in a sixteenth of the words; counted in full by
+// k_cell_blocks, which reads them again, they cost it 40 us of 400 at 1024^3 cells.
 template <class Ge>
 __global__ void __launch_bounds__(256) k_cell_coarse(CellArgs a) {
   chain_wait();
@@ -292,6 +297,10 @@ __global__ void __launch_bounds__(256) k_cell_coarse(CellArgs a) {
   const unsigned long long w = a.occ[blockIdx.y][block];
   const unsigned m = __ballot_sync(0xFFFFFFFFu, w != 0);
   if ((threadIdx.x & 31) == 0) a.coarse[blockIdx.y][block >> 5] = m;
+  if (m && ((block >> 5) * 0x9E3779B1u >> 28) == 0 && blockIdx.y < a.count) {
+    const uint32_t cells = __reduce_add_sync(0xFFFFFFFFu, (uint32_t) __popcll(w));
+    if ((threadIdx.x & 31) == 0) atomicAdd(&a.d[blockIdx.y].st->n_occ, 16 * cells);
+  }
   if constexpr (Ge::D == 3) {
     if (w == 0) return;
     const int bx = block % Ge::NB, by = block / Ge::NB % Ge::NB, bz = block / (Ge::NB * Ge::NB);
@@ -333,6 +342,29 @@ __device__ __forceinline__ Probe<Ge> probe_cell(uint32_t cell) {
   return p;
 }
 
+// The target's box in blocks: nothing of it lies outside.  (Its corners take the
+// same steps as the points.)
+template <class Ge>
+struct BlockBox {
+  int lo[Ge::D], hi[Ge::D];
+};
+
+template <class Ge>
+__device__ __forceinline__ BlockBox<Ge> block_box(const CellArgs& a, const CellGrid& g, int set) {
+  BlockBox<Ge> b;
+  const uint32_t(*ord)[4] = a.ord[a.swapped ? 1 - set : set];
+#pragma unroll
+  for (int k = 0; k < Ge::D; ++k) {
+    auto block = [&](float v) {
+      const float u = (v - g.lo[k]) * g.scale;
+      return u >= 0.0f ? (int) (min((uint32_t) u, (uint32_t) Ge::G - 1) >> Ge::kSub) : 0;
+    };
+    b.lo[k] = block(ord2f(ord[0][k]));
+    b.hi[k] = block(ord2f(ord[1][k]));
+  }
+  return b;
+}
+
 // Gap between the probe and block bk along axis k, less the padding.
 template <class Ge>
 __device__ __forceinline__ float block_gap(const Probe<Ge>& p, int k, int bk) {
@@ -341,7 +373,8 @@ __device__ __forceinline__ float block_gap(const Probe<Ge>& p, int k, int bk) {
   return fmaxf(fmaxf(c - p.hi[k], p.lo[k] - (c + S)) - Ge::kPad, 0.0f);
 }
 
-// A row of the coarse map, walked outward from the probe's block.
+// A row of the coarse map, walked outward from the probe's block (from the box's
+// nearest to it).
 template <class Ge>
 struct RowWalk {
   const unsigned long long* w = nullptr;  // the row's words; null: no row
@@ -349,10 +382,11 @@ struct RowWalk {
   unsigned long long m_right = 0, m_left = 0;
   float g2;  // the row's squared gap in y (and z)
 
-  __device__ __forceinline__ void open(const unsigned long long* rows, const Probe<Ge>& p, int by,
-                                       int bz) {
+  __device__ __forceinline__ void open(const unsigned long long* rows, const Probe<Ge>& p,
+                                       const BlockBox<Ge>& box, int by, int bz) {
     w = nullptr;
-    if ((uint32_t) by >= (uint32_t) Ge::NB || (Ge::D == 3 && (uint32_t) bz >= (uint32_t) Ge::NB))
+    if (by < box.lo[1] || by > box.hi[1] ||
+        (Ge::D == 3 && (bz < box.lo[Ge::D - 1] || bz > box.hi[Ge::D - 1])))
       return;
     g2 = block_gap<Ge>(p, 1, by);
     g2 *= g2;
@@ -361,8 +395,10 @@ struct RowWalk {
       g2 += gz * gz;
     }
     w = rows + (size_t) (Ge::D == 3 ? bz * Ge::NB + by : by) * Ge::kWords;
-    i_right = i_left = p.b[0] >> 6;
-    const unsigned long long m = w[i_right], up = ~0ull << (p.b[0] & 63);
+    // (A row of one word needs no better start than the probe's place.)
+    const int bx = Ge::kWords > 1 ? min(max(p.b[0], box.lo[0]), box.hi[0]) : p.b[0];
+    i_right = i_left = bx >> 6;
+    const unsigned long long m = w[i_right], up = ~0ull << (bx & 63);
     m_right = m & up;
     m_left = m & ~up;
   }
@@ -411,6 +447,36 @@ struct RowWalk {
   }
 };
 
+// Square rings of rows around the probe's place, moved into the target's box:
+// for a probe far from the box the nearest rows come first as well, and what lies
+// between takes no steps.  With rings around the probe itself, to the grid's ends,
+// one far cell's search took 290 us, and two 3-D sets of 1M points 3 extents apart
+// 16.6 ms undirected (the index alone 0.53, now 0.49).
+template <class Ge>
+struct Rings {
+  int c[2];      // the first row's y (and z)
+  float h[2];    // and its gaps
+  int last;      // rings past this one lie outside the box
+
+  __device__ __forceinline__ Rings(const Probe<Ge>& p, const BlockBox<Ge>& box) : last(0) {
+#pragma unroll
+    for (int k = 0; k < Ge::D - 1; ++k) {
+      const int lo = box.lo[k + 1], hi = box.hi[k + 1];
+      c[k] = min(max(p.b[k + 1], lo), hi);
+      h[k] = block_gap<Ge>(p, k + 1, c[k]);
+      last = max(last, max(c[k] - lo, hi - c[k]));
+    }
+  }
+  // Squared gap of ring q's rows, at least.
+  __device__ __forceinline__ float gap2(int q) const {
+    const float r = fmaxf((float) (Ge::S * (q - 1)) - Ge::kPad, 0.0f);
+    const float y = h[0] + r;
+    if constexpr (Ge::D == 2) return y * y;
+    const float z = h[1] + r;
+    return fminf(y * y + h[1] * h[1], h[0] * h[0] + z * z);
+  }
+};
+
 // Visits the target's occupied blocks around a probe, nearest rows first, with
 // a whole warp: the rows of blocks (along x) go round the lanes in square rings
 // (2-D: alternately above and below), and a lane walks a row's blocks outward
@@ -421,7 +487,8 @@ struct RowWalk {
 // Several warps may share a visit: `j` is the lane's first row, `stride` the
 // number of lanes.  WARP = false: each thread visits alone (j = 0, stride = 1).
 template <class Ge, bool WARP, class Reach, class F, class Step>
-__device__ __forceinline__ void visit_blocks(const Probe<Ge>& p, const uint32_t* coarse,
+__device__ __forceinline__ void visit_blocks(const Probe<Ge>& p, const BlockBox<Ge>& box,
+                                             const Rings<Ge>& rings, const uint32_t* coarse,
                                              int j, int stride, Reach reach, F f, Step step) {
   constexpr int D = Ge::D;
   const unsigned long long* rows = reinterpret_cast<const unsigned long long*>(coarse);
@@ -442,14 +509,13 @@ __device__ __forceinline__ void visit_blocks(const Probe<Ge>& p, const uint32_t*
         q = (j + 1) / 2;
         dy = (j & 1) ? q : -q;
       }
-      const float gap = fmaxf((float) (Ge::S * (q - 1)) - Ge::kPad, 0.0f);
-      if (q >= Ge::NB || gap * gap > reach()) {
+      if (q > rings.last || rings.gap2(q) > reach()) {
         j = -1;  // every further row is out of reach
         break;
       }
-      by = p.b[1] + dy;
-      bz = D == 3 ? p.b[2] + dz : 0;
-      row.open(rows, p, by, bz);
+      by = rings.c[0] + dy;
+      bz = D == 3 ? rings.c[1] + dz : 0;
+      row.open(rows, p, box, by, bz);
       j += stride;
     }
     if (WARP ? !__any_sync(0xFFFFFFFFu, x >= 0) : x < 0) return;
@@ -461,10 +527,10 @@ __device__ __forceinline__ void visit_blocks(const Probe<Ge>& p, const uint32_t*
 
 // Squared distance from a probe to the far corner of a near occupied block: the
 // smallest over the nearest blocks to either side in 81 rows of blocks around
-// the probe's (33 in 2-D), spaced so that they reach about 0.6 of sqrt(stop);
-// +inf when nothing lies there.
+// the rings' first (33 in 2-D), spaced so that they reach about 0.6 of
+// sqrt(stop); +inf when nothing lies there.
 template <class Ge>
-__device__ __forceinline__ float nearest_block(const Probe<Ge>& p,
+__device__ __forceinline__ float nearest_block(const Probe<Ge>& p, const Rings<Ge>& rings,
                                                const uint32_t* coarse, float stop) {
   constexpr int D = Ge::D;
   const unsigned long long* rows = reinterpret_cast<const unsigned long long*>(coarse);
@@ -479,8 +545,8 @@ __device__ __forceinline__ float nearest_block(const Probe<Ge>& p,
 #pragma unroll
   for (int j0 = 0; j0 < kRows; j0 += 32) {
     const int j = j0 + lane;
-    const int by = p.b[1] + (D == 3 ? j % 9 - 4 : j - 16) * step;
-    const int bz = D == 3 ? p.b[2] + (j / 9 - 4) * step : 0;
+    const int by = rings.c[0] + (D == 3 ? j % 9 - 4 : j - 16) * step;
+    const int bz = D == 3 ? rings.c[1] + (j / 9 - 4) * step : 0;
     if (j >= kRows || (uint32_t) by >= Ge::NB || (uint32_t) bz >= Ge::NB) continue;
     float r2 = far(1, by);
     r2 *= r2;
@@ -521,18 +587,25 @@ __device__ __forceinline__ float nearest_block(const Probe<Ge>& p,
 }
 
 // Squared lower and upper distance (cell units) from a probe to the nearest
-// of the target's occupied cells, by a warp or by each thread alone; the search stops once the upper one is
-// settled against `stop`.  lb2 is +inf when it stopped, or found no cell.
+// of the target's occupied cells, by a warp or by each thread alone; the search
+// stops once the upper one is settled against `stop`.  lb2 is +inf when it
+// stopped, or found no cell.  With `most` rings it ends after them: lb2 is then
+// at most the next ring's gap, ub2 of what it met.
 template <class Ge, bool WARP>
-__device__ __forceinline__ void cell_search(const Probe<Ge>& p,
+__device__ __forceinline__ void cell_search(const Probe<Ge>& p, const BlockBox<Ge>& box,
                                             const unsigned long long* occ,
                                             const uint32_t* coarse, float stop,
-                                            float* lb2, float* ub2) {
+                                            float* lb2, float* ub2, int most = Ge::NB) {
   constexpr int D = Ge::D;
   float lb = INFINITY, ub = INFINITY;
+  Rings<Ge> rings(p, box);
+  if (rings.last > most) {
+    lb = rings.gap2(most + 1);
+    rings.last = most;
+  }
   // The coarse map first: the far corner of the nearest occupied block bounds
   // the search from the start.
-  const float cap = WARP ? nearest_block<Ge>(p, coarse, stop) : INFINITY;
+  const float cap = WARP ? nearest_block<Ge>(p, rings, coarse, stop) : INFINITY;
   if (cap * kSlack < stop) {
     *lb2 = INFINITY;
     *ub2 = cap;
@@ -547,7 +620,8 @@ __device__ __forceinline__ void cell_search(const Probe<Ge>& p,
   };
   bool stopped = false;
   visit_blocks<Ge, WARP>(
-      p, coarse, WARP ? threadIdx.x & 31 : 0, WARP ? 32 : 1, [&]() { return fminf(lb, cap); },
+      p, box, rings, coarse, WARP ? threadIdx.x & 31 : 0, WARP ? 32 : 1,
+      [&]() { return fminf(lb, cap); },
       [&](uint32_t block, int bx, int by, int bz) {
         unsigned long long m = occ[block];
         while (m) {
@@ -631,7 +705,8 @@ __global__ void __launch_bounds__(kSearchThreads) k_cell_seed(CellArgs a) {
   const Probe<Ge> p = probe_cell<Ge>(block * 64 + __ffsll((long long) cells) - 1);
   const float stop = __uint_as_float(ld_relaxed_u32(&d.st->L2));
   float lb, ub;
-  cell_search<Ge, true>(p, a.occ[1 - d.qset], map, stop, &lb, &ub);
+  cell_search<Ge, true>(p, block_box<Ge>(a, g, 1 - d.qset), a.occ[1 - d.qset], map, stop, &lb, &ub,
+                        Ge::kSeedRings);
   if ((threadIdx.x & 31) == 0) {
     raise_level(d.st, lb);
     if (a.seeds_only && lb < INFINITY) start_at_level<Ge>(d, g, lb / kSlack);
@@ -683,6 +758,7 @@ __global__ void __launch_bounds__(256) k_cell_blocks(CellArgs a) {
     return;
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
+    d.st->level = d.st->L2;
     a.seen[blockIdx.y].L2 = d.st->L2;
     a.seen[blockIdx.y].off = d.st->off;  // a query without a cell
   }
@@ -837,6 +913,14 @@ __global__ void __launch_bounds__(256) k_cell_near(CellArgs a) {
 // kManyFar of them a thread per cell, which takes a tenth of the instructions.
 constexpr uint32_t kManyFar = 24576;
 
+// The search gives a direction up when most of the query set's cells are far (one
+// set around the other: hardly any is settled by the cells), or when the rows to
+// look through are too many: 8 million and one per point.  1M + 1M points, given
+// up and searched, and the index alone: 3-D shells of radius 1 and 1.05 1.42, 2.74
+// and 1.36 ms undirected; two cubes apart (64,000 cells by 289 rows) directed 0.47,
+// 0.93 and 0.47 ms; but 10M + 10M with 48,000 such cells 1.3, 0.91 and 1.12.
+constexpr float kMaxRows = 8e6f;
+
 template <class Ge>
 __global__ void __launch_bounds__(kSearchThreads) k_cell_search(CellArgs a) {
   chain_wait();
@@ -845,15 +929,28 @@ __global__ void __launch_bounds__(kSearchThreads) k_cell_search(CellArgs a) {
   const uint32_t n = d.st->n_far;
   const bool many = n > kManyFar;
   if (blockIdx.x * (many ? kSearchThreads : kSearchWarps) >= n) return;
-  const uint32_t* map = search_map<Ge>(a.coarse[1 - d.qset]);
   const CellGrid g = cell_grid<Ge>(a.ord);
+  const BlockBox<Ge> box = block_box<Ge>(a, g, 1 - d.qset);
+  // Rows of blocks per cell, at least.  (st->level: L2 rises from here on.)
+  const float r = 2.0f * ceilf(sqrtf(__uint_as_float(d.st->level)) / (float) Ge::S) + 1.0f;
+  float rows = fminf(r, (float) (box.hi[1] - box.lo[1] + 1));
+  if constexpr (Ge::D == 3) rows *= fminf(r, (float) (box.hi[2] - box.lo[2] + 1));
+  if ((many && n > d.st->n_occ / 2) || (float) n * rows > kMaxRows + (float) (d.nQ + d.nT)) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      d.st->wide = 1u;
+      atomicExch(&d.st->off, 1u);
+      start_at_level<Ge>(d, g, __uint_as_float(d.st->L2));  // for the index that takes over
+    }
+    return;
+  }
+  const uint32_t* map = search_map<Ge>(a.coarse[1 - d.qset]);
   const unsigned long long* occ = a.occ[1 - d.qset];
   float lb, ub;
   if (many) {
     for (uint32_t e = blockIdx.x * kSearchThreads + threadIdx.x; e < n;
          e += gridDim.x * kSearchThreads) {
       const float stop = settle_level(d, g, ld_relaxed_u32(&d.st->L2));
-      cell_search<Ge, false>(probe_cell<Ge>(d.far[e]), occ, map, stop, &lb, &ub);
+      cell_search<Ge, false>(probe_cell<Ge>(d.far[e]), box, occ, map, stop, &lb, &ub);
       d.far_ub[e] = ub;
       if (lb < INFINITY && lb / kSlack > __uint_as_float(ld_relaxed_u32(&d.st->L2)))
         raise_level(d.st, lb);
@@ -864,7 +961,7 @@ __global__ void __launch_bounds__(kSearchThreads) k_cell_search(CellArgs a) {
   for (uint32_t e = blockIdx.x * kSearchWarps + (threadIdx.x >> 5); e < n;
        e += gridDim.x * kSearchWarps) {
     const float stop = settle_level(d, g, ld_relaxed_u32(&d.st->L2));
-    cell_search<Ge, true>(probe_cell<Ge>(d.far[e]), occ, map, stop, &lb, &ub);
+    cell_search<Ge, true>(probe_cell<Ge>(d.far[e]), box, occ, map, stop, &lb, &ub);
     if (lane == 0) {
       d.far_ub[e] = ub;
       raise_level(d.st, lb);
@@ -919,6 +1016,7 @@ __global__ void __launch_bounds__(kSearchThreads) k_cell_mark(CellArgs a) {
   if (blockIdx.x * (many ? kSearchThreads : kMarkChunk) >= n) return;
   const uint32_t* map = search_map<Ge>(a.coarse[1 - d.qset]);
   const CellGrid g = cell_grid<Ge>(a.ord);
+  const BlockBox<Ge> box = block_box<Ge>(a, g, 1 - d.qset);
   const float stop = settle_level(d, g, d.st->L2);
   const unsigned long long* occ = a.occ[1 - d.qset];
   uint32_t* any_q = a.any[d.qset];
@@ -944,8 +1042,9 @@ __global__ void __launch_bounds__(kSearchThreads) k_cell_mark(CellArgs a) {
       mark_query(cell, ub);
       if (!(ub < INFINITY)) continue;
       const float r2 = reach_of(ub);
+      const Probe<Ge> p = probe_cell<Ge>(cell);
       visit_blocks<Ge, false>(
-          probe_cell<Ge>(cell), map, 0, 1, [&]() { return r2; },
+          p, box, Rings<Ge>(p, box), map, 0, 1, [&]() { return r2; },
           [&](uint32_t block, int, int, int) {
             if (__ldcg(d.N + block) == ~0ull) return;
             d.N[block] = ~0ull;
@@ -972,7 +1071,7 @@ __global__ void __launch_bounds__(kSearchThreads) k_cell_mark(CellArgs a) {
       const float r2 = reach_of(s_ub[i]);
       const Probe<Ge> p = probe_cell<Ge>(s_cell[i]);
       visit_blocks<Ge, true>(
-          p, map, threadIdx.x, kSearchThreads, [&]() { return r2; },
+          p, box, Rings<Ge>(p, box), map, threadIdx.x, kSearchThreads, [&]() { return r2; },
           [&](uint32_t block, int bx, int by, int bz) {
             unsigned long long m = occ[block], hit = 0ull;
             while (m) {
@@ -1253,6 +1352,7 @@ hd_status enqueue(Ctx& c, const DirInput* ins, int count, const F64Plan* plan, C
   }
   char* base = (char*) buf;
   a.ord = scalars(c, 0)->mbr_ord;
+  a.swapped = ins[0].dir;
   for (int k = 0; k < 2; ++k) {
     a.occ[k] = (unsigned long long*) (base + o_occ[k]);
     a.half[k] = (unsigned long long*) (base + o_half[k]);
@@ -1442,7 +1542,7 @@ hd_status cells_finish(Ctx& c, int count, const CellsRun& run, CellsLeft* left) 
     CellsLeft& l = left[k];
     l.done = h[k].done != 0;
     memcpy(&l.reach, &h[k].L2, 4);
-    l.reach = std::sqrt(l.reach);
+    l.reach = h[k].wide ? 0.0f : std::sqrt(l.reach);  // a finer grid is no remedy for that
     l.narrowed = !h[k].off && h[k].n_q > 0 && h[k].n_t > 0 && h[k].n_q <= run.cap_q[k] &&
                  h[k].n_t <= run.cap_t[k];
     l.q = run.q[k];

@@ -424,6 +424,9 @@ int cells_finer(uint64_t points, int dims, int level, float reach);
 struct CellDirState {
   uint32_t L2;       // float bits: squared lower bound of h in cell units
   uint32_t off;      // the filter gave up
+  uint32_t level;    // L2 as the seeds left it
+  uint32_t wide;     // it did so because too much is far
+  uint32_t n_occ;    // occupied query cells, about
   uint32_t n_cells;  // cells of open blocks,
   uint32_t n_rim;    // those without a target cell near by (3-D),
   uint32_t n_far;    // and those without one twice as far
