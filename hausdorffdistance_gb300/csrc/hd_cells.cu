@@ -66,7 +66,7 @@ constexpr uint32_t kNoCell = 0xFFFFFFFFu;
 constexpr float kSlack = 1.0001f;
 constexpr int kSearchWarps = 8, kSearchThreads = 32 * kSearchWarps;
 constexpr uint32_t kSeedWarps = 2048;    // sampled words of the coarse map, a cell of each
-constexpr float kMinReach = 2.0f;        // L in cell diagonals, at least
+constexpr float kMinReach = kCellsMinReach;
 constexpr uint64_t kOccSplit = 1000000;  // points from which the cells are set in two launches
 constexpr int kScanTile = 128;           // targets per item of the pair scan
 constexpr uint64_t kScanPairs = 400000000ull;  // pairs per direction the scan takes
@@ -595,7 +595,8 @@ template <class Ge, bool WARP>
 __device__ __forceinline__ void cell_search(const Probe<Ge>& p, const BlockBox<Ge>& box,
                                             const unsigned long long* occ,
                                             const uint32_t* coarse, float stop,
-                                            float* lb2, float* ub2, int most = Ge::NB) {
+                                            float* lb2, float* ub2, int most = Ge::NB,
+                                            uint32_t* cut = nullptr) {
   constexpr int D = Ge::D;
   float lb = INFINITY, ub = INFINITY;
   Rings<Ge> rings(p, box);
@@ -648,6 +649,8 @@ __device__ __forceinline__ void cell_search(const Probe<Ge>& p, const BlockBox<G
       });
   *lb2 = stopped ? INFINITY : lb;
   *ub2 = ub;
+  // (lb still at the bound of the rings left out.)
+  if (cut && !stopped && rings.last == most && lb == rings.gap2(most + 1)) *cut = 1u;
 }
 
 // Raises L from a finished search's lower distance.
@@ -706,7 +709,7 @@ __global__ void __launch_bounds__(kSearchThreads) k_cell_seed(CellArgs a) {
   const float stop = __uint_as_float(ld_relaxed_u32(&d.st->L2));
   float lb, ub;
   cell_search<Ge, true>(p, block_box<Ge>(a, g, 1 - d.qset), a.occ[1 - d.qset], map, stop, &lb, &ub,
-                        Ge::kSeedRings);
+                        Ge::kSeedRings, &d.st->cut);
   if ((threadIdx.x & 31) == 0) {
     raise_level(d.st, lb);
     if (a.seeds_only && lb < INFINITY) start_at_level<Ge>(d, g, lb / kSlack);
@@ -1268,6 +1271,7 @@ __global__ void __launch_bounds__(256) k_cell_solve(CellArgs a) {
   }
 }
 
+constexpr size_t kStateBytes = 4096;  // both directions' states and seed words
 constexpr size_t kStageState = 3072, kStageSeeds = 3584;  // in the pinned staging (4 KB)
 
 uint64_t cap_queries(uint64_t n) { return n / 8 + 8192; }
@@ -1307,7 +1311,7 @@ hd_status enqueue(Ctx& c, const DirInput* ins, int count, const F64Plan* plan, C
   hd_status s;
   // Zeroed words first: state, occupied cells, U, N, maps of marked blocks.
   const size_t fine = (size_t) Ge::kBlocks * 8, coarse = (size_t) Ge::kCoarse * 4;
-  size_t off = 256;
+  size_t off = kStateBytes;
   auto take = [&](size_t bytes) {
     const size_t o = off;
     off += (bytes + 255) / 256 * 256;
@@ -1496,13 +1500,19 @@ hd_status cells_begin(Ctx& c, const DirInput* ins, int count, int level, const F
   return HD_OK;
 }
 
-hd_status cells_seed(Ctx& c, const DirInput* ins, int count, bool* seeded) {
+hd_status cells_seed(Ctx& c, const DirInput* ins, int count) {
   CellArgs a{};
   bool no_room = false;
   const hd_status s =
       ins[0].dims == 3 ? enqueue<Geo<3, 8>>(c, ins, count, nullptr, a, false, true, &no_room)
                        : enqueue<Geo<2, 12>>(c, ins, count, nullptr, a, false, true, &no_room);
-  *seeded = s == HD_OK && !no_room;
+  // Zeroed words behind the states, for the scan's own seeds.
+  uint32_t* words = (uint32_t*) (a.d[0].st + 2);
+  static_assert(2 * sizeof(CellDirState) + 2 * kSeedWords * 4 <= kStateBytes, "state");
+  for (int k = 0; k < count; ++k)
+    c.cell_seeds[ins[k].dir] = s == HD_OK && !no_room
+                                   ? CellSeeds{a.d[k].st, words + k * kSeedWords}
+                                   : CellSeeds{};
   return s;
 }
 

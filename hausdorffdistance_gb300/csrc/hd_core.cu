@@ -63,12 +63,13 @@ hd_status ensure(Ctx& c, BufSlot slot, size_t bytes, void** out) {
       DevBuf& filter = c.bufs[kBufCells];
       if (e != cudaSuccess && slot != kBufCells && !c.cells_live && filter.p) {
         // The cell filter's bitmaps and lists are not needed any more: their
-        // room goes to the index.
+        // room goes to the index (or to the scan, which then takes its own seeds).
         (void) cudaGetLastError();
         if ((e = cudaStreamSynchronize(c.stream)) != cudaSuccess)
           return cuda_fail(c, e, "sync before realloc");
         cudaFree(filter.p);
         filter = DevBuf{};
+        c.cell_seeds[0] = c.cell_seeds[1] = CellSeeds{};
         e = grow(bytes);
       }
       if (e != cudaSuccess) {
@@ -391,10 +392,11 @@ hd_status run_direction(Ctx& c, const DirInput& in, int variant, int* used,
 // Early-break scans of at least this many points (|A| + |B|, times the
 // directions, which share the cost) start from the cell filter's lower bound (30
 // us) instead of 152 seed rows scanned in full (20 us).  Without it and with it,
-// us: directed 3-D planes 20,000 x 15,000 184 and 163, 2-D uniform 19,000 x 18,000
-// 146 and 115, clusters 20,000 x 20,000 125 and 130, 60,000 x 50,000 251 and 188,
-// 1M x 1M 2500 and 1025; undirected clusters 15,000 x 15,000 216 and 185; below,
-// directed clusters 13,000 x 13,000 108 and 132.
+// us, three inputs each: directed 3-D planes 20,000 x 15,000 187 and 163, 2-D
+// uniform 19,000 x 18,000 173 and 143, clusters 18,000 x 18,000 134 and 130, 20,000
+// x 18,000 from the host 139 and 109, 20,000 x 20,000 126 and 126, 25,000 x 25,000
+// 161 and 139, 1M x 1M 2500 and 1020; undirected clusters 15,000 x 15,000 218 and
+// 188; below, directed clusters 13,000 x 13,000 108 and 132.
 constexpr uint64_t kSeedMinPoints = 35000;
 
 hd_status check_status(Ctx& c, const HostScalars& h, int ndir) {
@@ -548,6 +550,7 @@ hd_status hd_solve(hd_ctx* c, const float* A, uint64_t n_a, const float* B,
   c->last_mean[0] = c->last_mean[1] = 0.0;
   c->last_outside[0] = c->last_outside[1] = 0.0;
   c->seeded[0] = c->seeded[1] = false;
+  c->cell_seeds[0] = c->cell_seeds[1] = CellSeeds{};
   c->last_skew[0] = c->last_skew[1] = 0.0;
 
   hd_status s;
@@ -728,9 +731,7 @@ hd_status hd_solve(hd_ctx* c, const float* A, uint64_t n_a, const float* B,
       // The early-break scan starts from the cell filter's lower bound.
       if (used[0] == HD_VARIANT_EB && (n_dims == 2 || n_dims == 3) &&
           (n_a + n_b) * ndir >= kSeedMinPoints) {
-        bool seeded = false;
-        if ((r = cells_seed(*c, ins, ndir, &seeded)) != HD_OK) return r;
-        for (int d = 0; d < ndir; ++d) c->seeded[d] |= seeded;
+        if ((r = cells_seed(*c, ins, ndir)) != HD_OK) return r;
       }
       for (int d = 0; d < ndir; ++d) {
         c->ev_base = 12 * d;

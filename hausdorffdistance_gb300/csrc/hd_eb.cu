@@ -93,25 +93,13 @@ __device__ __forceinline__ void load_a(const float* __restrict__ A, uint64_t i,
   }
 }
 
+// Whether the cell filter's seeds started the running maximum near the final one.
+// Where their bound is but a few diagonals, or ends with the rings that a seed looks
+// through, it may lie far below.
 template <int D>
-__global__ void k_eb_pack(const float* __restrict__ B, uint64_t nB, Perm perm,
-                          typename EbPt<D>::T* out, uint64_t nPad) {
-  chain_wait();
-  for (uint64_t j = blockIdx.x * (uint64_t) blockDim.x + threadIdx.x; j < nPad;
-       j += (uint64_t) gridDim.x * blockDim.x) {
-    if constexpr (D == 2) {
-      float2 v = make_float2(INFINITY, INFINITY);
-      if (j < nB) v = *reinterpret_cast<const float2*>(B + 2 * perm(j));
-      out[j] = v;
-    } else {
-      float4 v = make_float4(INFINITY, INFINITY, INFINITY, 0.0f);
-      if (j < nB) {
-        uint64_t s = perm(j);
-        v = make_float4(B[3 * s], B[3 * s + 1], B[3 * s + 2], 0.0f);
-      }
-      out[j] = v;
-    }
-  }
+__device__ __forceinline__ bool starts_near(const CellDirState* cells) {
+  return cells && !cells->cut &&
+         __uint_as_float(cells->L2) >= kCellsMinReach * kCellsMinReach * D;
 }
 
 template <int D>
@@ -124,15 +112,80 @@ __device__ __forceinline__ float tile_d2(float ax, float ay, float az,
   }
 }
 
+// The packed set.  Behind the cell filter's seeds the same pass scans the scan's
+// own n_seed seeds if it needs them, a thread each over the points that its CTA
+// packs; minima meet as complements in cs.words (zero at first), and the last CTA
+// raises the running maximum.  Planes 1M x 1M directed 8.36 -> 7.55 ms with them
+// (7.58 without the filter), targets in two corners, 100k, 0.73 -> 0.25.  (As a list
+// scan of its own, launched empty where they are not needed, they cost 20,000
+// clusters 5 of 128 us.)
+template <int D>
+__global__ void __launch_bounds__(kEbThreads)
+    k_eb_pack(const float* __restrict__ A, const float* __restrict__ B, uint64_t nB, Perm perm,
+              typename EbPt<D>::T* out, uint64_t nPad, CellSeeds cs, Perm permA, uint32_t n_seed,
+              DevScalars* sc) {
+  chain_wait();
+  __shared__ typename EbPt<D>::T s_pt[kEbThreads];
+  const uint32_t tid = threadIdx.x;
+  const bool scan = cs.state && n_seed && !starts_near<D>(cs.state);
+  float ax = 0.f, ay = 0.f, az = 0.f, m = FLT_MAX;
+  uint32_t ia = 0;
+  if (scan && tid < n_seed) {
+    ia = (uint32_t) permA(tid);
+    load_a<D>(A, ia, ax, ay, az);
+  }
+  // (nPad is a multiple of the CTA's threads.)
+  for (uint64_t j = blockIdx.x * (uint64_t) blockDim.x + tid; j < nPad;
+       j += (uint64_t) gridDim.x * blockDim.x) {
+    typename EbPt<D>::T v;
+    if constexpr (D == 2) {
+      v = make_float2(INFINITY, INFINITY);
+      if (j < nB) v = *reinterpret_cast<const float2*>(B + 2 * perm(j));
+    } else {
+      v = make_float4(INFINITY, INFINITY, INFINITY, 0.0f);
+      if (j < nB) {
+        uint64_t s = perm(j);
+        v = make_float4(B[3 * s], B[3 * s + 1], B[3 * s + 2], 0.0f);
+      }
+    }
+    out[j] = v;
+    if (!scan) continue;
+    __syncthreads();
+    s_pt[tid] = v;
+    __syncthreads();
+    if (tid < n_seed) {
+#pragma unroll 8
+      for (int k = 0; k < kEbThreads; ++k) {
+        float z = 0.f;
+        if constexpr (D == 3) z = s_pt[k].z;
+        m = fminf(m, tile_d2<D>(ax, ay, az, s_pt[k].x, s_pt[k].y, z));
+      }
+    }
+    if (tid == 0) atomicAdd(&sc->pairs, (unsigned long long) n_seed * kEbThreads);
+  }
+  if (!scan) return;
+  if (tid < n_seed) atomicMax(cs.words + tid, ~__float_as_uint(m));
+  __threadfence();
+  __shared__ bool s_last;
+  __syncthreads();
+  if (tid == 0) s_last = atomicAdd(cs.words + kSeedWords - 1, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!s_last || tid >= n_seed) return;
+  __threadfence();
+  atomicMax(&sc->max_key, pack_max(__uint_as_float(~__ldcg(cs.words + tid)), ia));
+}
+
 // S: A points carried per thread (4 for large sets; 2 or 1 when the set is
 // too small to give every SM a full complement of 4-slot CTAs).
 template <int D, int S = kEbSlots>
 __global__ void __launch_bounds__(kEbThreads)
     k_eb_main(const float* __restrict__ A, Perm permA, uint64_t a_begin,
               uint64_t a_end, const typename EbPt<D>::T* Bp,
-              uint32_t nTiles, uint32_t capTiles, DevScalars* sc,
-              HeavyEntry* heavy, uint32_t heavy_cap) {
+              uint32_t nTiles, uint32_t capFar, uint32_t capNear, const CellDirState* cells,
+              DevScalars* sc, HeavyEntry* heavy, uint32_t heavy_cap) {
   chain_wait();
+  // (Not from a word of sc, whose line the visit counter keeps busy: 8 us.)
+  const uint32_t capTiles = starts_near<D>(cells) ? capNear : capFar;
   using PT = typename EbPt<D>::T;
   constexpr uint32_t kTileBytes = kEbTile * sizeof(PT);
   __shared__ __align__(128) PT tile[2][kEbTile];
@@ -628,22 +681,29 @@ hd_status run_eb_dim(Ctx& c, const DirInput& in) {
   Perm pB{in.nB, pick_multiplier(in.nB, seed + 1), (seed * 7919u) % in.nB};
   Perm pA{in.nA, pick_multiplier(in.nA, seed + 2), (seed * 104729u) % in.nA};
 
-  {
-    int grid = (int) std::min<uint64_t>((nPad + 255) / 256, (uint64_t) c.num_sms * 16);
-    launch_next(c.stream, true, k_eb_pack<D>, grid, 256, in.B, in.nB, pB, (PT*) pb, nPad);
-    if ((s = after_launch(c, "eb_pack")) != HD_OK) return s;
-  }
-  mark(c, 1);
-  mark(c, 2);
   // Seeds: the first visited A points, scanned in full (the running maximum
   // is still zero) by the tile-wise list pass.  Their list entries sit at the
   // end of the deferred-point list, which the main pass fills from the start.
   // An AUTO solve whose selector already scanned seeds and a sample of A
-  // against B starts from the maximum they set instead.
+  // against B starts from the maximum they set instead; behind the cell filter's
+  // seeds the device decides (k_eb_pack), and the main pass visits every point.
+  const CellSeeds cells = c.cell_seeds[in.dir];
   const uint32_t n_seed =
-      c.seeded[in.dir] ? 0u : (uint32_t) std::min<uint64_t>(in.nA, (uint64_t) c.num_sms);
-  HeavyEntry* seeds = (HeavyEntry*) ph + (in.nA - n_seed);
-  if (n_seed > 0) {
+      c.seeded[in.dir]
+          ? 0u
+          : (uint32_t) std::min<uint64_t>(in.nA, (uint64_t) std::min(c.num_sms, kEbThreads));
+  static_assert(kSeedWords > kEbThreads, "seed words");
+  const uint64_t first = cells.state ? 0 : n_seed;  // of the main pass
+  {
+    int grid = (int) std::min<uint64_t>((nPad + 255) / 256, (uint64_t) c.num_sms * 16);
+    launch_next(c.stream, true, k_eb_pack<D>, grid, kEbThreads, in.A, in.B, in.nB, pB, (PT*) pb, nPad,
+                cells, pA, n_seed, sc);
+    if ((s = after_launch(c, "eb_pack")) != HD_OK) return s;
+  }
+  mark(c, 1);
+  mark(c, 2);
+  if (n_seed > 0 && !cells.state) {
+    HeavyEntry* seeds = (HeavyEntry*) ph + (in.nA - n_seed);
     k_eb_seed_list<<<(n_seed + 255) / 256, 256, 0, c.stream>>>(pA, n_seed, nTiles, seeds);
     if ((s = after_launch(c, "eb_seed_list")) != HD_OK) return s;
     cudaError_t e = eb_list_pass<D>(c.stream, c.num_sms, in.A, (const PT*) pb, nTiles, seeds,
@@ -652,14 +712,14 @@ hd_status run_eb_dim(Ctx& c, const DirInput& in) {
     if (e != cudaSuccess) return cuda_fail(c, e, "eb_seed");
   }
   mark(c, 3);
-  if (in.nA > n_seed) {
+  if (in.nA > first) {
     // Slots per thread: the most (4, 2, 1) that still fill every resident CTA
     // of a full grid, so that a small set spreads over all SMs instead of
     // leaving most of them idle (every slot of a thread is computed).
     constexpr decltype(&k_eb_main<D, 4>) fns[3] = {k_eb_main<D, 4>, k_eb_main<D, 2>,
                                                    k_eb_main<D, 1>};
     const int slots[3] = {4, 2, 1};
-    const uint64_t rest = in.nA - n_seed;
+    const uint64_t rest = in.nA - first;
     int pick = 2, occ = 1;
     for (int k = 0; k < 3; ++k) {
       int o = 0;
@@ -677,19 +737,20 @@ hd_status run_eb_dim(Ctx& c, const DirInput& in) {
     // Pairs a point scans before it is paused (deferred): an option, else
     // clamp(|B| / div, min, max) from the tuning table.  Pausing is not only
     // a tail guard: a paused point resumes under a higher running maximum.
-    uint64_t cap = c.opt.eb_cap_pairs;
-    if (cap == 0) {
-      // A 3-D scan that starts near its final maximum settles most points in a
-      // tile or two; what is left holds whole CTAs until the cap (1M clusters:
-      // 1.19 ms with the table's cap of 4,096 pairs, 1.03 with half; 2-D points,
-      // which need thousands of pairs, only move from one kernel to the other).
-      const uint64_t half = D == 3 && c.seeded[in.dir] ? 2 : 1;
-      cap = std::min<uint64_t>(std::max<uint64_t>(in.nB / (tuning().eb_cap_div * half),
-                                                  tuning().eb_cap_min / half),
-                               tuning().eb_cap_max);
-    }
-    const uint32_t capTiles = (uint32_t) std::max<uint64_t>(1, cap / kEbTile);
-    const uint32_t heavy_cap = (uint32_t) (in.nA - n_seed);
+    // A 3-D scan that starts near its final maximum settles most points in a
+    // tile or two; what is left holds whole CTAs until the cap (1M clusters:
+    // 1.19 ms with the table's cap of 4,096 pairs, 1.03 with half; 2-D points,
+    // which need thousands of pairs, only move from one kernel to the other).
+    auto tiles = [&](uint64_t half) {
+      uint64_t cap = c.opt.eb_cap_pairs;
+      if (cap == 0)
+        cap = std::min<uint64_t>(std::max<uint64_t>(in.nB / (tuning().eb_cap_div * half),
+                                                    tuning().eb_cap_min / half),
+                                 tuning().eb_cap_max);
+      return (uint32_t) std::max<uint64_t>(1, cap / kEbTile);
+    };
+    const uint32_t cap_far = tiles(1), cap_near = tiles(D == 3 ? 2 : 1);
+    const uint32_t heavy_cap = (uint32_t) (in.nA - first);
     // Checkpoints: the main pass runs in parts; after each part the points
     // it deferred are finished before the next part starts.  Deferred points
     // include the outliers, whose distances are the ones that lift the
@@ -699,16 +760,16 @@ hd_status run_eb_dim(Ctx& c, const DirInput& in) {
     const uint64_t wave = (uint64_t) grid * per_cta;
     uint64_t ends[kEbMaxParts];
     int parts = 0;
-    uint64_t last = n_seed;
+    uint64_t last = first;
     for (uint64_t div : kEbCheckDiv) {
-      const uint64_t e = n_seed + rest / div;
+      const uint64_t e = first + rest / div;
       if (e >= last + wave && in.nA >= e + wave) {
         ends[parts++] = e;
         last = e;
       }
     }
     ends[parts++] = in.nA;
-    uint64_t a_begin = n_seed;
+    uint64_t a_begin = first;
     for (int part = 0; part < parts; ++part) {
       uint64_t a_end = ends[part];
       if (part > 0) {
@@ -718,7 +779,8 @@ hd_status run_eb_dim(Ctx& c, const DirInput& in) {
         if ((s = after_launch(c, "eb_mark")) != HD_OK) return s;
       }
       launch_next(c.stream, true, fns[pick], grid, kEbThreads, in.A, pA, a_begin, a_end,
-                  (const PT*) pb, nTiles, capTiles, sc, (HeavyEntry*) ph, heavy_cap);
+                  (const PT*) pb, nTiles, cap_far, cap_near, cells.state, sc,
+                  (HeavyEntry*) ph, heavy_cap);
       if ((s = after_launch(c, "eb_main")) != HD_OK) return s;
       if (part == parts - 1) mark(c, 4);
       launch_next(c.stream, true, k_eb_heavy<D>, c.num_sms * 4, kEbThreads, in.A, (const PT*) pb,
@@ -801,7 +863,7 @@ cudaError_t noalloc_direction(cudaStream_t st, int num_sms, const float* A, uint
   Perm pB{nB, pick_multiplier(nB, 1), 0};
   Perm pA{nA, pick_multiplier(nA, 2), 0};
   int grid = (int) std::min<uint64_t>((nPad + 255) / 256, (uint64_t) num_sms * 16);
-  k_eb_pack<D><<<grid, 256, 0, st>>>(B, nB, pB, pb, nPad);
+  k_eb_pack<D><<<grid, kEbThreads, 0, st>>>(A, B, nB, pB, pb, nPad, CellSeeds{}, pA, 0u, sc);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   const uint32_t n_seed = (uint32_t) std::min<uint64_t>(nA, (uint64_t) num_sms);
@@ -837,8 +899,9 @@ cudaError_t noalloc_direction(cudaStream_t st, int num_sms, const float* A, uint
     const PT* b_ptr = pb;
     uint32_t heavy_cap = (uint32_t) (nA - n_seed);
     uint64_t a_begin = n_seed, a_end = nA;
-    void* args[] = {&a_ptr, &pA, &a_begin, &a_end, &b_ptr, (void*) &nTiles, &capTiles, &sc,
-                    &heavy, &heavy_cap};
+    const CellDirState* no_cells = nullptr;
+    void* args[] = {&a_ptr, &pA, &a_begin, &a_end, &b_ptr, (void*) &nTiles, &capTiles, &capTiles,
+                    &no_cells, &sc, &heavy, &heavy_cap};
     if ((e = cudaLaunchKernel(fns[pick], dim3(g), dim3(kEbThreads), args, 0, st)) != cudaSuccess)
       return e;
     k_eb_heavy<D><<<num_sms * 4, kEbThreads, 0, st>>>(A, pb, nTiles, sc, heavy, &sc->heavy_count,

@@ -215,6 +215,15 @@ struct SortedSet {
   uint32_t mask = sorted_mask(kSortLowBitsSplit);  // the sorted code bits
 };
 
+// What the cell filter's seeds left of a direction, on the device (null: they did
+// not run), and kSeedWords zeroed words.
+struct CellDirState;
+constexpr int kSeedWords = 320;
+struct CellSeeds {
+  const CellDirState* state = nullptr;
+  uint32_t* words = nullptr;
+};
+
 struct Ctx {
   int device = 0;
   int num_sms = 0;
@@ -284,6 +293,9 @@ struct Ctx {
   // The selector's sampled scans already raised this direction's running
   // maximum (the EB variant then skips its own seed pass).
   bool seeded[2] = {false, false};
+  // The cell filter's seeds did: the EB variant looks there whether it needs its
+  // own.
+  CellSeeds cell_seeds[2];
   double last_skew[2] = {0.0, 0.0};
 };
 
@@ -426,6 +438,7 @@ struct CellDirState {
   uint32_t off;      // the filter gave up
   uint32_t level;    // L2 as the seeds left it
   uint32_t wide;     // it did so because too much is far
+  uint32_t cut;      // a seed met nothing in the rings it looks through
   uint32_t n_occ;    // occupied query cells, about
   uint32_t n_cells;  // cells of open blocks,
   uint32_t n_rim;    // those without a target cell near by (3-D),
@@ -448,9 +461,11 @@ struct CellsRun {
 };
 hd_status cells_begin(Ctx& c, const DirInput* ins, int count, int level, const F64Plan* plan,
                       bool boxes_known, CellsRun* run);
-// The filter's seeds alone: starts the directions' running maxima at their L
-// (seeded: false when there was no room).  Takes no read-back.
-hd_status cells_seed(Ctx& c, const DirInput* ins, int count, bool* seeded);
+// The filter's seeds alone: starts the directions' running maxima at their L and
+// leaves c.cell_seeds (none when there was no room).  Takes no read-back.
+hd_status cells_seed(Ctx& c, const DirInput* ins, int count);
+// The filter settles nothing below an L of this many cell diagonals.
+constexpr float kCellsMinReach = 2.0f;
 // Waits for the filter's seeds alone: off[k] where it will give direction k up
 // (reach[k]: its L in cells), so that the index can be enqueued behind it.  False
 // when the filter did not run: there are no seeds to wait behind.
