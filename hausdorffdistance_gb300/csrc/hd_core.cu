@@ -399,6 +399,17 @@ hd_status run_direction(Ctx& c, const DirInput& in, int variant, int* used,
 // 188; below, directed clusters 13,000 x 13,000 108 and 132.
 constexpr uint64_t kSeedMinPoints = 35000;
 
+// A is sorted while B is copied, before it is known that the sort is of use, when
+// it ends with the copy: about 100 us and 35 ps a point, against 19 ps a float over
+// the host link.  Sets that the filter gives up, us without the early sort, with it,
+// and before there was a filter: 3-D planes 5M + 5M 1745, 1600 and 1638, 15M + 15M
+// 4290, 3615 and 3706, jittered copies 10M + 10M 7366, 7000 and 6700.  Where the sort
+// outlasts the copy, sets that the filter settles pay for it: clusters 5M + 3.2M 754
+// and 862, 2-D with outliers 4M + 4M 846 and 860 (10M clusters 1495 and 1492).
+bool sort_first(uint64_t nA, uint64_t nB, int dims) {
+  return 19e-6 * (double) nB * dims >= 100.0 + 35e-6 * (double) nA;
+}
+
 hd_status check_status(Ctx& c, const HostScalars& h, int ndir) {
   for (int d = 0; d < ndir; ++d) {
     uint32_t st = h.s[d].status;
@@ -542,7 +553,7 @@ hd_status hd_solve(hd_ctx* c, const float* A, uint64_t n_a, const float* B,
   memset(out, 0, sizeof(*out));
   out->hd_ba = -1.0;
   c->timing = (flags & HD_TIMING) != 0;
-  c->sorted_valid = false;
+  c->sorted_valid = c->first_sorted = c->first_running = false;
   c->boxes_known = false;
   c->cells_live = false;
   c->ev_base = 0;
@@ -554,6 +565,13 @@ hd_status hd_solve(hd_ctx* c, const float* A, uint64_t n_a, const float* B,
   c->last_skew[0] = c->last_skew[1] = 0.0;
 
   hd_status s;
+  struct Join {  // whatever ends the call, its stream is behind an early sort
+    Ctx& c;
+    ~Join() {
+      join_first(c);
+      c.first_sorted = false;
+    }
+  } join{*c};
   const float* dA = A;
   const float* dB = B;
   mark_abs(*c, 24);  // start of the whole call (copies included)
@@ -566,18 +584,29 @@ hd_status hd_solve(hd_ctx* c, const float* A, uint64_t n_a, const float* B,
     small = variant == HD_VARIANT_AUTO && select_variant_by_size(*c, n_a, n_b, n_dims, &va) &&
             va == HD_VARIANT_EB && select_variant_by_size(*c, n_b, n_a, n_dims, &vb);
   }
+  // The cell filter runs before the indexes (not before an early-break scan,
+  // which eb_only_threshold may ask for).  It does not wait for the selector:
+  // its kernels follow the sample's, and the host evaluates the sample while
+  // they run.
+  bool cells = !small && cells_apply(*c, n_a, n_b, n_dims) &&
+               (variant == HD_VARIANT_LBVH ||
+                (variant == HD_VARIANT_AUTO && c->opt.eb_only_threshold == 0));
   if (!small && (s = init_scalars(*c)) != HD_OK) return s;
   if (!(flags & HD_DEVICE_PTRS)) {
     // An undirected solve known (from the sizes alone) to take the LBVH in
-    // both directions sorts A while B is still being copied.
+    // both directions sorts A while B is still being copied; one that the cell
+    // filter takes first as well, in case the index follows.
     int v0 = variant, v1 = variant;
     bool known = variant != HD_VARIANT_AUTO;
     if (!known)
       known = select_variant_by_size(*c, n_a, n_b, n_dims, &v0) &&
               select_variant_by_size(*c, n_b, n_a, n_dims, &v1);
-    if (undirected && known && v0 == HD_VARIANT_LBVH && v1 == HD_VARIANT_LBVH &&
-        n_a + n_b >= kSplitMinPoints && !cells_apply(*c, n_a, n_b, n_dims)) {
+    const bool index = undirected && known && v0 == HD_VARIANT_LBVH && v1 == HD_VARIANT_LBVH &&
+                       n_a + n_b >= kSplitMinPoints;
+    if (index && !cells) {
       if ((s = spatial_upload_sort(*c, A, n_a, B, n_b, n_dims, &dA, &dB)) != HD_OK) return s;
+    } else if (index && sort_first(n_a, n_b, n_dims)) {
+      if ((s = spatial_upload_first(*c, A, n_a, B, n_b, n_dims, &dA, &dB)) != HD_OK) return s;
     } else {
       if ((s = copy_in(*c, A, n_a, n_dims, kBufA, &dA)) != HD_OK) return s;
       if ((s = copy_in(*c, B, n_b, n_dims, kBufB, &dB)) != HD_OK) return s;
@@ -593,13 +622,6 @@ hd_status hd_solve(hd_ctx* c, const float* A, uint64_t n_a, const float* B,
                       d == 0 ? n_b : n_a, n_dims, d, count, variant == HD_VARIANT_AUTO};
     used[d] = variant;
   }
-  // The cell filter runs before the indexes (not before an early-break scan,
-  // which eb_only_threshold may ask for).  It does not wait for the selector:
-  // its kernels follow the sample's, and the host evaluates the sample while
-  // they run.
-  bool cells = cells_apply(*c, n_a, n_b, n_dims) &&
-               (variant == HD_VARIANT_LBVH ||
-                (variant == HD_VARIANT_AUTO && c->opt.eb_only_threshold == 0));
   bool have_result = false;  // the scalars are already in the pinned staging
   CellsRun cells_state;
   const int level = cells_level(n_a + n_b, n_dims);
@@ -611,7 +633,6 @@ hd_status hd_solve(hd_ctx* c, const float* A, uint64_t n_a, const float* B,
   };
   if (small) {
     used[0] = used[1] = HD_VARIANT_EB;
-    cells = false;
   } else if (variant == HD_VARIANT_AUTO) {
     Selection sel;
     c->ev_base = 0;
@@ -684,6 +705,7 @@ hd_status hd_solve(hd_ctx* c, const float* A, uint64_t n_a, const float* B,
         if (e != cudaSuccess) return cuda_fail(*c, e, "copy result");
       }
       if ((r = cells_finish(*c, ndir, cells_state, left)) != HD_OK) return r;
+      if ((r = join_first(*c)) != HD_OK) return r;
       have_result = cells_state.ran;
       for (int d = 0; d < ndir; ++d) left[d].done |= indexed[d];
       for (int d = 0; d < ndir; ++d)

@@ -282,6 +282,9 @@ struct Ctx {
   // are shared by both directions of an undirected solve.
   SortedSet sorted[2];
   bool sorted_valid = false;
+  // Set 0 alone is sorted, or being so on index_side (spatial_upload_first), and
+  // whether the call's stream has yet to wait for that.
+  bool first_sorted = false, first_running = false;
   bool boxes_known = false;  // DevScalars[0].mbr_ord holds the call's boxes
   // Sampler statistic of the last AUTO decision per direction (p80 of the
   // sampled early-break iteration counts; 0 when no sample was drawn).
@@ -489,7 +492,7 @@ hd_status index_beside(Ctx& c, F index) {
   s = index();
   c.stream = main;
   if (s != HD_OK) {
-    c.sorted_valid = false;
+    c.sorted_valid = c.first_sorted = false;
     cudaStreamSynchronize(c.index_side);
     if (c.batch_side) cudaStreamSynchronize(c.batch_side);
     return s;
@@ -538,6 +541,13 @@ hd_status spatial_prepare(Ctx& c, const DirInput& in, const SortedSet** q,
 // then sorts B (sets c.sorted, c.sorted_valid); *dA, *dB = device copies.
 hd_status spatial_upload_sort(Ctx& c, const float* hA, uint64_t nA, const float* hB, uint64_t nB,
                               int dims, const float** dA, const float** dB);
+// Host inputs that the cell filter takes first: copies A and B, and sorts A on the
+// index's stream while B arrives, for an index that may follow (plain copies when
+// there is no room to sort in).
+hd_status spatial_upload_first(Ctx& c, const float* hA, uint64_t nA, const float* hB, uint64_t nB,
+                               int dims, const float** dA, const float** dB);
+// The call's stream waits for that sort.
+hd_status join_first(Ctx& c);
 // Boxes of the call's two sets, into DevScalars[0].mbr_ord.
 hd_status spatial_boxes(Ctx& c, const DirInput& in);
 // Morton-sorts listed points in the common frame of the call's boxes: out[2k]

@@ -415,6 +415,10 @@ static hd_status spatial_sort(Ctx& c, const float* A, uint64_t nA, const float* 
   hd_status s;
   SortScratch x;
   if ((s = sort_scratch(c, nA, nB, false, &x)) != HD_OK) return s;
+  if (c.first_sorted) {  // A was, while B was copied
+    c.first_sorted = false;
+    return sort_set(c, 1, B, nB, dims, x, c.stream, sb);
+  }
   if ((s = ensure_side(c)) != HD_OK) return s;
   cudaError_t e;
   if ((e = cudaEventRecord(c.batch_fork, c.stream)) != cudaSuccess ||
@@ -460,6 +464,44 @@ hd_status spatial_upload_sort(Ctx& c, const float* hA, uint64_t nA, const float*
   *dA = (const float*) pa;
   *dB = (const float*) pb;
   return HD_OK;
+}
+
+hd_status spatial_upload_first(Ctx& c, const float* hA, uint64_t nA, const float* hB, uint64_t nB,
+                               int dims, const float** dA, const float** dB) {
+  hd_status s;
+  void *pa, *pb;
+  const size_t bytes_a = (size_t) nA * dims * sizeof(float), bytes_b = (size_t) nB * dims * sizeof(float);
+  if ((s = ensure(c, kBufA, bytes_a, &pa)) != HD_OK) return s;
+  if ((s = ensure(c, kBufB, bytes_b, &pb)) != HD_OK) return s;
+  SortScratch x;
+  s = sort_scratch(c, nA, nB, false, &x);
+  const bool room = s == HD_OK;
+  if (s == HD_ERR_OOM) c.last_error.clear();
+  else if (s != HD_OK) return s;
+  if ((s = ensure_side(c)) != HD_OK || (s = ensure_index_side(c)) != HD_OK) return s;
+  cudaError_t e;
+  if ((e = cudaMemcpyAsync(pa, hA, bytes_a, cudaMemcpyHostToDevice, c.stream)) != cudaSuccess ||
+      (e = cudaEventRecord(c.batch_fork, c.stream)) != cudaSuccess ||
+      (e = cudaMemcpyAsync(pb, hB, bytes_b, cudaMemcpyHostToDevice, c.stream)) != cudaSuccess)
+    return cuda_fail(c, e, "copy inputs to device");
+  *dA = (const float*) pa;
+  *dB = (const float*) pb;
+  if (!room) return HD_OK;
+  if ((e = cudaStreamWaitEvent(c.index_side, c.batch_fork, 0)) != cudaSuccess)
+    return cuda_fail(c, e, "fork");
+  c.first_running = true;
+  s = sort_set(c, 0, *dA, nA, dims, x, c.index_side, &c.sorted[0]);
+  c.first_sorted = s == HD_OK;
+  if ((e = cudaEventRecord(c.index_join, c.index_side)) != cudaSuccess)
+    return cuda_fail(c, e, "index stream");
+  return s;
+}
+
+hd_status join_first(Ctx& c) {
+  if (!c.first_running) return HD_OK;
+  c.first_running = false;
+  const cudaError_t e = cudaStreamWaitEvent(c.stream, c.index_join, 0);
+  return e == cudaSuccess ? HD_OK : cuda_fail(c, e, "index stream");
 }
 
 hd_status spatial_boxes(Ctx& c, const DirInput& in) {
@@ -530,6 +572,7 @@ __global__ void k_gather_left(LeftLists l, const uint32_t* __restrict__ order,
 
 hd_status spatial_sort_left(Ctx& c, const CellsLeft* left, int count, int dims, SortedSet* out) {
   hd_status s;
+  c.first_sorted = false;  // its codes and leaf boxes are written over
   uint32_t L = c.opt.leaf_size ? std::min<uint32_t>(c.opt.leaf_size, 32) : 16;
   while (L & (L - 1)) L &= L - 1;
   LeftLists l{};
