@@ -1278,14 +1278,18 @@ uint64_t cap_queries(uint64_t n) { return n / 8 + 8192; }
 uint64_t cap_targets(uint64_t n) { return n / 4 + 8192; }
 constexpr uint64_t kCapCells = 1ull << 23;
 
-// Grids: 2^8, 2^9, 2^10 cells per axis in 3-D, 2^12, 2^13, 2^14 in 2-D.  2-D sets
-// from kFine2Points points start at the second, their answer being a few cells of
-// the first; a direction whose L turned out too few cells is tried again on
-// the grid where it is kFinerReach diagonals, if the sets are large enough for
-// that grid's maps (a set's cells are 16 and 128 MB in 3-D, 8 and 32 in 2-D).
-constexpr int kLevels = 3;
+// Grids by level: 2^8 cells per axis in 3-D; 2^12 in 2-D, and 2^13 from
+// kFine2Points points, whose answer is a few cells of the first.  A 3-D direction
+// that is too few cells there is tried again on 2^10 (maps of 128 MB a set) if its L
+// is kFinerReach diagonals there, from kFinestPoints points.  The index alone and
+// that grid, us: directed planes 16M + 16M 2495 and 2487, 14M + 16M 2375 and 2460, 18M
+// + 18M 2771 and 2590, undirected 21M + 21M 3310 and 2950.  With A sorted beside B's
+// copy the index is ahead for longer: 21M + 21M 4770 and 5290, 30M + 30M 6700 and
+// 6660.  (In 2-D a grid of 2^14 never paid: uniform 21M + 21M 6095 without it, 6990
+// with it, whose lists ran over.)
+constexpr int kFinest = 2;
 constexpr uint64_t kFine2Points = 1500000;
-constexpr uint64_t kLevelPoints[kLevels] = {0, ~0ull, 40000000};
+constexpr uint64_t kFinestPoints = 33000000, kFinestPointsSorted = 60000000;
 constexpr float kFinerReach = 2.5f;
 
 }  // namespace
@@ -1464,12 +1468,10 @@ hd_status enqueue(Ctx& c, const DirInput* ins, int count, const F64Plan* plan, C
 
 int cells_level(uint64_t points, int dims) { return dims == 2 && points >= kFine2Points ? 1 : 0; }
 
-int cells_finer(uint64_t points, int dims, int level, float reach) {
-  for (int up = level + 1; up < kLevels; ++up)
-    if (points >= kLevelPoints[up] &&
-        reach * (float) (1 << (up - level)) >= kFinerReach * (dims == 3 ? 1.732f : 1.414f))
-      return up;
-  return -1;
+int cells_finer(uint64_t points, int dims, int level, float reach, bool sorted) {
+  const bool take = dims == 3 && points >= (sorted ? kFinestPointsSorted : kFinestPoints) &&
+                    reach * (float) (1 << (kFinest - level)) >= kFinerReach * 1.732f;
+  return take ? kFinest : -1;
 }
 
 hd_status cells_begin(Ctx& c, const DirInput* ins, int count, int level, const F64Plan* plan,
@@ -1482,9 +1484,9 @@ hd_status cells_begin(Ctx& c, const DirInput* ins, int count, int level, const F
   };
   hd_status s;
   if (ins[0].dims == 3)
-    s = level == 0 ? go(Geo<3, 8>{}) : level == 1 ? go(Geo<3, 9>{}) : go(Geo<3, 10>{});
+    s = level == 0 ? go(Geo<3, 8>{}) : go(Geo<3, 10>{});
   else
-    s = level == 0 ? go(Geo<2, 12>{}) : level == 1 ? go(Geo<2, 13>{}) : go(Geo<2, 14>{});
+    s = level == 0 ? go(Geo<2, 12>{}) : go(Geo<2, 13>{});
   if (s != HD_OK || no_room) return s;
   run->ran = true;
   run->wrote = plan == nullptr;

@@ -747,7 +747,7 @@ hd_status hd_solve(hd_ctx* c, const float* A, uint64_t n_a, const float* B,
       float reach[2];
       if ((r = cells_hopeless(*c, ndir, n_dims, cells_state, off, reach)) != HD_OK) return r;
       for (int d = 0; d < ndir; ++d)
-        indexed[d] = off[d] && cells_finer(n_a + n_b, n_dims, level, reach[d]) < 0;
+        indexed[d] = off[d] && cells_finer(n_a + n_b, n_dims, level, reach[d], c->first_sorted) < 0;
       auto index = [&]() -> hd_status {
         if (indexed[0] && indexed[1] && fused) return run_lbvh_pair(*c, ins[0], ins[1]);
         for (int d = 0; d < ndir; ++d)
@@ -792,7 +792,7 @@ hd_status hd_solve(hd_ctx* c, const float* A, uint64_t n_a, const float* B,
       n = 0;
       for (int d = 0; d < ndir; ++d) {
         if (left[d].done || left[d].narrowed) continue;
-        const int finer = cells_finer(n_a + n_b, n_dims, level, left[d].reach);
+        const int finer = cells_finer(n_a + n_b, n_dims, level, left[d].reach, c->first_sorted);
         CellsLeft fine;
         if (finer >= 0) {
           CellsRun again;

@@ -429,9 +429,10 @@ struct CellsLeft {
 constexpr uint64_t kCellsMinPoints = 40000;
 bool cells_apply(const Ctx& c, uint64_t nA, uint64_t nB, int dims);
 // The grid (level) to start on, and the one to try again on when the filter
-// neither finished nor narrowed a direction (its L: `reach` cells); -1: none.
+// neither finished nor narrowed a direction (its L: `reach` cells; sorted: a set is
+// sorted already); -1: none.
 int cells_level(uint64_t points, int dims);
-int cells_finer(uint64_t points, int dims, int level, float reach);
+int cells_finer(uint64_t points, int dims, int level, float reach, bool sorted);
 // Filters `count` directions: the call's (ins[k].dir == k), or one of them.  With a plan, queries are
 // settled by the FP64 listing pass's level, and the pair scan leaves the open
 // queries' FP32 minima; no direction is finished here.
