@@ -279,10 +279,9 @@ __global__ void k_f64_round(const double* __restrict__ X, uint64_t total, float*
 
 // The same with two points per step by 16-byte loads, for sets of 2-D or 3-D
 // points that begin on a 16-byte boundary.  HBM bound (24 or 36 bytes a point,
-// 0.75 of the copy rate at 10M); half as many steps: the call on 300k x 400k
-// points 216 -> 208 us, 2M x 3M in 2-D 433 -> 427, 4M x 5M 372 -> 370, but 10M x 10M
-// 505 -> 510: so not for sets of kRoundPairsBelow points and more.
-constexpr uint64_t kRoundPairsBelow = 7000000;
+// 0.75 of the copy rate at 10M); half as many steps.  The call a point and a pair
+// at a time, us: 3-D 300k x 400k 239 and 230, 2M + 2M 311 and 306, 10M + 10M 506 and
+// 507, 13M + 13M 583 and 577; 2-D 2M + 3M 357 and 350, 10M + 10M 2863 and 2841.
 template <int D>
 __global__ void k_f64_round_pairs(const double* __restrict__ X, uint64_t total,
                                   float* __restrict__ Xf, RoundStats* st,
@@ -1009,7 +1008,7 @@ hd_status hd_solve_f64(hd_ctx* c, const double* A, uint64_t n_a, const double* B
         (int) std::max<uint64_t>(1, std::min<uint64_t>((total + 255) / 256, (uint64_t) c->num_sms * 8));
     uint32_t* ord = &scalars(*c, 0)->mbr_ord[k][0][0];
     auto kern = n_dims == 2 ? k_f64_round<2> : n_dims == 3 ? k_f64_round<3> : k_f64_round<0>;
-    if (spatial_dims && nn[k] < kRoundPairsBelow && ((uintptr_t) d64[k] & 15) == 0)
+    if (spatial_dims && ((uintptr_t) d64[k] & 15) == 0)
       kern = n_dims == 2 ? k_f64_round_pairs<2> : k_f64_round_pairs<3>;
     kern<<<grid, 256, 0, c->stream>>>(d64[k], total, (float*) p, &aux->round[k], ord);
     if ((s = after_launch(*c, "f64_round")) != HD_OK) return s;
