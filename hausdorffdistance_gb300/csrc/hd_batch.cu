@@ -846,7 +846,7 @@ __device__ __forceinline__ void cta_direction(const BatchArgs& a, uint32_t p, in
   for (int it = 0; it < kBestFirst; ++it) {
     if (it > 0) {
       top = TopRow{thr, 0u};
-#pragma unroll 4
+#pragma unroll 8
       for (uint32_t row = tid; row < nx; row += kBatchThreads) top.add(wb[row], row);
     }
     const unsigned long long cand = block_max_u64(top.key(thr), s_red);
@@ -965,31 +965,34 @@ template <int D>
 __global__ void __launch_bounds__(kBatchThreads) k_batch_small(BatchArgs a) {
   const int lane = threadIdx.x & 31;
   // First the CTA-path directions, one per block: they sit among the first
-  // n_big ranks of the plan, largest first.
+  // n_big ranks of the plan, largest first.  A block's (and below a warp's) first
+  // place in the queue is its own, so that a few long directions go to as many SMs:
+  // taken as they come, 200 problems of 4,096 rows went to the SMs that started
+  // first (incoherent 3-D sets, undirected, 10.0 ms, with own places 5.0; 8 walks of
+  // 65,536 points 2.75 ms and 0.63).
   __shared__ unsigned long long s_q;
-  for (;;) {
-    __syncthreads();
-    if (threadIdx.x == 0) s_q = atomicAdd(a.taken, 1ull);
-    __syncthreads();
-    const uint64_t q = s_q;
-    if (q >= (uint64_t) a.n_big * a.ndir) break;
+  for (uint64_t q = blockIdx.x; q < (uint64_t) a.n_big * a.ndir;) {
     const uint32_t r = (uint32_t) (q / a.ndir);
     const int d = (int) (q % a.ndir);
     const uint32_t p = a.order[r];
     const hd_problem pr = a.probs[p];
     const uint64_t nx = d == 0 ? pr.n_a : pr.n_b;
-    if (nx <= (uint64_t) a.small_rows || nx > (uint64_t) a.pipe_rows) continue;
-    cta_direction<D>(a, p, d, pr, d == 0 ? a.wb_a + pr.offset_a : a.wb_b + pr.offset_b);
+    if (nx > (uint64_t) a.small_rows && nx <= (uint64_t) a.pipe_rows)
+      cta_direction<D>(a, p, d, pr, d == 0 ? a.wb_a + pr.offset_a : a.wb_b + pr.offset_b);
+    __syncthreads();
+    if (threadIdx.x == 0) s_q = gridDim.x + atomicAdd(a.taken, 1ull);
+    __syncthreads();
+    q = s_q;
   }
   // Then the one-warp directions, one per warp; the next one is asked for
   // before this one's work.
   const uint64_t npd = (uint64_t) a.nprob * a.ndir;
-  unsigned long long mine = 0;
-  if (lane == 0) mine = atomicAdd(a.taken + 1, 1ull);
+  const uint64_t nw = (uint64_t) gridDim.x * (kBatchThreads / 32);
+  unsigned long long mine = (uint64_t) (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
   for (;;) {
     const uint64_t q = __shfl_sync(0xFFFFFFFFu, mine, 0);
     if (q >= npd) break;
-    if (lane == 0) mine = atomicAdd(a.taken + 1, 1ull);
+    if (lane == 0) mine = nw + atomicAdd(a.taken + 1, 1ull);
     const uint32_t r = (uint32_t) (q / a.ndir);
     const int d = (int) (q % a.ndir);
     const uint32_t p = a.order[r];
@@ -1478,9 +1481,10 @@ hd_status batch_solve(Ctx& c, const float* A, uint64_t total_a, const float* B, 
   for (int k = 0; k < 5; ++k) {
     int occ = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, g.fns[k], kBatchThreads, 0);
-    const uint64_t warps = k < 3 ? chunks : (k == 3 ? long_cap : n * ndir);
+    // (The one-warp path: a block per direction while they are few.)
+    const uint64_t blocks = k == 4 ? n * ndir : ((k < 3 ? chunks : long_cap) + 7) / 8;
     g.grids[k] = (int) std::max<uint64_t>(
-        1, std::min<uint64_t>((uint64_t) c.num_sms * std::max(occ, 1), (warps + 7) / 8));
+        1, std::min<uint64_t>((uint64_t) c.num_sms * std::max(occ, 1), blocks));
   }
 
   // One graph: reset, plan, window, seed, sweep, long rows, certification,
