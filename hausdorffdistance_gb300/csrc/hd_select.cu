@@ -248,9 +248,16 @@ bool select_variant_by_size(const Ctx& c, uint64_t nA, uint64_t nB, int dims, in
   const double pairs = (double) nA * (double) nB;
   if (dims != 2 && dims != 3) {
     // The tiles take about 95 us per direction at least; the scan passes that at
-    // 1.4e6 pairs in 10-D, 4e6 in 4-D.
+    // 1.4e6 pairs in 10-D, 4e6 in 4-D.  They pack every row of A as well, 0.2 ns a
+    // padded coordinate and product, which few targets don't repay: scan and tiles, us,
+    // 4-D 1M x 2,400 527 and 605, 200k x 1,200 166 and 164, 20k x 600 93 and 92; 10-D 1M x
+    // 300 254 and 322, 1M x 600 376 and 360, 20k x 300 103 and 97; 32-D 1M x 100 317 and
+    // 335, 1M x 300 434 and 384; in 64-D the tiles are ahead from 100 targets.
     const double least = tu.bf16_min_pairs * (dims <= 8 ? 2.0 : 1.0);
-    *v = dims <= kBf16MaxDims && pairs >= least ? HD_VARIANT_BF16 : HD_VARIANT_EB;
+    const uint64_t few = dims <= 8 ? 600 : dims <= 16 ? 300 : dims <= 32 ? 100 : 1;
+    const uint64_t wide = dims <= 8 ? 150 : dims <= 16 ? 1500 : dims <= 32 ? 5000 : ~0ull;
+    const bool tiles = dims <= kBf16MaxDims && pairs >= least && nB >= few && nA / nB <= wide;
+    *v = tiles ? HD_VARIANT_BF16 : HD_VARIANT_EB;
     return true;
   }
   const bool sample = c.opt.always_sample != 0;

@@ -188,3 +188,20 @@ def test_auto_where_bounds_have_no_value(engine, kind, dims, na, nb):
         d2 = hd_oracle.exact(a, b[keep], 32)[0]
         assert got[0][0] == np.sqrt(np.float32(d2)) and keep[got[0][3]]
         assert hd_oracle.dist2_f32(a[got[0][2]], b[got[0][3]]) == np.float32(d2)
+
+
+# Few targets don't repay packing A: there AUTO scans, in either direction by its
+# own sizes.
+@pytest.mark.parametrize("dims,na,nb,tiles", [
+    (4, 200_000, 599, False), (4, 20_000, 600, True), (4, 151_000, 1000, False),
+    (10, 100_000, 299, False), (16, 20_000, 300, True), (16, 600_000, 320, False),
+    (32, 100_000, 99, False), (32, 100_000, 100, True), (64, 100_000, 20, True)])
+def test_auto_scans_for_few_targets(engine, dims, na, nb, tiles):
+    rng = np.random.default_rng(dims + nb)
+    a = rng.standard_normal((na, dims)).astype(np.float32)
+    b = rng.standard_normal((nb, dims)).astype(np.float32)
+    r = engine.solve(a, b)
+    d2 = hd_oracle.exact(a, b, 32)[0]
+    assert np.float32(r.hd_f32) == np.sqrt(np.float32(d2))
+    assert hd_oracle.dist2_f32(a[r.ia], b[r.ib]) == np.float32(d2)
+    assert r.variant_used == (4 if tiles else 1)
