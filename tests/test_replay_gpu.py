@@ -54,13 +54,11 @@ def test_given_up_sets_replay():
     a, b = synth.planes3d(120_000, seed=4)
     ta, tb = torch.from_numpy(a[:100_000]).cuda(), torch.from_numpy(b).cuda()
     with hd.Engine() as engine, hd.Engine(lbvh_budget=257) as index:  # the table's and a visit
-        times = []
-        for e in (engine, index):
-            ts = []
-            for _ in range(60):
+        times = {engine: [], index: []}
+        for _ in range(60):  # in turn
+            for e, ts in times.items():
                 torch.cuda.synchronize()
                 t = time.perf_counter()
                 e.solve(ta, tb, variant="auto")
                 ts.append(time.perf_counter() - t)
-            times.append(np.median(ts[5:]))
-        assert times[0] < 1.1 * times[1], times
+        assert min(times[engine]) < 1.1 * min(times[index])
