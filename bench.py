@@ -370,7 +370,11 @@ def _fp32_issue_peak(local, sm_mhz):
     return sms * 128 * (sm_mhz or 2070.0) * 1e6
 
 
-CELL_FILTER_MIN_POINTS = 40000  # |A| + |B|: csrc/hd_internal.h, kCellsMinPoints
+def _cell_filter_min_points():
+    """|A| + |B| from which the cell filter goes before the index."""
+    import re
+    path = os.path.join(ROOT, "hausdorffdistance_gb300", "csrc", "hd_internal.h")
+    return int(re.search(r"kCellsMinPoints = (\d+);", open(path).read()).group(1))
 
 
 def _lbvh_phases(n_a, n_b, dims, undirected, rc, phase):
@@ -457,14 +461,18 @@ def bench_single(eng, name, n, steps, warmup, args, ctx):
     used = (hd._lib.VARIANT_NAMES.get(res.variant_used),
             hd._lib.VARIANT_NAMES.get(res.variant_used_ba) if undirected else None)
     roof, phases = None, []
-    if res.variant_used == hd._lib.VARIANT_LBVH and 2 * n >= CELL_FILTER_MIN_POINTS:
-        # The cell filter (and the LBVH over what it leaves): the points are read
-        # for the boxes and for the occupied cells, their cell codes written and
-        # read; the rest of the chain works on the maps and on short lists.
-        alg = 2 * n * (2 * dims * 4 + 8)
+    if res.variant_used == hd._lib.VARIANT_LBVH and 2 * n >= _cell_filter_min_points():
+        # The cell filter, and the LBVH over what it left or gave up (if nodes were
+        # visited): the points are read for the boxes and for the occupied cells,
+        # their cell codes written and read; the index adds the nodes and leaves it
+        # visited.
+        alg = (2 * n * (2 * dims * 4 + 8) + rc.visited_nodes * 32
+               + rc.visited_leaves * 16 * dims * 4)
         t_ms = float(sum(phase))
         ach = alg / (t_ms / 1e3) / 1e9
-        roof = {"bound": "hbm", "kernel": "cell_filter", "achieved": ach,
+        roof = {"bound": "hbm",
+                "kernel": "cell_filter+lbvh" if rc.visited_nodes else "cell_filter",
+                "achieved": ach,
                 "peak": peaks["hbm_gbs"], "unit": "GB/s", "frac": ach / peaks["hbm_gbs"],
                 "traffic": None, "algorithmic_bytes": alg, "ms": t_ms,
                 "issue_active_ncu": None, "peak_source": pkind + " hbm_gbs"}
