@@ -7,9 +7,9 @@
 // Work decomposition.  A problem-direction (problem p, A->B or B->A) is cut
 // into items of 32 query rows; one warp processes one item, one lane per
 // row.  Items are ordered largest problem first (longest-processing-time
-// order over |A|*|B|, by octaves, from a radix sort inside the graph).  Warps take chunks of consecutive items in grid-stride order and
-// walk from item to item, so the item -> problem lookup is one binary search
-// per chunk.  The graph runs:
+// order over |A|*|B|, by octaves, from a radix sort inside the graph).  Warps
+// take chunks of consecutive items in grid-stride order and walk from item to
+// item, so the item -> problem lookup is one binary search per chunk.  The graph runs:
 //   plan:   sort keys, radix sort, item counts, exclusive scan;
 //   window: every row takes the minimum over a few points of the other set
 //           around its relative position (row * |Y| / |X|), an upper bound on

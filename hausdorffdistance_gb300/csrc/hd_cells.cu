@@ -32,22 +32,25 @@
 // strictly nearer than L <= h and cannot be the maximum, so value, pair and
 // direction are those of the full search.  The filter gives up (the whole
 // sets go to the index) when L is not several cell diagonals: then the cells
-// are too coarse to tell the points apart.
+// are too coarse to tell the points apart; and when too much is far to search
+// (k_cell_search).
 //
 // What it gave (undirected, device inputs, one GB300; before: both sets sorted
 // and gathered, both trees built, every query walked): 3-D clusters 10M + 10M
-// 1.55 -> 0.38 ms, LiDAR planes 50M + 50M 7.8 -> 4.0 ms, 2-D uniform 200k + 200k
-// with outliers 0.285 -> 0.150 ms, 4M + 3M 0.89 -> 0.45 ms; directed 1M + 0.7M
-// clusters 0.42 -> 0.23 ms.  On 10M + 10M clusters 200 of 20M points stay open.
+// 1.55 -> 0.34 ms, LiDAR planes 50M + 50M 7.7 -> 4.0 ms, 2-D uniform 200k + 200k
+// with outliers 0.29 -> 0.12 ms, 4M + 4M 1.03 -> 0.47 ms; directed 1M + 0.7M
+// clusters 0.43 -> 0.19 ms.  On 10M + 10M clusters 200 of 20M points stay open.
+// What it costs where it gives up, by the cells or late: planes directed 3M + 4M
+// 0.77 -> 0.86 ms, 12M + 20M 2.31 -> 2.45, 2-D uniform 21M + 21M 5.5 -> 6.3, shells of
+// 1M points 1.36 -> 1.42.
 // Its bound there: four passes over the points (box 43 us, cells 83, collect 35)
 // at 5 to 6 TB/s, and a chain of eight small kernels (150 us).
 //
 // Geometry is in units of a cell.  A coordinate's cell unit u = (v - lo) *
 // scale carries two roundings relative to at most G cells, under G 2^-23, and
 // a gap compares two of them: kPad = G 2^-21 widens every cell by twice that.
-// Squared bounds carry kSlack,
-// which covers the roundings of their own arithmetic and of the FP32 pair
-// formula (each a few 2^-24).
+// Squared bounds carry kSlack, which covers the roundings of their own arithmetic
+// and of the FP32 pair formula (each a few 2^-24).
 #include <algorithm>
 #include <cfloat>
 #include <cmath>
@@ -774,6 +777,9 @@ __global__ void __launch_bounds__(256) k_cell_blocks(CellArgs a) {
   // blocks apart along x still are within it (-1: none).
   constexpr int kRows = D == 3 ? 25 : 7;
   __shared__ int s_far[kRows];
+  // (A pair settled here may lie G 2^-22 cells further apart per axis than its
+  // blocks, whose far corners are at least sqrt(2) blocks apart: at 2^13 cells 0.05 %
+  // of the square, under the 0.1 % taken off.)
   const float reach = (stop / kSlack) / (float) (Ge::S * Ge::S) * 0.999f;
   const int step = max(1, (int) (sqrtf(reach) * (D == 3 ? 0.3f : 0.2f)));
   if (threadIdx.x < kRows) {
@@ -788,70 +794,70 @@ __global__ void __launch_bounds__(256) k_cell_blocks(CellArgs a) {
   __shared__ uint32_t s_sum[8], s_base;
   for (uint32_t block = blockIdx.x * 256 + threadIdx.x; block < Ge::kBlocks;
        block += gridDim.x * 256) {
-  const bool some = (a.coarse[d.qset][block >> 5] >> (block & 31)) & 1u;
-  if (!__syncthreads_or(some)) continue;
-  const unsigned long long m = some ? a.occ[d.qset][block] : 0ull;
-  bool open = m != 0;
-  if (open) {
-    const int bx = block % Ge::NB, by = block / Ge::NB % Ge::NB;
-    const int bz = D == 3 ? block / (Ge::NB * Ge::NB) : 0;
-    const unsigned long long* rows = reinterpret_cast<const unsigned long long*>(a.coarse[1 - d.qset]);
-    // The row's word (3-D) or the words within reach (2-D).
-    auto row = [&](int j) -> unsigned long long {
-      const int y = by + (D == 3 ? j % 5 - 2 : j - 3) * step;
-      const int z = D == 3 ? bz + (j / 5 - 2) * step : 0;
-      const int far = s_far[j];
-      if (far < 0 || (uint32_t) y >= (uint32_t) Ge::NB || (uint32_t) z >= (uint32_t) Ge::NB) return 0;
-      const unsigned long long* w = rows + (size_t) (D == 3 ? z * Ge::NB + y : y) * Ge::kWords;
-      const int x0 = max(bx - far, 0), x1 = min(bx + far, Ge::NB - 1);
-      unsigned long long any = 0;
-      for (int k = x0 >> 6; k <= x1 >> 6; ++k) {
-        unsigned long long bits = ld_global_u64(w + k);
-        if (k == x0 >> 6) bits &= ~0ull << (x0 & 63);
-        if (k == x1 >> 6) bits &= ~0ull >> (63 - (x1 & 63));
-        any |= bits;
+    const bool some = (a.coarse[d.qset][block >> 5] >> (block & 31)) & 1u;
+    if (!__syncthreads_or(some)) continue;
+    const unsigned long long m = some ? a.occ[d.qset][block] : 0ull;
+    bool open = m != 0;
+    if (open) {
+      const int bx = block % Ge::NB, by = block / Ge::NB % Ge::NB;
+      const int bz = D == 3 ? block / (Ge::NB * Ge::NB) : 0;
+      const unsigned long long* rows = reinterpret_cast<const unsigned long long*>(a.coarse[1 - d.qset]);
+      // The row's word (3-D) or the words within reach (2-D).
+      auto row = [&](int j) -> unsigned long long {
+        const int y = by + (D == 3 ? j % 5 - 2 : j - 3) * step;
+        const int z = D == 3 ? bz + (j / 5 - 2) * step : 0;
+        const int far = s_far[j];
+        if (far < 0 || (uint32_t) y >= (uint32_t) Ge::NB || (uint32_t) z >= (uint32_t) Ge::NB) return 0;
+        const unsigned long long* w = rows + (size_t) (D == 3 ? z * Ge::NB + y : y) * Ge::kWords;
+        const int x0 = max(bx - far, 0), x1 = min(bx + far, Ge::NB - 1);
+        unsigned long long any = 0;
+        for (int k = x0 >> 6; k <= x1 >> 6; ++k) {
+          unsigned long long bits = ld_global_u64(w + k);
+          if (k == x0 >> 6) bits &= ~0ull << (x0 & 63);
+          if (k == x1 >> 6) bits &= ~0ull >> (63 - (x1 & 63));
+          any |= bits;
+        }
+        return any;
+      };
+      // The middle row first, then five (2-D: three) at a time.
+      open = row(kRows / 2) == 0;
+      constexpr int kGroup = D == 3 ? 5 : 3;
+      for (int j0 = 0; j0 < kRows && open; j0 += kGroup) {
+        unsigned long long any = 0;
+#pragma unroll
+        for (int k = 0; k < kGroup; ++k)
+          if (j0 + k < kRows) any |= row(j0 + k);
+        open = any == 0;
       }
-      return any;
-    };
-    // The middle row first, then five (2-D: three) at a time.
-    open = row(kRows / 2) == 0;
-    constexpr int kGroup = D == 3 ? 5 : 3;
-    for (int j0 = 0; j0 < kRows && open; j0 += kGroup) {
-      unsigned long long any = 0;
-#pragma unroll
-      for (int k = 0; k < kGroup; ++k)
-        if (j0 + k < kRows) any |= row(j0 + k);
-      open = any == 0;
     }
-  }
-  // Room for the open blocks' cells, one atomic per CTA.
-  const uint32_t cnt = open ? (uint32_t) __popcll(m) : 0u;
-  uint32_t incl = cnt;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // Room for the open blocks' cells, one atomic per CTA.
+    const uint32_t cnt = open ? (uint32_t) __popcll(m) : 0u;
+    uint32_t incl = cnt;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-    if (lane >= o) incl += v;
-  }
-  if (lane == 31) s_sum[warp] = incl;
-  __syncthreads();
-  uint32_t base = 0, total = 0;
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+      if (lane >= o) incl += v;
+    }
+    if (lane == 31) s_sum[warp] = incl;
+    __syncthreads();
+    uint32_t base = 0, total = 0;
 #pragma unroll
-  for (int k = 0; k < 8; ++k) {
-    if (k < warp) base += s_sum[k];
-    total += s_sum[k];
-  }
-  if (total == 0) continue;
-  if (threadIdx.x == 0) s_base = atomicAdd(&d.st->n_cells, total);
-  __syncthreads();
-  base += s_base + incl - cnt;
-  unsigned long long rest = open ? m : 0ull;
-  while (rest) {
-    const int t = __ffsll((long long) rest) - 1;
-    rest &= rest - 1;
-    if (base < d.cap_cells) d.cells[base] = block * 64 + t;
-    ++base;
-  }
+    for (int k = 0; k < 8; ++k) {
+      if (k < warp) base += s_sum[k];
+      total += s_sum[k];
+    }
+    if (total == 0) continue;
+    if (threadIdx.x == 0) s_base = atomicAdd(&d.st->n_cells, total);
+    __syncthreads();
+    base += s_base + incl - cnt;
+    unsigned long long rest = open ? m : 0ull;
+    while (rest) {
+      const int t = __ffsll((long long) rest) - 1;
+      rest &= rest - 1;
+      if (base < d.cap_cells) d.cells[base] = block * 64 + t;
+      ++base;
+    }
   }
 }
 
@@ -977,8 +983,9 @@ __global__ void __launch_bounds__(kSearchThreads) k_cell_search(CellArgs a) {
 // for them among kMarkChunk far cells at a time and takes each with all its
 // warps.  They sit together in the list, so that a CTA's chunk is taken from all
 // over it (10M clusters 53 -> 43 us against chunks of neighbours, two thirds of
-// the SMs idle then; the call 350 -> 345, 1M 203 -> 195).  Of more than kManyFar far cells many may be marked: then a thread per
-// cell marks whole blocks within the distance.
+// the SMs idle then; the call 350 -> 345, 1M 203 -> 195).  Of more than kManyFar far
+// cells many may be marked: then a thread per cell marks whole blocks within the
+// distance.
 constexpr uint32_t kMarkChunk = 8;
 
 // Where the map of blocks is too large for shared memory, a top map of 2^18
@@ -1334,7 +1341,8 @@ hd_status enqueue(Ctx& c, const DirInput* ins, int count, const F64Plan* plan, C
     o_N[k] = take(fine);
   }
   const size_t zero_bytes = off;
-  size_t o_coarse[2], o_code[2], o_cells[2], o_masks[2], o_rim[2], o_far[2], o_fub[2], o_q[2], o_qmin[2], o_t[2];
+  size_t o_coarse[2], o_code[2], o_cells[2], o_masks[2], o_rim[2], o_far[2], o_fub[2];
+  size_t o_q[2], o_qmin[2], o_t[2];
   for (int k = 0; k < 2; ++k) {
     o_coarse[k] = take(coarse);
     o_code[k] = take((n[k] + 3) / 4 * 16);

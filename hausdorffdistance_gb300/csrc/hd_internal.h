@@ -433,9 +433,9 @@ bool cells_apply(const Ctx& c, uint64_t nA, uint64_t nB, int dims);
 // sorted already); -1: none.
 int cells_level(uint64_t points, int dims);
 int cells_finer(uint64_t points, int dims, int level, float reach, bool sorted);
-// Filters `count` directions: the call's (ins[k].dir == k), or one of them.  With a plan, queries are
-// settled by the FP64 listing pass's level, and the pair scan leaves the open
-// queries' FP32 minima; no direction is finished here.
+// Filters `count` directions: the call's (ins[k].dir == k), or one of them.  With
+// a plan, queries are settled by the FP64 listing pass's level, and the pair scan
+// leaves the open queries' FP32 minima; no direction is finished here.
 // Without a plan the results of finished directions are in the pinned staging
 // (DevScalars by direction).  boxes_known: DevScalars[0].mbr_ord already holds
 // the sets' boxes.

@@ -11,8 +11,8 @@
 //      points of A (k = sample_rate * |A|, clamped to [64, 256]) run the
 //      early-break scan against B, one CTA each, B visited in a
 //      pseudo-random order, counting the B points each visited before it
-//      stopped (in rounds of 64, capped at 16,384).  Seeds and completed samples also seed the running maximum
-//      that the chosen variant starts from.
+//      stopped (in rounds of 64, capped at 16,384).  Seeds and completed samples
+//      also seed the running maximum that the chosen variant starts from.
 //   2. The EB cost of the full set is ~ |A| * mean pairs, mean being the
 //      average of the sampled counts; the index-based cost is ~ |A| + |B|
 //      point operations.  EB is chosen when
@@ -47,8 +47,8 @@
 //      LBVH, both without sampling (at the largest sizes the grid's worst
 //      cases cost tens of times the LBVH while its best cases save ~20%);
 //      inputs with n_dims other than 2 or 3 take the split-BF16 tiles (padded
-//      with zeros to a multiple of 16) when n_dims is at most 64 and the pair
-//      count is large, else the FP32 scan.  10-D unit rows, 60,000 x 50,000:
+//      with zeros to a multiple of 16) when n_dims is at most 64, the pair count
+//      is large and the targets are not few, else the FP32 scan.  10-D unit rows, 60,000 x 50,000:
 //      7.6 ms by the scan, 0.54 by the tiles; 24-D, 9,000 x 8,000: 0.80 and 0.12.
 //   All thresholds come from the autotuner's table
 //   (hausdorffdistance_gb300/autotune.py fits them over a sweep of

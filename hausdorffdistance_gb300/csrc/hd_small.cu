@@ -1,7 +1,7 @@
 // Small 2-D and 3-D sets: the whole solve in one kernel, every pair.
 //
-// Up to kSmallPairs pairs per direction, all pairs cost less than the launches of an early
-// break (src/hd_impl/hausdorff_distance_early_break.h:117-219 needs its seeds,
+// Up to kSmallPairs pairs per direction, all pairs cost less than the launches of
+// an early break (src/hd_impl/hausdorff_distance_early_break.h:117-219 needs its seeds,
 // its scan, its stragglers and the certification one after the other, twice
 // for an undirected solve).  A CTA takes items of a query tile (QPT queries
 // per thread) by a chunk of targets in shared memory and lowers the queries'
