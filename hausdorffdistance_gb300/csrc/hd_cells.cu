@@ -1301,9 +1301,15 @@ constexpr float kFinerReach = 2.5f;
 
 }  // namespace
 
-bool cells_apply(const Ctx& c, uint64_t nA, uint64_t nB, int dims) {
+// Not for one direction against few targets: hardly a cell of the queries is near
+// one.  The index alone and the filter first, us: 1M x 3,000 uniform 3-D 326 and 655,
+// 10M x 100 2-D 650 and 1055, FP64 1M x 1,000 311 and 362 (undirected the other
+// direction makes up for it).
+constexpr uint64_t kCellsMaxRatio = 128;
+
+bool cells_apply(const Ctx& c, uint64_t nA, uint64_t nB, int dims, bool undirected) {
   return (dims == 2 || dims == 3) && nA + nB >= kCellsMinPoints &&
-         c.opt.lbvh_budget == tuning().lbvh_budget;
+         (undirected || nA / kCellsMaxRatio <= nB) && c.opt.lbvh_budget == tuning().lbvh_budget;
 }
 
 namespace {

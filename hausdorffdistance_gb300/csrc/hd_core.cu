@@ -397,7 +397,9 @@ hd_status run_direction(Ctx& c, const DirInput& in, int variant, int* used,
 // x 18,000 from the host 139 and 109, 20,000 x 20,000 126 and 126, 25,000 x 25,000
 // 161 and 139, 1M x 1M 2500 and 1020; undirected clusters 15,000 x 15,000 218 and
 // 188; below, directed clusters 13,000 x 13,000 108 and 132.
-constexpr uint64_t kSeedMinPoints = 35000;
+// A scan of a small set is over before that: 20 x 60,000 54 and 83, 100 x 1M 168
+// and 602, 1 x 1M 71 and 245.
+constexpr uint64_t kSeedMinPoints = 35000, kSeedMinSet = 8000;
 
 // A is sorted while B is copied, before it is known that the sort is of use, when
 // it ends with the copy: about 100 us and 35 ps a point, against 19 ps a float over
@@ -647,7 +649,7 @@ hd_status hd_solve(hd_ctx* c, const float* A, uint64_t n_a, const float* B,
   // which eb_only_threshold may ask for).  It does not wait for the selector:
   // its kernels follow the sample's, and the host evaluates the sample while
   // they run.
-  bool cells = !small && cells_apply(*c, n_a, n_b, n_dims) &&
+  bool cells = !small && cells_apply(*c, n_a, n_b, n_dims, undirected) &&
                (variant == HD_VARIANT_LBVH ||
                 (variant == HD_VARIANT_AUTO && c->opt.eb_only_threshold == 0));
   if (!small && (s = init_scalars(*c)) != HD_OK) return s;
@@ -826,7 +828,7 @@ hd_status hd_solve(hd_ctx* c, const float* A, uint64_t n_a, const float* B,
     } else {
       // The early-break scan starts from the cell filter's lower bound.
       if (used[0] == HD_VARIANT_EB && (n_dims == 2 || n_dims == 3) &&
-          (n_a + n_b) * ndir >= kSeedMinPoints) {
+          (n_a + n_b) * ndir >= kSeedMinPoints && std::min(n_a, n_b) >= kSeedMinSet) {
         if ((r = cells_seed(*c, ins, ndir)) != HD_OK) return r;
       }
       for (int d = 0; d < ndir; ++d) {

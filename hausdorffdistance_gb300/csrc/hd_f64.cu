@@ -1132,7 +1132,7 @@ hd_status hd_solve_f64(hd_ctx* c, const double* A, uint64_t n_a, const double* B
     // the filter's other kernels.
     bool open[2] = {true, undirected}, off[2] = {false, false};
     CellsLeft left[2];
-    if (cells_apply(*c, n_a, n_b, n_dims)) {
+    if (cells_apply(*c, n_a, n_b, n_dims, undirected)) {
       CellsRun run;
       float reach[2];
       plan_of(0, ndir);

@@ -427,7 +427,7 @@ struct CellsLeft {
   uint64_t nq = 0, nt = 0;
 };
 constexpr uint64_t kCellsMinPoints = 40000;
-bool cells_apply(const Ctx& c, uint64_t nA, uint64_t nB, int dims);
+bool cells_apply(const Ctx& c, uint64_t nA, uint64_t nB, int dims, bool undirected);
 // The grid (level) to start on, and the one to try again on when the filter
 // neither finished nor narrowed a direction (its L: `reach` cells; sorted: a set is
 // sorted already); -1: none.
