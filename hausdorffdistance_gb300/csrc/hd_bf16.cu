@@ -22,8 +22,8 @@
 // below the lower bound L of some completed row cannot be the maximum and is
 // dropped, and the remaining rows are packed together before the next run.
 // Undirected, one GB300, every pair before, runs now: 64-D unit rows 1M x 1M
-// 422 -> 85 ms, 250k x 250k 28.1 -> 7.4 ms, 64k x 64k 2.19 -> 1.60 ms; 16-D
-// 500k x 300k directed 21.7 -> 3.9 ms.
+// 425 -> 85 ms (80 to 89 by the chip's power cap), 250k x 250k 28.1 -> 7.4 ms,
+// 64k x 64k 2.19 -> 1.60 ms; 16-D 500k x 300k directed 21.7 -> 3.9 ms.
 //
 // Kernel shape (one CTA per 256 A rows = two 128-row regions, 6 warps, 1 CTA
 // per SM):
